@@ -55,6 +55,10 @@ def _emu_lib():
         lib.cmf_emu_colsum.argtypes = [i, i, vp, vp, vp]
         lib.cmf_emu_mse_grad.argtypes = [i, i, i, vp, vp, vp, vp, vp, vp]
         lib.cmf_emu_adam.argtypes = [i, vp, vp, vp, vp, vp, f, f, f, f, i, f, vp]
+        lib.cmf_emu_adam_set.argtypes = [i, vp, vp, vp, vp, vp, vp, vp, f, f, f, f, i, vp]
+        lib.cmf_emu_loss_grad_ws_floats.restype = C.c_size_t
+        lib.cmf_emu_loss_grad_ws_floats.argtypes = [i]
+        lib.cmf_emu_loss_grad.argtypes = [i, i, vp, vp, vp, vp, vp, vp, vp, vp, C.c_size_t, vp]
         lib.cmf_emu_features.argtypes = [C.POINTER(EmuNet), C.POINTER(EmuMember), i, vp, i, i, i, vp, vp]
         lib.cmf_emu_rollout.argtypes = [C.POINTER(EmuNet), C.POINTER(EmuMember), i, vp, vp, i, i, d, i, vp, vp]
         lib.cmf_emu_mlp_pack_bytes.restype = C.c_size_t
@@ -239,18 +243,33 @@ class MLP:
 
     def adam(self, wd: float = 0.0):
         self.step += 1
-        for k in range(4):
-            echeck(self.lib.cmf_emu_adam(self.W[k].numel(), self.W[k].data_ptr(), self.Wb[k].data_ptr(), self.gW[k].data_ptr(),
-                                         self.mW[k].data_ptr(), self.vW[k].data_ptr(), self.lr, 0.9, 0.999, 1e-8, self.step,
-                                         wd, self.stream), "adam")
-            echeck(self.lib.cmf_emu_adam(self.b[k].numel(), self.b[k].data_ptr(), None, self.gb[k].data_ptr(),
-                                         self.mb[k].data_ptr(), self.vb[k].data_ptr(), self.lr, 0.9, 0.999, 1e-8, self.step,
-                                         0.0, self.stream), "adam")
+        w = self.W + self.b
+        p8 = C.c_void_p * 8
+        ptrs = lambda ts: p8(*[t.data_ptr() for t in ts])  # noqa: E731
+        echeck(self.lib.cmf_emu_adam_set(8, (C.c_int32 * 8)(*[t.numel() for t in w]), ptrs(w),
+                                         p8(*[t.data_ptr() for t in self.Wb], None, None, None, None), ptrs(self.gW + self.gb),
+                                         ptrs(self.mW + self.mb), ptrs(self.vW + self.vb),
+                                         (C.c_float * 8)(wd, wd, wd, wd, 0.0, 0.0, 0.0, 0.0), self.lr, 0.9, 0.999, 1e-8,
+                                         self.step, self.stream), "adam")
 
     def loss_and_grad(self, X, t, valid: int):
+        """Mean-squared error over the first `valid` rows (0-dim tensor) and its gradients in gW/gb."""
         torch = self.torch
-        Y, acts = self.forward(X)
         R = X.shape[0]
+        # one pass over the rows on the tensor cores; rows in another layout take the layer-by-layer chain
+        if (X.dtype == torch.bfloat16 and X.shape[1:] == (IN,) and R > 0 and R % 64 == 0 and X.is_contiguous()
+                and X.data_ptr() % 16 == 0 and t.dtype == torch.float32 and t.is_contiguous()):
+            need = int(self.lib.cmf_emu_loss_grad_ws_floats(R))
+            if getattr(self, "_tws", None) is None or self._tws.numel() < need:
+                self._tws = torch.empty(need, dtype=torch.float32, device=self.dev)
+            loss = torch.empty((), dtype=torch.float32, device=self.dev)
+            p4 = C.c_void_p * 4
+            ptrs = lambda ts: p4(*[v.data_ptr() for v in ts])  # noqa: E731
+            echeck(self.lib.cmf_emu_loss_grad(R, valid, X.data_ptr(), t.data_ptr(), ptrs(self.Wb), ptrs(self.b), ptrs(self.gW),
+                                              ptrs(self.gb), loss.data_ptr(), self._tws.data_ptr(), self._tws.numel(),
+                                              self.stream), "loss_grad")
+            return loss
+        Y, acts = self.forward(X)
         dY = torch.empty(R, OUT, dtype=torch.float32, device=self.dev)
         dYb = torch.empty(R, OUT, dtype=torch.bfloat16, device=self.dev)
         parts = torch.empty((R + 255) // 256, dtype=torch.float32, device=self.dev)

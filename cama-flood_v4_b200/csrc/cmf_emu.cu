@@ -278,12 +278,22 @@ __global__ void k_colsum(int rows, int cols, const float *__restrict__ X, float 
     }
 }
 
-// Adam on fp32 master weights, bf16 copy for the tensor cores
-__global__ void k_adam(int n, float *w, __nv_bfloat16 *wb, const float *__restrict__ grad, float *m, float *v, float lr,
-                       float b1, float b2, float eps, float bc1, float bc2, float wd) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const float gr = grad[i] + wd * w[i];
+// Adam on fp32 master weights, bf16 copy for the tensor cores; up to 8 tensors in one launch, tensor
+// k on blockIdx.y (the 8 tensors of a training step took 8 launches, each far below a wave)
+constexpr int kAdamMax = 8;
+struct AdamSet {
+    int n[kAdamMax];
+    float *w[kAdamMax];
+    __nv_bfloat16 *wb[kAdamMax];
+    const float *grad[kAdamMax];
+    float *m[kAdamMax], *v[kAdamMax];
+    float wd[kAdamMax];
+};
+__global__ void k_adam(AdamSet a, float lr, float b1, float b2, float eps, float bc1, float bc2) {
+    const int k = blockIdx.y, i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= a.n[k]) return;
+    float *w = a.w[k], *m = a.m[k], *v = a.v[k];
+    const float gr = a.grad[k][i] + a.wd[k] * w[i];
     const float mi = b1 * m[i] + (1.f - b1) * gr;
     const float vi = b2 * v[i] + (1.f - b2) * gr * gr;
     m[i] = mi;
@@ -291,7 +301,7 @@ __global__ void k_adam(int n, float *w, __nv_bfloat16 *wb, const float *__restri
     const float upd = lr * (mi / bc1) / (sqrtf(vi / bc2) + eps);
     const float wn = w[i] - upd;
     w[i] = wn;
-    if (wb) wb[i] = __float2bfloat16_rn(wn);
+    if (a.wb[k]) a.wb[k][i] = __float2bfloat16_rn(wn);
 }
 
 // mean-squared-error gradient on column 0 of Y [rows][ldy]: dY = 2 (Y - t) / rows (other columns 0),
@@ -1033,6 +1043,384 @@ __global__ void k_splitk_reduce(int M, int N, int splits, const float *__restric
     C[(size_t)r * ldc + c] = x;
 }
 
+
+// ------------------------------------------------------------------------------------------
+// Fused training step on tcgen05: loss, every weight gradient and every bias gradient of the 4-layer
+// MLP in one pass over the rows (k_train), then one reduction over the CTAs (k_train_reduce).
+//
+// A persistent grid of at most one CTA per SM keeps the bf16 weights in shared memory and takes
+// 128-row tiles t = b, b + G, ...; a tile's activations and dZ never leave the SM, and the weight
+// gradients accumulate in tensor memory over all tiles of the CTA.  Every matrix (rows x columns,
+// column-contiguous in global memory) is stored once, in the canonical no-swizzle layout, and serves
+// each product it enters through the descriptor's major-ness:
+//   forward      D[r][n]  = a[r][k]  W[k][n]     A K-major,  B MN-major
+//   data grad    D[r][k]  = dZ[r][n] W[k][n]     A K-major,  B K-major
+//   weight grad  D[n][k] += dZ[r][n] a[r][k]     A MN-major, B MN-major
+// dZ of a layer replaces that layer's activations in place once their products are done.  The
+// rounding points are those of the layer-by-layer chain (bf16 inputs, weights, activations and dZ;
+// fp32 accumulation, bias, loss and bias gradients), and the K=16 steps of the forward and data
+// products run in its order, so the dZ are its bits; the row sums of the gradients are taken per CTA
+// and then in CTA order, the same on every run.
+// Tensor memory: D 0..127, gW1 128..255, gW2 256..383, gW0 384..447, gW3 448..463, Y 464..479.
+// Bound: the chain of 8 dependent products of a tile (about 0.5 us each); 16 warps share every
+// epilogue (32 columns of one row per thread) to keep its other half short.  Measured with k_adam
+// (loss_and_grad + adam, per step): 16,384 rows 2136 us (layer by layer, about 45 launches) -> 34.5
+// us; 131,072 rows 4934 -> 90 us.
+// ------------------------------------------------------------------------------------------
+constexpr int kTrThreads = 512;
+constexpr int kTrW0 = 0;                                  // [64 k][128 n]
+constexpr int kTrW1 = kTrW0 + 64 * 128 * 2;               // [128 k][128 n]
+constexpr int kTrW2 = kTrW1 + 128 * 128 * 2;
+constexpr int kTrW3 = kTrW2 + 128 * 128 * 2;              // [128 k][16 n], column 0 real
+constexpr int kTrX = kTrW3 + 128 * 16 * 2;                // two [128 r][64 k] tiles
+constexpr int kTrXBytes = 128 * 64 * 2;
+constexpr int kTrAct = kTrX + 2 * kTrXBytes;              // a1, a2, a3 (then dZ0, dZ1, dZ2): [128 r][128]
+constexpr int kTrActBytes = 128 * 128 * 2;
+constexpr int kTrDY = kTrAct + 3 * kTrActBytes;           // [128 r][16], column 0 real
+constexpr int kTrBias = kTrDY + 128 * 16 * 2;             // b0 b1 b2 (3 x 128 floats), W3 column 0, dY (bf16 values)
+constexpr int kTrMisc = kTrBias + 5 * 128 * 4;            // three mbarriers, TMEM address, b3
+constexpr int kTrSmem = kTrMisc + 3 * 8 + 8;
+constexpr int kTrCols = 512;
+constexpr uint32_t kTrGW1 = 128, kTrGW2 = 256, kTrGW0 = 384, kTrGW3 = 448, kTrY = 464;
+// one CTA's partial sums in the workspace (floats)
+constexpr int kTrPW0 = 0, kTrPW1 = kTrPW0 + 64 * 128, kTrPW2 = kTrPW1 + 128 * 128, kTrPW3 = kTrPW2 + 128 * 128;
+constexpr int kTrPb = kTrPW3 + 128;                       // gb0 gb1 gb2, then gb3[0] and the loss
+constexpr int kTrPart = kTrPb + 3 * 128 + 2;
+
+// rows [0, rows) of a global matrix (columns [0, C), C % 8 == 0) into the canonical layout of an
+// R-row matrix, rows past `rows` zero; 8 consecutive threads write one 128-byte core matrix
+__device__ __forceinline__ void tr_load(unsigned char *dst, int R, int C, const __nv_bfloat16 *__restrict__ src, int ld,
+                                        int rows) {
+    const int chunks = C / 8;
+    for (int e = threadIdx.x; e < R * chunks; e += kTrThreads) {
+        const int q = e >> 3, c = q % chunks, r = (q / chunks) * 8 + (e & 7);
+        uint4 v = make_uint4(0u, 0u, 0u, 0u);
+        if (r < rows) v = *reinterpret_cast<const uint4 *>(src + (size_t)r * ld + c * 8);
+        *reinterpret_cast<uint4 *>(dst + canon_off(r, c * 8, R)) = v;
+    }
+}
+
+// one product of `steps` K=16 instructions; a and b are matrices of ra and rb rows in the canonical
+// layout, taken K-major (K = columns) or MN-major (K = rows)
+template <bool AMn, bool BMn>
+__device__ __forceinline__ void tr_mma(uint32_t d, uint32_t a, int ra, uint32_t b, int rb, int N, int steps, bool acc) {
+    const uint32_t idesc = umma_idesc_bf16_f32(128, N) | (AMn ? 1u << 15 : 0u) | (BMn ? 1u << 16 : 0u);
+    const uint32_t pa = ra * 16, pb = rb * 16;            // byte distance of 8-column groups
+    for (int s = 0; s < steps; s++) {
+        const uint64_t ad = AMn ? umma_smem_desc(a + s * 256, 128, pa) : umma_smem_desc(a + s * 2 * pa, pa, 128);
+        const uint64_t bd = BMn ? umma_smem_desc(b + s * 256, 128, pb) : umma_smem_desc(b + s * 2 * pb, pb, 128);
+        umma_bf16(d, ad, bd, idesc, (acc || s > 0) ? 1u : 0u);
+    }
+}
+
+// sums of v[0..31] over the warp's 32 lanes by halving exchanges: lane l returns the sum of v[l]
+__device__ __forceinline__ float tr_colsum(float (&v)[32], int lane) {
+#pragma unroll
+    for (int h = 16; h >= 1; h >>= 1) {
+        const bool up = lane & h;
+#pragma unroll
+        for (int j = 0; j < h; j++) {
+            const float send = up ? v[j] : v[j + h], keep = up ? v[j + h] : v[j];
+            v[j] = keep + __shfl_xor_sync(0xffffffffu, send, h);
+        }
+    }
+    return v[0];
+}
+
+// hidden layer epilogue of row r, columns c0..c0+31: bias, ReLU, bf16 into the activation buffer
+__device__ __forceinline__ void tr_hidden(uint32_t taddr, const float *bias, unsigned char *act, int r, int c0) {
+    uint32_t v[32];
+    tmem_ld32(taddr, v);
+    tmem_wait_ld();
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        uint4 u;
+        uint32_t *w = reinterpret_cast<uint32_t *>(&u);
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            const int c = 8 * q + 2 * j;
+            w[j] = pack_bf16x2(fmaxf(__uint_as_float(v[c]) + bias[c0 + c], 0.f),
+                               fmaxf(__uint_as_float(v[c + 1]) + bias[c0 + c + 1], 0.f));
+        }
+        *reinterpret_cast<uint4 *>(act + canon_off(r, c0 + 8 * q, 128)) = u;
+    }
+}
+
+__device__ __forceinline__ float bf16_lo(uint32_t u) { return __uint_as_float(u << 16); }
+__device__ __forceinline__ float bf16_hi(uint32_t u) { return __uint_as_float(u & 0xffff0000u); }
+
+// dZ = dA where the activation is positive: fp32 values stay in v (for the bias gradient), their
+// bf16 roundings come back packed
+__device__ __forceinline__ void tr_mask(float (&v)[32], const unsigned char *act, int r, int c0, uint4 (&u)[4]) {
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        const uint4 a = *reinterpret_cast<const uint4 *>(act + canon_off(r, c0 + 8 * q, 128));
+        const uint32_t aw[4] = {a.x, a.y, a.z, a.w};
+        uint32_t *w = reinterpret_cast<uint32_t *>(&u[q]);
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            const int c = 8 * q + 2 * j;
+            v[c] = bf16_lo(aw[j]) > 0.f ? v[c] : 0.f;
+            v[c + 1] = bf16_hi(aw[j]) > 0.f ? v[c + 1] : 0.f;
+            w[j] = pack_bf16x2(v[c], v[c + 1]);
+        }
+    }
+}
+__device__ __forceinline__ void tr_put(unsigned char *act, int r, int c0, const uint4 (&u)[4]) {
+#pragma unroll
+    for (int q = 0; q < 4; q++) *reinterpret_cast<uint4 *>(act + canon_off(r, c0 + 8 * q, 128)) = u[q];
+}
+
+struct TrainArgs {
+    const __nv_bfloat16 *X, *W[4];
+    const float *t, *b[4];
+    int rows, valid;
+    float *ws;
+};
+
+__global__ void __launch_bounds__(kTrThreads, 1) k_train(TrainArgs a, int wait_limit) {
+    extern __shared__ __align__(1024) unsigned char sm[];
+    float *sbias = reinterpret_cast<float *>(sm + kTrBias), *sw3 = sbias + 3 * 128, *sdy = sw3 + 128;
+    uint64_t *mbar = reinterpret_cast<uint64_t *>(sm + kTrMisc);
+    uint32_t *tslot = reinterpret_cast<uint32_t *>(mbar + 3);
+    float *sb3 = reinterpret_cast<float *>(tslot + 1);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, G = gridDim.x;
+    const int ntiles = (a.rows + 127) / 128;
+    // ---- weights, biases and the first tile into shared memory
+    tr_load(sm + kTrW0, 64, 128, a.W[0], 128, 64);
+    tr_load(sm + kTrW1, 128, 128, a.W[1], 128, 128);
+    tr_load(sm + kTrW2, 128, 128, a.W[2], 128, 128);
+    tr_load(sm + kTrW3, 128, 16, a.W[3], 64, 128);
+    tr_load(sm + kTrX, 128, 64, a.X + (size_t)blockIdx.x * 128 * 64, 64, a.rows - (int)blockIdx.x * 128);
+    for (int e = tid; e < 128 * 16 * 2 / 16; e += kTrThreads) reinterpret_cast<uint4 *>(sm + kTrDY)[e] = make_uint4(0u, 0u, 0u, 0u);
+    if (tid < 128) {
+        for (int l = 0; l < 3; l++) sbias[l * 128 + tid] = a.b[l][tid];
+        sw3[tid] = __bfloat162float(a.W[3][(size_t)tid * 64]);
+    }
+    if (tid == 0) {
+        *sb3 = a.b[3][0];
+        for (int q = 0; q < 3; q++) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(smem_u32(mbar + q)) : "memory");
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
+                     :: "r"(smem_u32(tslot)), "r"(kTrCols) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    fence_async_smem();
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = *tslot, sb = smem_u32(sm), m0 = smem_u32(mbar), m1 = smem_u32(mbar + 1);
+    const int q = warp & 3, cg = warp >> 2;              // TMEM lanes 32q.., columns 32cg..
+    const int r = 32 * q + lane, c0 = 32 * cg;           // this thread's row and first column
+    const uint32_t trow = tmem + ((uint32_t)(32 * q) << 16);
+    unsigned char *act[3] = {sm + kTrAct, sm + kTrAct + kTrActBytes, sm + kTrAct + 2 * kTrActBytes};
+    const uint32_t sact[3] = {sb + kTrAct, sb + kTrAct + kTrActBytes, sb + kTrAct + 2 * kTrActBytes};
+    const uint32_t sw[3] = {sb + kTrW0, sb + kTrW1, sb + kTrW2};
+    uint32_t p0 = 0, p1 = 0;                             // phases of the two mbarriers
+    float gb[3] = {0.f, 0.f, 0.f}, gb3 = 0.f, loss = 0.f;
+    bool fail = false;
+    // a bounded wait for a commit; one that runs out ends the tile loop at the next block barrier
+    auto wait = [&](uint32_t mb, uint32_t &ph) {
+        if (!mbar_wait(mb, ph, wait_limit)) fail = true;
+        ph ^= 1u;
+        tc_fence_after();
+    };
+    // shared-memory operands and tensor-memory reads of every thread are done: the next product may
+    // start; false, for every thread alike, when a thread's wait ran out
+    auto publish = [&]() -> bool {
+        fence_async_smem();
+        tc_fence_before();
+        const bool bad = __syncthreads_or(fail);
+        tc_fence_after();
+        return !bad;
+    };
+    const bool issuer = tid == 0;
+    bool ok = true;
+    int it = 0;
+    for (int t = blockIdx.x; t < ntiles; t += G, it++) {
+        const bool more = it > 0;                        // gradients accumulate after the first tile
+        const uint32_t sx = sb + kTrX + (it & 1) * kTrXBytes;
+        // the next tile's rows: two 16-byte chunks per thread, stored below into the other buffer
+        uint4 xn[2];
+        const int tn = t + G;
+#pragma unroll
+        for (int e = 0; e < 2; e++) {
+            const int i = tid + e * kTrThreads, c = (i >> 3) & 7, rr = (i >> 6) * 8 + (i & 7);
+            xn[e] = make_uint4(0u, 0u, 0u, 0u);
+            if (tn < ntiles && tn * 128 + rr < a.rows)
+                xn[e] = *reinterpret_cast<const uint4 *>(a.X + ((size_t)tn * 128 + rr) * 64 + c * 8);
+        }
+        const int row = t * 128 + r;
+        const float target = (cg == 0 && row < a.valid && row < a.rows) ? a.t[row] : 0.f;
+        // ---- forward
+        if (issuer) { tr_mma<false, true>(tmem, sx, 128, sw[0], 64, 128, 4, false); umma_commit(m0); }
+        wait(m0, p0);
+        if (tn < ntiles)                                 // the other buffer's last reader (gW0 of the previous tile) is done
+#pragma unroll
+            for (int e = 0; e < 2; e++) {
+                const int i = tid + e * kTrThreads, c = (i >> 3) & 7, rr = (i >> 6) * 8 + (i & 7);
+                *reinterpret_cast<uint4 *>(sm + kTrX + ((it + 1) & 1) * kTrXBytes + canon_off(rr, c * 8, 128)) = xn[e];
+            }
+        tr_hidden(trow + c0, sbias, act[0], r, c0);
+        if (!(ok = publish())) break;
+#pragma unroll
+        for (int l = 1; l < 3; l++) {
+            if (issuer) { tr_mma<false, true>(tmem, sact[l - 1], 128, sw[l], 128, 128, 8, false); umma_commit(m0); }
+            wait(m0, p0);
+            tr_hidden(trow + c0, sbias + 128 * l, act[l], r, c0);
+            if (!(ok = publish())) break;
+        }
+        if (!ok) break;
+        // ---- output layer, loss and dY
+        if (issuer) { tr_mma<false, true>(tmem + kTrY, sact[2], 128, sb + kTrW3, 128, 16, 8, false); umma_commit(m0); }
+        wait(m0, p0);
+        if (cg == 0) {
+            uint32_t yv;
+            tmem_ld1(trow + kTrY, yv);
+            tmem_wait_ld();
+            const float e = (row < a.valid && row < a.rows) ? (__uint_as_float(yv) + *sb3) - target : 0.f;
+            const float dy = 2.f * e / (float)a.valid;
+            const __nv_bfloat16 dyb = __float2bfloat16_rn(row < a.rows ? dy : 0.f);
+            loss += e * e;
+            gb3 += row < a.rows ? dy : 0.f;
+            *reinterpret_cast<__nv_bfloat16 *>(sm + kTrDY + canon_off(r, 0, 128)) = dyb;
+            sdy[r] = __bfloat162float(dyb);
+        }
+        if (!(ok = publish())) break;
+        // ---- gW3 += a3^T dY;  dZ2 = dY W3^T where a3 > 0 (one exact product per element)
+        if (issuer) { tr_mma<true, true>(tmem + kTrGW3, sact[2], 128, sb + kTrDY, 128, 16, 8, more); umma_commit(m0); }
+        float v[32];
+        uint4 u[4];
+        {
+            const float dy = sdy[r];
+#pragma unroll
+            for (int j = 0; j < 32; j++) v[j] = dy * sw3[c0 + j];
+            tr_mask(v, act[2], r, c0, u);
+            gb[2] += tr_colsum(v, lane);
+        }
+        wait(m0, p0);
+        tr_put(act[2], r, c0, u);
+        if (!(ok = publish())) break;
+        // ---- layers 2 and 1: dA = dZ W^T, gW += dZ^T a, dZ of the layer below in place of its activations
+#pragma unroll
+        for (int l = 2; l >= 1; l--) {
+            if (issuer) {
+                tr_mma<false, false>(tmem, sact[l], 128, sw[l], 128, 128, 8, false);
+                umma_commit(m0);
+                tr_mma<true, true>(tmem + (l == 2 ? kTrGW2 : kTrGW1), sact[l], 128, sact[l - 1], 128, 128, 8, more);
+                umma_commit(m1);
+            }
+            wait(m0, p0);
+            uint32_t d[32];
+            tmem_ld32(trow + c0, d);
+            tmem_wait_ld();
+#pragma unroll
+            for (int j = 0; j < 32; j++) v[j] = __uint_as_float(d[j]);
+            tr_mask(v, act[l - 1], r, c0, u);
+            gb[l - 1] += tr_colsum(v, lane);
+            wait(m1, p1);                                // the weight gradient has read the activations
+            tr_put(act[l - 1], r, c0, u);
+            if (!(ok = publish())) break;
+        }
+        if (!ok) break;
+        // ---- gW0 += dZ0^T X; completes before the next tile's first product, which is issued after it
+        if (issuer) tr_mma<true, true>(tmem + kTrGW0, sact[0], 128, sx, 128, 64, 8, more);
+    }
+    // every product issued so far completes (one more commit tracks them all, waited for with the full
+    // bound also after a failure) before the sums are read and the columns released
+    if (issuer) umma_commit(smem_u32(mbar + 2));
+    fail = !mbar_wait(smem_u32(mbar + 2), 0u, kTcWaitLimit) || !ok;
+    const bool failed = __syncthreads_or(fail);
+    tc_fence_after();
+    if (failed) {
+        if (tid == 0) atomicExch(&g_mlp_tc_status, 1);
+    } else {
+        float *out = a.ws + (size_t)blockIdx.x * kTrPart;
+        uint32_t d[32];
+        // D lanes are n, columns k: consecutive lanes store consecutive n of one k
+#pragma unroll
+        for (int l = 1; l < 3; l++) {
+            tmem_ld32(trow + (l == 1 ? kTrGW1 : kTrGW2) + c0, d);
+            tmem_wait_ld();
+#pragma unroll
+            for (int j = 0; j < 32; j++) out[(l == 1 ? kTrPW1 : kTrPW2) + (c0 + j) * 128 + r] = __uint_as_float(d[j]);
+        }
+        if (cg < 2) {
+            tmem_ld32(trow + kTrGW0 + c0, d);
+            tmem_wait_ld();
+#pragma unroll
+            for (int j = 0; j < 32; j++) out[kTrPW0 + (c0 + j) * 128 + r] = __uint_as_float(d[j]);
+        } else if (cg == 2) {
+            uint32_t g;
+            tmem_ld1(trow + kTrGW3, g);
+            tmem_wait_ld();
+            out[kTrPW3 + r] = __uint_as_float(g);
+        }
+        // bias gradients: thread (q, cg, lane) holds column c0 + lane over rows 32q..; the four row
+        // quarters are added in order (the activation buffers are free now)
+        float *sg = reinterpret_cast<float *>(sm + kTrAct);
+#pragma unroll
+        for (int l = 0; l < 3; l++) sg[(l * 4 + q) * 128 + c0 + lane] = gb[l];
+        if (cg == 0) {
+            for (int o = 16; o > 0; o >>= 1) {
+                gb3 += __shfl_down_sync(0xffffffffu, gb3, o);
+                loss += __shfl_down_sync(0xffffffffu, loss, o);
+            }
+            if (lane == 0) { sg[12 * 128 + q] = gb3; sg[12 * 128 + 4 + q] = loss; }
+        }
+        __syncthreads();
+        if (tid < 3 * 128) {
+            const float *p = sg + (tid >> 7) * 4 * 128 + (tid & 127);
+            out[kTrPb + tid] = ((p[0] + p[128]) + p[256]) + p[384];
+        } else if (tid < 3 * 128 + 2) {
+            const float *p = sg + 12 * 128 + 4 * (tid - 3 * 128);
+            out[kTrPb + tid] = ((p[0] + p[1]) + p[2]) + p[3];
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    if (warp == 0)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem), "r"(kTrCols) : "memory");
+}
+
+// Gradients and loss from the CTAs' partial sums.  32 consecutive outputs per block, 8 slices of the
+// CTAs each: a slice adds its partials in CTA order, the slices are added in order.
+struct TrainOut {
+    float *gW[4], *gb[4], *loss;
+    int parts, valid;
+};
+constexpr int kTrOutW3 = kTrPW3, kTrOutB = kTrOutW3 + 128 * 64, kTrOutN = kTrOutB + 3 * 128 + 64 + 1;
+constexpr int kTrSlices = 8;
+__global__ void __launch_bounds__(32 * kTrSlices) k_train_reduce(const float *__restrict__ ws, TrainOut o) {
+    const int e = blockIdx.x * 32 + (threadIdx.x & 31), sl = threadIdx.x >> 5;
+    // output e: gW0 gW1 gW2 as in the partials, gW3 [128][64] (column 0 real), gb0 gb1 gb2, gb3 [64], loss
+    int src = -1;
+    if (e < kTrOutW3) src = e;
+    else if (e < kTrOutB) src = ((e - kTrOutW3) & 63) == 0 ? kTrPW3 + ((e - kTrOutW3) >> 6) : -1;
+    else if (e < kTrOutB + 3 * 128 + 1) src = kTrPb + (e - kTrOutB);
+    else if (e == kTrOutN - 1) src = kTrPb + 3 * 128 + 1;
+    const int per = (o.parts + kTrSlices - 1) / kTrSlices, p0 = sl * per, p1 = min(o.parts, p0 + per);
+    float x = 0.f;
+    if (src >= 0)
+#pragma unroll 8
+        for (int p = p0; p < p1; p++) x += ws[(size_t)p * kTrPart + src];
+    __shared__ float s[kTrSlices][32];
+    s[sl][threadIdx.x & 31] = x;
+    __syncthreads();
+    if (sl != 0 || e >= kTrOutN) return;
+    for (int k = 1; k < kTrSlices; k++) x += s[k][threadIdx.x];
+    if (e < kTrPW1) o.gW[0][e - kTrPW0] = x;
+    else if (e < kTrPW2) o.gW[1][e - kTrPW1] = x;
+    else if (e < kTrOutW3) o.gW[2][e - kTrPW2] = x;
+    else if (e < kTrOutB) o.gW[3][e - kTrOutW3] = x;
+    else if (e < kTrOutB + 3 * 128) o.gb[(e - kTrOutB) >> 7][(e - kTrOutB) & 127] = x;
+    else if (e < kTrOutN - 1) o.gb[3][e - kTrOutB - 3 * 128] = x;
+    else *o.loss = x / (float)o.valid;
+}
+
 }  // namespace
 
 extern "C" {
@@ -1149,10 +1537,75 @@ int cmf_emu_colsum(int rows, int cols, const float *X, float *out, void *stream)
     return CMF_OK;
 }
 
+int cmf_emu_adam_set(int count, const int32_t *n, float *const *w, void *const *wb, const float *const *grad, float *const *m,
+                     float *const *v, const float *wd, float lr, float b1, float b2, float eps, int step, void *stream) {
+    if (count < 1 || count > kAdamMax || !n || !w || !wb || !grad || !m || !v || !wd)
+        return emu_err(CMF_E_ARG, "cmf_emu_adam_set: 1 to 8 tensors");
+    AdamSet a{};
+    int most = 0;
+    for (int k = 0; k < count; k++) {
+        a.n[k] = n[k]; a.w[k] = w[k]; a.wb[k] = (__nv_bfloat16 *)wb[k]; a.grad[k] = grad[k];
+        a.m[k] = m[k]; a.v[k] = v[k]; a.wd[k] = wd[k];
+        if (n[k] > most) most = n[k];
+    }
+    const float bc1 = 1.f - powf(b1, (float)step), bc2 = 1.f - powf(b2, (float)step);
+    k_adam<<<dim3((most + 255) / 256, count), 256, 0, (cudaStream_t)stream>>>(a, lr, b1, b2, eps, bc1, bc2);
+    EMU_TRY(cudaGetLastError());
+    return CMF_OK;
+}
+
 int cmf_emu_adam(int n, float *w, void *wb, const float *grad, float *m, float *v, float lr, float b1, float b2, float eps,
                  int step, float wd, void *stream) {
-    const float bc1 = 1.f - powf(b1, (float)step), bc2 = 1.f - powf(b2, (float)step);
-    k_adam<<<(n + 255) / 256, 256, 0, (cudaStream_t)stream>>>(n, w, (__nv_bfloat16 *)wb, grad, m, v, lr, b1, b2, eps, bc1, bc2, wd);
+    const int32_t nn = n;
+    return cmf_emu_adam_set(1, &nn, &w, &wb, &grad, &m, &v, &wd, lr, b1, b2, eps, step, stream);
+}
+
+size_t cmf_emu_loss_grad_ws_floats(int rows) {
+    if (rows <= 0) return 0;
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+        return 0;
+    const int ntiles = (rows + 127) / 128;
+    return (size_t)(ntiles < sms ? ntiles : sms) * kTrPart;
+}
+
+int cmf_emu_loss_grad(int rows, int valid, const void *X, const float *t, const void *const *W, const float *const *b,
+                      float *const *gW, float *const *gb, float *loss, float *workspace, size_t workspace_floats,
+                      void *stream) {
+    if (rows <= 0 || rows % 64 || !X || !t || !W || !b || !gW || !gb || !loss || !workspace)
+        return emu_err(CMF_E_ARG, "cmf_emu_loss_grad: null argument, or rows not a multiple of 64");
+    TrainArgs a{};
+    TrainOut o{};
+    uintptr_t align = (uintptr_t)X;
+    for (int l = 0; l < 4; l++) {
+        if (!W[l] || !b[l] || !gW[l] || !gb[l]) return emu_err(CMF_E_ARG, "cmf_emu_loss_grad: null parameter tensor");
+        a.W[l] = (const __nv_bfloat16 *)W[l];
+        a.b[l] = b[l];
+        o.gW[l] = gW[l];
+        o.gb[l] = gb[l];
+        align |= (uintptr_t)W[l];
+    }
+    if (align & 15) return emu_err(CMF_E_ARG, "cmf_emu_loss_grad: X and the weights must be 16-byte aligned");
+    int dev = 0, major = 0, sms = 0;
+    EMU_TRY(cudaGetDevice(&dev));
+    EMU_TRY(cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, dev));
+    if (major != 10) return emu_err(CMF_E_NO_DEVICE, "cmf_emu_loss_grad: needs an sm_100 device");
+    EMU_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    const int ntiles = (rows + 127) / 128, grid = ntiles < sms ? ntiles : sms;
+    if (workspace_floats < (size_t)grid * kTrPart)
+        return emu_err(CMF_E_ARG, "cmf_emu_loss_grad: workspace smaller than cmf_emu_loss_grad_ws_floats()");
+    a.X = (const __nv_bfloat16 *)X;
+    a.t = t;
+    a.rows = rows;
+    a.valid = valid;
+    a.ws = workspace;
+    o.loss = loss;
+    o.parts = grid;
+    o.valid = valid;
+    EMU_TRY(cudaFuncSetAttribute(k_train, cudaFuncAttributeMaxDynamicSharedMemorySize, kTrSmem));
+    k_train<<<grid, kTrThreads, kTrSmem, (cudaStream_t)stream>>>(a, g_tc_wait_limit);
+    EMU_TRY(cudaGetLastError());
+    k_train_reduce<<<(kTrOutN + 31) / 32, 32 * kTrSlices, 0, (cudaStream_t)stream>>>(workspace, o);
     EMU_TRY(cudaGetLastError());
     return CMF_OK;
 }

@@ -393,6 +393,21 @@ int cmf_emu_mse_grad(int rows, int valid, int ldy, const float *Y, const float *
                      float *loss_part, void *stream);
 int cmf_emu_adam(int n, float *w, void *wb, const float *grad, float *m, float *v, float lr, float b1, float b2,
                  float eps, int step, float wd, void *stream);
+/* The same update of up to 8 tensors in one launch (wb[k] may be NULL: no bf16 copy). */
+int cmf_emu_adam_set(int count, const int32_t *n, float *const *w, void *const *wb, const float *const *grad,
+                     float *const *m, float *const *v, const float *wd, float lr, float b1, float b2, float eps,
+                     int step, void *stream);
+/* Loss and parameter gradients of the 4-layer MLP in one pass over the rows on the tcgen05 tensor
+ * cores: X [rows][64] bf16 and W[0..3] bf16 ([64][128], [128][128], [128][128], [128][64]; output
+ * column 0) row-major and 16-byte aligned, b[0..3] and t fp32, rows % 64 == 0.  Writes gW[0..3],
+ * gb[0..3] (fp32, every element) and *loss = sum over the first `valid` rows of (y - t)^2 / valid,
+ * with the rounding points of the layer-by-layer chain and the same bits on every run.
+ * workspace: cmf_emu_loss_grad_ws_floats(rows) floats.  The three arrays of pointers are host
+ * arrays.  A launch that gives up a bounded MMA wait reports through cmf_emu_mlp_tc_status. */
+size_t cmf_emu_loss_grad_ws_floats(int rows);
+int cmf_emu_loss_grad(int rows, int valid, const void *X, const float *t, const void *const *W, const float *const *b,
+                      float *const *gW, float *const *gb, float *loss, float *workspace, size_t workspace_floats,
+                      void *stream);
 /* 14 local features + 2 channels x `hops` (<= 8) upstream messages + 2 Manning estimates -> the
  * first 32 columns of X rows (bf16, ldx % 8 == 0, X 16-byte aligned), for nmembers members whose
  * state arrays start at the member-0 views in mb (member-major [M][N]); member m's rows start at

@@ -467,3 +467,81 @@ def test_snapshot_cells_uniform_and_weighted():
         hits[idx] += 1
     light = hits[np.r_[20:100, 200:N]] / 200.0
     assert abs(light.mean() - (k - 20) / (N - 120)) < 0.005
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows,valid", [(64, 64), (64, 1), (192, 130), (128 * 148, 128 * 148), (128 * 149 + 64, 128 * 149 + 3),
+                                        (128 * 300, 38000)])
+def test_fused_training_step_matches_layerwise_chain(rows, valid):
+    """The one-pass loss and gradients against the layer-by-layer kernels (forward, mse_grad, backward):
+    the same rounding points, sums of `rows` fp32 products in another order.  The bound is the fp32
+    rounding of a sum over the rows: its terms' absolute sum times rows * 2^-24 covers any order."""
+    import torch
+
+    from cmf_b200.emulator import MLP, OUT, _emu_lib, echeck
+
+    dev = torch.device("cuda", 0)
+    rng = np.random.default_rng(rows)
+    mlp = MLP(dev, seed=4)
+    W, b = _rand_params(rng, 0.15)
+    mlp.load({"W": W, "b": b})
+    X = torch.tensor(rng.standard_normal((rows, 64)), device=dev).to(torch.bfloat16)     # every input column in use
+    t = torch.tensor(rng.standard_normal(rows).astype(np.float32), device=dev)
+    loss = mlp.loss_and_grad(X, t, valid)
+    got = [g.clone() for g in mlp.gW + mlp.gb]
+    again = mlp.loss_and_grad(X, t, valid)
+    assert torch.equal(loss, again) and all(torch.equal(x, y) for x, y in zip(got, mlp.gW + mlp.gb))
+    Y, acts = mlp.forward(X)
+    dY = torch.empty(rows, OUT, device=dev)
+    dYb = torch.empty(rows, OUT, dtype=torch.bfloat16, device=dev)
+    parts = torch.empty((rows + 255) // 256, device=dev)
+    echeck(mlp.lib.cmf_emu_mse_grad(rows, valid, OUT, Y.data_ptr(), t.data_ptr(), dY.data_ptr(), dYb.data_ptr(),
+                                    parts.data_ptr(), mlp.stream), "mse_grad")
+    mlp.backward(acts, dY, dYb)
+    torch.cuda.synchronize()
+    assert _emu_lib().cmf_emu_mlp_tc_status() == 0
+    eps = 2.0 ** -24
+    ref = float(parts.double().sum() / valid)
+    assert abs(float(loss) - ref) <= rows * eps * ref
+    # absolute sums of the products behind each gradient, from the chain's own activations and dZ
+    dZ, mags = dYb.double(), [None] * 8
+    for li in (3, 2, 1, 0):
+        a = acts[li].double()
+        mags[li] = a.abs().T @ dZ.abs()
+        mags[4 + li] = dZ.abs().sum(0) * (1 + 2.0 ** -8)
+        if li:
+            dA = dZ @ mlp.Wb[li].double().T
+            dZ = torch.where(a > 0, dA, 0.0).to(torch.bfloat16).double()
+    for k, (g, r, mag) in enumerate(zip(got, mlp.gW + mlp.gb, mags)):
+        # 2^-8: a dZ recomputed here in 64 bits may round to the neighbouring bf16 value
+        bound = 2.0 * rows * eps * mag * (1 + 2.0 ** -7)
+        assert bool(((g - r).double().abs() <= bound).all()), (k, float(((g - r).double().abs() - bound).max()))
+
+
+@pytest.mark.gpu
+def test_fused_training_step_bounded_wait_reports():
+    """With a wait bound of 0 the training launch gives up, drains its products, reports once, and the
+    next step with the default bound is correct again."""
+    import torch
+
+    from cmf_b200.emulator import MLP, _emu_lib
+
+    lib, dev = _emu_lib(), torch.device("cuda", 0)
+    mlp = MLP(dev, seed=5)
+    X = torch.zeros(4096, 64, dtype=torch.bfloat16, device=dev)
+    X[:, :32] = torch.randn(4096, 32, device=dev, generator=torch.Generator(device=dev).manual_seed(1)).to(torch.bfloat16)
+    t = torch.ones(4096, device=dev)
+    ref = mlp.loss_and_grad(X, t, 4096)
+    torch.cuda.synchronize()
+    assert lib.cmf_emu_mlp_tc_status() == 0
+    try:
+        assert lib.cmf_emu_mlp_tc_set_wait_limit(0) == 0
+        mlp.loss_and_grad(X, t, 4096)
+        torch.cuda.synchronize()
+        assert lib.cmf_emu_mlp_tc_status() == 1
+    finally:
+        lib.cmf_emu_mlp_tc_set_wait_limit(-1)
+    again = mlp.loss_and_grad(X, t, 4096)
+    torch.cuda.synchronize()
+    assert lib.cmf_emu_mlp_tc_status() == 0
+    assert torch.equal(ref, again)
