@@ -20,7 +20,7 @@ LIB = os.path.join(LIBDIR, "libcmf_b200.so")
 INCLUDE = os.path.join(os.path.dirname(HERE), "include")
 
 SOURCES = ["cmf_engine.cu", "cmf_emu.cu", "cmf_host.cpp"]
-HEADERS = ["cmf_kernels.cuh"]
+HEADERS = ["cmf_kernels.cuh", "cmf_persist.cuh", "cmf_resident.cuh"]
 SYNTH_LIB = os.path.join(LIBDIR, "libcmf_synth.so")
 SYNTH_SOURCE = "cmf_synth.cpp"
 # the generator's loops must round like numpy's element-wise operations: no contraction

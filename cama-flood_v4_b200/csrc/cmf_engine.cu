@@ -9,6 +9,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cmath>
 #include <chrono>
 #include <map>
 #include <mutex>
@@ -21,6 +22,7 @@
 #include "../../include/cmf_gpu.h"
 #include "cmf_kernels.cuh"
 #include "cmf_persist.cuh"
+#include "cmf_resident.cuh"
 
 namespace {
 
@@ -82,6 +84,8 @@ struct cmf_gpu_ctx {
     std::vector<void *> allocs;
     Sched sched;                // the launch schedule of the outer step
     int persist_grid = 0;       // co-resident CTAs of the persistent kernel (0: it cannot run here)
+    cmf::ResArgs res{};         // its resident form (group 0: a member does not fit the SMs)
+    int res_threads = 0;
     bool l2_window = false;     // the hot maps sit under a persisting L2 access-policy window
     bool persist = false;       // outer steps run as one persistent cooperative launch
     Tuner tune;                 // online autotuner state
@@ -215,6 +219,11 @@ int build_net(cmf_gpu_ctx *c, const cmf_map_ptrs *mp) {
         up_ptr[i + 1] = (int)up_idx.size();
     }
     c->E = up_idx.size();
+    std::vector<int> xpos(N, -1);
+    int degmax = 0;
+    for (size_t k = 0; k < up_idx.size(); k++) xpos[up_idx[k]] = (int)k;
+    for (int i = 0; i < N; i++) degmax = std::max(degmax, up_ptr[i + 1] - up_ptr[i]);
+    c->res.edges = degmax < (1 << (32 - cmf::kResDegShift)) && c->E < (size_t(1) << cmf::kResDegShift) ? (int)c->E : -1;
     constexpr int S = cmf::kUpSlots;
     std::vector<int> up_ell((size_t)S * N, -1);
     for (int i = 0; i < N; i++) {
@@ -224,7 +233,7 @@ int build_net(cmf_gpu_ctx *c, const cmf_map_ptrs *mp) {
     }
     int rc;
     if ((rc = c->upload(&n.next, next)) || (rc = c->upload(&n.up_ptr, up_ptr)) || (rc = c->upload(&n.up_idx, up_idx)) ||
-        (rc = c->upload(&n.up_ell, up_ell)))
+        (rc = c->upload(&n.up_ell, up_ell)) || (rc = c->upload(&c->res.xpos, xpos)))
         return rc;
     std::vector<int> i2mask(mp->i2mask, mp->i2mask + N);
     if ((rc = c->upload(&n.i2mask, i2mask))) return rc;
@@ -265,13 +274,17 @@ int build_net(cmf_gpu_ctx *c, const cmf_map_ptrs *mp) {
     } else {
         if ((rc = c->upload(&n.fldhgt, std::vector<double>(1, 0.0)))) return rc;
     }
+    std::vector<int> h_po_ptr(N + 1, 0), h_pi_ptr(N + 1, 0), h_i1dam(N, 0), h_dam_id(N, -1), h_lev_id(N, -1), h_pu, h_pd, h_skip;
     // ---- bifurcation paths
     {
         const int P = n.P, Lp = n.Lp;
-        std::vector<int> pu(std::max(P, 1), -1), pd(std::max(P, 1), -1), skip(std::max(P, 1), 3);
+        std::vector<int> &pu = h_pu, &pd = h_pd, &skip = h_skip;
+        pu.assign(std::max(P, 1), -1);
+        pd.assign(std::max(P, 1), -1);
+        skip.assign(std::max(P, 1), 3);
         std::vector<double> dst(std::max(P, 1), 1.0), elv((size_t)std::max(P * Lp, 1), 0.0), wth(elv.size(), 1.0),
             man(std::max(Lp, 1), 0.0);
-        std::vector<int> po_ptr(N + 1, 0), po_idx, pi_ptr(N + 1, 0), pi_idx;
+        std::vector<int> &po_ptr = h_po_ptr, &pi_ptr = h_pi_ptr, po_idx, pi_idx;
         if (P > 0) {
             if (Lp > 64) return set_err(CMF_E_UNSUPPORTED, "NPTHLEV above 64");
             for (int p = 0; p < P; p++) {
@@ -301,17 +314,31 @@ int build_net(cmf_gpu_ctx *c, const cmf_map_ptrs *mp) {
             for (int p : po_idx) if (p < 0 || p >= P) return set_err(CMF_E_ARG, "I1P_OUT out of range");
             for (int p : pi_idx) if (p < 0 || p >= P) return set_err(CMF_E_ARG, "I1P_INF out of range");
         }
-        if (po_idx.empty()) po_idx.push_back(0);
-        if (pi_idx.empty()) pi_idx.push_back(0);
-        if ((rc = c->upload(&n.pth_up, pu)) || (rc = c->upload(&n.pth_dn, pd)) || (rc = c->upload(&n.pth_skip, skip)) ||
-            (rc = c->upload(&n.pth_dst, dst)) || (rc = c->upload(&n.pth_elv, elv)) || (rc = c->upload(&n.pth_wth, wth)) ||
-            (rc = c->upload(&n.pth_man, man)) || (rc = c->upload(&n.pout_ptr, po_ptr)) || (rc = c->upload(&n.pout_idx, po_idx)) ||
-            (rc = c->upload(&n.pinf_ptr, pi_ptr)) || (rc = c->upload(&n.pinf_idx, pi_idx)))
+        // the ends of paths by cell (Net::pend)
+        std::vector<int> pos(N, -1), ptr(1, 0);
+        std::vector<int2> ends;
+        for (int i = 0; i < N; i++) {
+            if (po_ptr[i + 1] == po_ptr[i] && pi_ptr[i + 1] == pi_ptr[i]) continue;
+            pos[i] = (int)ptr.size() - 1;
+            for (int e = po_ptr[i]; e < po_ptr[i + 1]; e++) {
+                const int p = po_idx[e];
+                ends.push_back(make_int2(p, skip[p] & 1 ? -1 : pu[p] == i ? pd[p] : -2));
+            }
+            for (int e = pi_ptr[i]; e < pi_ptr[i + 1]; e++) {
+                const int p = pi_idx[e];
+                ends.push_back(make_int2(~p, skip[p] & 1 ? -1 : pd[p] == i ? pu[p] : -2));
+            }
+            ptr.push_back((int)ends.size());
+        }
+        if ((rc = c->upload(&n.path_pos, pos)) || (rc = c->upload(&n.pend_ptr, ptr)) || (rc = c->upload(&n.pend, ends))) return rc;
+        if ((rc = c->upload(&n.pth_up, pu)) || (rc = c->upload(&n.pth_dn, pd)) || (rc = c->upload(&n.pth_dst, dst)) || (rc = c->upload(&n.pth_elv, elv)) || (rc = c->upload(&n.pth_wth, wth)) ||
+            (rc = c->upload(&n.pth_man, man)))
             return rc;
+        CUDA_TRY(cudaStreamSynchronize(c->stream));
     }
     // ---- levee: compact the cells that do not carry the no-levee sentinels
     {
-        std::vector<int> lev_id(N, -1);
+        std::vector<int> &lev_id = h_lev_id;
         std::vector<double> lh, lf, bh, ld, lb, lt, lfl;
         if (c->opts.llevee) {
             if (!mp->levhgt || !mp->levfrc || !mp->bashgt || !mp->levdst || !mp->levbassto || !mp->levtopsto || !mp->levfilsto)
@@ -335,7 +362,7 @@ int build_net(cmf_gpu_ctx *c, const cmf_map_ptrs *mp) {
     }
     // ---- dams
     {
-        std::vector<int> i1dam(N, 0), dam_id(N, -1), stat;
+        std::vector<int> &i1dam = h_i1dam, &dam_id = h_dam_id, stat;
         std::vector<double> qn, qf, qa, con, eme, nor, adj, rvu;
         if (c->opts.ldamout) {
             if (!mp->damseq || !mp->damstat || !mp->i1dam) return set_err(CMF_E_ARG, "dam table pointer missing");
@@ -362,6 +389,63 @@ int build_net(cmf_gpu_ctx *c, const cmf_map_ptrs *mp) {
             (rc = c->upload(&n.convol, con)) || (rc = c->upload(&n.emevol, eme)) || (rc = c->upload(&n.norvol, nor)) ||
             (rc = c->upload(&n.adjvol, adj)) || (rc = c->upload(&n.r_volupa, rvu)))
             return rc;
+    }
+    // ---- what each cell takes part in, the dam cells, and the resident kernel's order of cells: dam
+    // cells, other ends of paths, the rest, each class ascending
+    {
+        std::vector<unsigned char> fl(N, 0);
+        std::vector<int> dams, rules, order, pos(N, -1), dup_ptr, dup_idx;
+        std::vector<double> vel, velf;
+        for (int i = 0; i < N; i++) {
+            unsigned f = 0;
+            if (h_i1dam[i] > 0) f |= cmf::C_DAM | (h_i1dam[i] == 10 && i < R ? cmf::C_KIN : 0);
+            if (h_dam_id[i] >= 0) f |= cmf::C_DAMID;
+            if (h_po_ptr[i + 1] > h_po_ptr[i] || h_pi_ptr[i + 1] > h_pi_ptr[i]) f |= cmf::C_PATH;
+            if (h_lev_id[i] >= 0) f |= cmf::C_LEV;
+            fl[i] = (unsigned char)f;
+            if (f & cmf::C_DAM) (f & cmf::C_KIN ? dams : rules).push_back(i);
+        }
+        dams.insert(dams.end(), rules.begin(), rules.end());
+        n.ndam_cells = (int)dams.size();
+        dup_ptr.push_back(0);
+        for (size_t q = 0; q < dams.size(); q++) {
+            const int i = dams[q];
+            pos[i] = (int)q;
+            if (h_dam_id[i] >= 0)
+                for (int e = up_ptr[i]; e < up_ptr[i + 1]; e++)
+                    if (h_i1dam[up_idx[e]] == 10 || h_i1dam[up_idx[e]] == 11) dup_idx.push_back(up_idx[e]);
+            dup_ptr.push_back((int)dup_idx.size());
+            // UPDATE_INFLOW 1c (src/cmf_ctrl_damout_mod.F90): (1/n) * slope**0.5, correctly rounded as on the device
+            double v = 0.0, vf = 0.0;
+            if (fl[i] & cmf::C_KIN) {
+                double slope = (mp->elevtn[i] - mp->elevtn[next[i]]) * (1.0 / mp->nxtdst[i]);
+                slope = slope > n.pminslp ? slope : n.pminslp;
+                v = (1.0 / mp->rivman[i]) * std::sqrt(slope);
+                vf = (1.0 / n.pmanfld) * std::sqrt(0.005 < slope ? 0.005 : slope);
+            }
+            vel.push_back(v);
+            velf.push_back(vf);
+        }
+        // the two kinds of dam cells in tiles of their own (-1: no cell): one warp would walk both rules
+        const size_t nkin = dams.size() - rules.size();
+        order.assign(dams.begin(), dams.begin() + nkin);
+        while (nkin && order.size() % 32) order.push_back(-1);
+        order.insert(order.end(), rules.begin(), rules.end());
+        for (int i = 0; i < N; i++) if ((fl[i] & cmf::C_PATH) && !(fl[i] & cmf::C_DAM)) order.push_back(i);
+        for (int i = 0; i < N; i++) if (!(fl[i] & (cmf::C_PATH | cmf::C_DAM))) order.push_back(i);
+        if ((rc = c->upload(&n.cflag, fl)) || (rc = c->upload(&n.dam_cells, dams)) || (rc = c->upload(&n.dam_pos, pos)) ||
+            (rc = c->upload(&n.dam_up_ptr, dup_ptr)) || (rc = c->upload(&n.dam_up_idx, dup_idx)) ||
+            (rc = c->upload(&n.kin_vel, vel)) || (rc = c->upload(&n.kin_velf, velf)) || (rc = c->upload(&c->res.order, order)))
+            return rc;
+        c->res.cells = (int)order.size();
+        // levees at the ends of paths
+        for (int p = 0; p < n.P; p++) {
+            const int e[2] = {h_pu[p], h_pd[p]};
+            for (int k = 0; k < 2; k++)
+                if (e[k] >= 0 && h_lev_id[e[k]] >= 0 && mp->levfrc[e[k]] < 1.0) h_skip[p] |= 4 << k;
+        }
+        if ((rc = c->upload(&n.pth_skip, h_skip))) return rc;
+        CUDA_TRY(cudaStreamSynchronize(c->stream));
     }
     return CMF_OK;
 }
@@ -396,8 +480,7 @@ int hot_maps_window(cmf_gpu_ctx *c) {
         {(const void **)&n.inv_rivwth, N * 8}, {(const void **)&n.inv_rivlen, N * 8},
         {(const void **)&n.next, N * 4}, {(const void **)&n.up_ptr, (N + 1) * 4}, {(const void **)&n.up_idx, c->E * 4},
         {(const void **)&n.up_ell, N * 4 * cmf::kUpSlots},
-        {(const void **)&n.i1dam, N * 4}, {(const void **)&n.dam_id, N * 4}, {(const void **)&n.lev_id, N * 4},
-        {(const void **)&n.pout_ptr, (N + 1) * 4}, {(const void **)&n.pinf_ptr, (N + 1) * 4}};
+        {(const void **)&n.cflag, N}};
     size_t total = 0;
     for (const Item &it : items) total += (it.bytes + 255) & ~(size_t)255;
     int max_persist = 0, max_win = 0;
@@ -489,15 +572,15 @@ int alloc_state(cmf_gpu_ctx *c) {
 }
 
 // phase A and phase C in the schedule's occupancy profile; grids cover the cells of every member,
-// then (phases A and C) the bifurcation paths
+// then the bifurcation paths, then (phase A) the dam cells
 void launch_flux(cmf_gpu_ctx *c) {
     const Sched &q = c->sched;
-    const int nc = nblk(c->dims.nseqall, q.bf);
-    const dim3 g(nc + nblk(c->net.P, q.bf), c->dims.nmembers);
+    const int nc = nblk(c->dims.nseqall, q.bf), np = nblk(cmf::path_threads(c->net.P, c->net.Lp), q.bf);
+    const dim3 g(nc + np + nblk(c->net.ndam_cells, q.bf), c->dims.nmembers);
     if (q.prof)
-        cmf::k_flux<cmf::kFluxMinBlocksSmall><<<g, q.bf, 0, c->stream>>>(c->net, c->st, nc);
+        cmf::k_flux<cmf::kFluxMinBlocksSmall><<<g, q.bf, 0, c->stream>>>(c->net, c->st, nc, np);
     else
-        cmf::k_flux<cmf::kFluxMinBlocksWide><<<g, q.bf, 0, c->stream>>>(c->net, c->st, nc);
+        cmf::k_flux<cmf::kFluxMinBlocksWide><<<g, q.bf, 0, c->stream>>>(c->net, c->st, nc, np);
 }
 void launch_rate(cmf_gpu_ctx *c, int advance, cudaGraphConditionalHandle cond, int use_cond) {
     const dim3 g(nblk(c->dims.nseqall, c->sched.br), c->dims.nmembers);
@@ -506,7 +589,7 @@ void launch_rate(cmf_gpu_ctx *c, int advance, cudaGraphConditionalHandle cond, i
 void launch_store(cmf_gpu_ctx *c) {
     const Sched &q = c->sched;
     const int nc = nblk(c->dims.nseqall, q.bs);
-    const dim3 g(nc + nblk(c->net.P, q.bs), c->dims.nmembers);
+    const dim3 g(nc + nblk(cmf::path_threads(c->net.P, c->net.Lp), q.bs), c->dims.nmembers);
     if (q.prof)
         cmf::k_store<cmf::kStoreMinBlocksSmall><<<g, q.bs, cmf::store_smem(q.bs), c->stream>>>(c->net, c->st, nc);
     else
@@ -593,32 +676,68 @@ int sync_dt_def(cmf_gpu_ctx *c, double dt_def) {
 }
 
 // ---- persistent schedule: one cooperative launch per outer step --------------------------------
+// The persistent schedule runs the resident kernel when one member's cells fit the SMs (one CTA per SM
+// with kResMaxSlots tiles), and k_persist for larger members.  Members are grouped evenly over the
+// fewest groups that fit.
 int persist_setup(cmf_gpu_ctx *c) {
-    CUDA_TRY(cudaFuncSetAttribute(cmf::k_persist, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cmf::kPersistSmem));
-    int per_sm = 0, nsm = 0;
-    CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, cmf::k_persist, cmf::kTile, cmf::kPersistSmem));
+    int per_sm = 0, nsm = 0, coop = 0;
     CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->device));
-    int coop = 0;
     CUDA_TRY(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, c->device));
-    c->persist_grid = coop ? per_sm * nsm : 0;
+    if (!coop) return CMF_OK;
+    const long long tpm = (c->res.cells + 31) / 32, M = c->dims.nmembers;
+    const long long fit = std::min({(long long)nsm * cmf::kResMaxSlots / tpm, (long long)cmf::kResMaxGroup, M});
+    if (fit >= 1 && c->res.edges >= 0) {
+        const long long groups = (M + fit - 1) / fit, group = (M + groups - 1) / groups, tiles = group * tpm;
+        cmf::ResArgs &a = c->res;
+        const int grid = (int)std::min<long long>(nsm, tiles);
+        a.slots = (int)((tiles + grid - 1) / grid);
+        // a warp per tile and per path tile, up to the CTA's limit
+        const long long ptiles = group * (cmf::path_threads(c->net.P, c->net.Lp) / 32);
+        const int threads = 32 * (int)std::min<long long>(cmf::kResThreads / 32, a.slots + (ptiles + grid - 1) / grid + 1);
+        CUDA_TRY(cudaFuncSetAttribute(cmf::k_resident, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)cmf::res_smem(cmf::kResMaxSlots)));
+        CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, cmf::k_resident, threads, cmf::res_smem(a.slots)));
+        if (per_sm >= 1) {
+            a.tpm = (int)tpm;
+            a.group = (int)group;
+            a.wait_ns = cmf::kWaitNsDefault;
+            a.selftest = 0;
+            int rc;
+            const size_t gn = (size_t)group * c->res.edges;
+            if ((rc = c->alloc(&a.raw, gn)) || (rc = c->alloc(&a.out, gn)) ||
+                (rc = c->alloc(&a.terms, (size_t)cmf::kBudgets * group * tpm * 32)))
+                return rc;
+            c->persist_grid = grid;
+            c->res_threads = threads;
+            return CMF_OK;
+        }
+    }
+    CUDA_TRY(cudaFuncSetAttribute(cmf::k_persist, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cmf::kPersistSmem));
+    CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, cmf::k_persist, cmf::kTile, cmf::kPersistSmem));
+    c->persist_grid = per_sm * nsm;
     return CMF_OK;
 }
 
-cmf::PersistArgs persist_args(const cmf_gpu_ctx *c) {
-    cmf::PersistArgs a{};
-    a.tpm = (c->dims.nseqall + cmf::kTile - 1) / cmf::kTile;
-    a.ppm = c->net.P > 0 ? (c->net.P + cmf::kTile - 1) / cmf::kTile : 0;
-    a.wait_ns = cmf::kWaitNsDefault;
-    a.selftest = 0;
-    return a;
-}
-
-int launch_persist(cmf_gpu_ctx *c, cmf::PersistArgs a) {
+// one outer step as one cooperative launch; wait_ns > 0: the bounded-wait self-test instead
+int launch_persist(cmf_gpu_ctx *c, unsigned long long selftest_ns = 0) {
     if (c->persist_grid < 1) return set_err(CMF_E_UNSUPPORTED, "the persistent kernel cannot be co-resident on this device");
     CUDA_TRY(cudaMemsetAsync(&c->st.loop->bar, 0, sizeof(unsigned), c->stream));
-    void *args[] = {&c->net, &c->st, &a};
-    CUDA_TRY(cudaLaunchCooperativeKernel((const void *)cmf::k_persist, dim3(c->persist_grid), dim3(cmf::kTile), args,
-                                         cmf::kPersistSmem, c->stream));
+    if (c->res.group > 0) {
+        cmf::ResArgs a = c->res;
+        if (selftest_ns) { a.wait_ns = selftest_ns; a.selftest = 1; }
+        void *args[] = {&c->net, &c->st, &a};
+        CUDA_TRY(cudaLaunchCooperativeKernel((const void *)cmf::k_resident, dim3(c->persist_grid), dim3(c->res_threads), args,
+                                             cmf::res_smem(a.slots), c->stream));
+    } else {
+        cmf::PersistArgs a{};
+        a.tpm = (c->dims.nseqall + cmf::kTile - 1) / cmf::kTile;
+        a.ppm = (cmf::path_threads(c->net.P, c->net.Lp) + cmf::kTile - 1) / cmf::kTile;
+        a.wait_ns = selftest_ns ? selftest_ns : cmf::kWaitNsDefault;
+        a.selftest = selftest_ns != 0;
+        void *args[] = {&c->net, &c->st, &a};
+        CUDA_TRY(cudaLaunchCooperativeKernel((const void *)cmf::k_persist, dim3(c->persist_grid), dim3(cmf::kTile), args,
+                                             cmf::kPersistSmem, c->stream));
+    }
     c->launches += 1;
     return CMF_OK;
 }
@@ -706,7 +825,7 @@ int launch_outer(cmf_gpu_ctx *c) {
     int rc;
     if ((rc = tune_begin(c, trial))) return rc;
     if (c->persist) {
-        if ((rc = launch_persist(c, persist_args(c)))) return rc;
+        if ((rc = launch_persist(c))) return rc;
     } else if (c->opts.launch_mode == 0) {
         CUDA_TRY(cudaGraphLaunch(c->exec, c->stream));
         c->launches += 3;   // prologue and epilogue; the loop body adds 3 per sub-step (counted on read-back)
@@ -1166,10 +1285,7 @@ int cmf_gpu_ctx_persist_selftest(cmf_gpu_ctx *c, int64_t wait_ns) {
     if (!c) return set_err(CMF_E_STATE, "no context");
     if (wait_ns < 1000 || wait_ns > 2000000000LL) return set_err(CMF_E_ARG, "wait_ns must lie in [1 us, 2 s]");
     CUDA_TRY(cudaSetDevice(c->device));
-    cmf::PersistArgs a = persist_args(c);
-    a.wait_ns = (unsigned long long)wait_ns;
-    a.selftest = 1;
-    int rc = launch_persist(c, a);
+    int rc = launch_persist(c, (unsigned long long)wait_ns);
     if (rc) return rc;
     int berr = 0;
     CUDA_TRY(cudaMemcpyAsync(&berr, &c->st.loop->bar_err, sizeof berr, cudaMemcpyDeviceToHost, c->stream));
@@ -1837,8 +1953,9 @@ __global__ void k_noalloc_stage(cmf::Net n, cmf::State s, double *blockmin) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     double key = 1.0e308;
     if (i < n.N) {
-        const cmf::StageOut o = cmf::stage_def(n, cmf::OwnG{n, s}, i, s.rivsto[i], s.fldsto[i]);
-        cmf::store_stage(n, s, i, i, o);
+        const cmf::OwnG w{n, s};
+        const cmf::StageOut o = cmf::stage(n, w, i, cmf::stage_map(w, i), s.rivsto[i], s.fldsto[i], 0.0);
+        cmf::store_stage(n, s, w, i, i, o);
         if (n.ladpstp && n.i2mask[i] == 0)
             key = cmf::cfl_key(n.pcadp, (i < n.R) ? n.nxtdst[i] : n.pdstmth, n.pgrv, o.rivdph);
     }

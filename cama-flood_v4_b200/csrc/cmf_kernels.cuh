@@ -106,9 +106,16 @@ struct Net {
     const double *__restrict__ fldstomax, *__restrict__ fldgrd, *__restrict__ fldhgt;   // [L][N]
     // bifurcation paths
     const int *__restrict__ pth_up, *__restrict__ pth_dn;   // [P] 0-based, -1 outside domain
-    const int *__restrict__ pth_skip;                        // [P] bit0 plain/LSPAMAT skip, bit1 levee skip
+    const int *__restrict__ pth_skip;                        // [P] bit0 plain/LSPAMAT skip, bit1 levee skip, bits 2
+                                                             // and 3: a levee fraction below 1 at the ends
     const double *__restrict__ pth_dst, *__restrict__ pth_elv, *__restrict__ pth_wth, *__restrict__ pth_man;
-    const int *__restrict__ pout_ptr, *__restrict__ pout_idx, *__restrict__ pinf_ptr, *__restrict__ pinf_idx;
+    // the ends of paths: per cell with C_PATH its position (path_pos [N]), per position a range of entries,
+    // the cell's I1P_OUT paths and then its I1P_INF paths, each in list order.  An entry holds the path
+    // (x, ~path for I1P_INF) and the cell at its other end (y; -1: not rescaled, -2: the cell is
+    // not this path's end), so a path's flow and the
+    // rate it may need come one load after the entry.
+    const int *__restrict__ path_pos, *__restrict__ pend_ptr;
+    const int2 *__restrict__ pend;
     // levee (compact per levee cell)
     const int *__restrict__ lev_id;     // [N] -1 when the cell carries the no-levee sentinels
     const double *__restrict__ levhgt, *__restrict__ levfrc, *__restrict__ bashgt, *__restrict__ levdst;
@@ -117,11 +124,28 @@ struct Net {
     const int *__restrict__ i1dam;      // [N]
     const int *__restrict__ dam_id;     // [N] compact dam of the cell or -1
     const int *__restrict__ dam_stat;   // [D]
+    // what a cell takes part in (CellFlag), and the cells of reservoir operation (I1DAM > 0), which run
+    // in warps of their own: one such lane made its whole warp walk the rules' dependent loads and powers
+    const unsigned char *__restrict__ cflag;                 // [N]
+    const int *__restrict__ dam_cells;                       // kinematic cells first, then the dams
+    int ndam_cells;
+    // by position in dam_cells: the cell's position [N], its upstream cells that feed a dam's inflow
+    // (I1DAM 10 or 11, I1UPST order), and the static factors of the kinematic velocities
+    const int *__restrict__ dam_pos, *__restrict__ dam_up_ptr, *__restrict__ dam_up_idx;
+    const double *__restrict__ kin_vel, *__restrict__ kin_velf;
     const double *__restrict__ qn, *__restrict__ qf, *__restrict__ qa, *__restrict__ convol;
     const double *__restrict__ emevol, *__restrict__ norvol, *__restrict__ adjvol, *__restrict__ r_volupa;
     double pgrv, pmanfld, pdstmth, pcadp, pminslp, dfrcinc;
     int ladpstp, lfldout, lpthout, ldamout, llevee, ldamh22, ldiag;
     int ldiag_out;   // CMF_DIAG_AVEMAX_OUTPUT after every outer step, fused into its last sub-step
+};
+
+enum CellFlag : unsigned {
+    C_DAM = 1,                 // I1DAM > 0: outflow by cell_dam
+    C_KIN = 2,                 // I1DAM == 10 on a river cell: kinematic outflow upstream of a dam
+    C_DAMID = 4,               // a dam's storage stands here
+    C_PATH = 8,                // an end of a bifurcation path
+    C_LEV = 16                 // levee parameters
 };
 
 // Per-member state, member-major [M][N] (paths [M][Lp][P] / [M][P]).
@@ -149,18 +173,16 @@ struct State {
 __device__ __forceinline__ double dmax(double a, double b) { return (a > b) ? a : b; }
 __device__ __forceinline__ double dmin(double a, double b) { return (a < b) ? a : b; }
 
-// Own-cell reads of the per-cell code go through an accessor (OwnG: the arrays in global memory,
-// static maps through the read-only path), so that a kernel could stage a cell's own values
-// elsewhere without touching the arithmetic.  Static maps are indexed by the cell i, member state
-// by g = m*N + i; reads of another cell (downstream, upstream, path ends) go to global memory
-// through Net/State.
+// The per-cell code reads and writes a cell through an accessor, so that the same arithmetic runs on
+// arrays in global memory (OwnG, the phase kernels) and on state held on the SM (OwnR, the resident
+// kernel).  Static maps are indexed by the cell i and read through the read-only path, member state
+// by g = m*N + i; `nb` reads a value another cell or path owns.
 #define CMF_OWN_STATIC(name) \
     __device__ __forceinline__ double name(int i) const { return __ldg(&n.name[i]); }
 #define CMF_OWN_STATE(name) \
     __device__ __forceinline__ double name(size_t g) const { return s.name[g]; }
-struct OwnG {
+struct OwnMaps {
     const Net &n;
-    const State &s;
     CMF_OWN_STATIC(rivelv) CMF_OWN_STATIC(elevtn) CMF_OWN_STATIC(nxtdst) CMF_OWN_STATIC(rivwth)
     CMF_OWN_STATIC(rivhgt) CMF_OWN_STATIC(rivlen) CMF_OWN_STATIC(rivman) CMF_OWN_STATIC(grarea)
     CMF_OWN_STATIC(rivstomax) CMF_OWN_STATIC(inv_nxtdst) CMF_OWN_STATIC(inv_rivwth) CMF_OWN_STATIC(inv_rivlen)
@@ -169,17 +191,72 @@ struct OwnG {
     __device__ __forceinline__ int up_hi(int i) const { return __ldg(&n.up_ptr[i + 1]); }
     __device__ __forceinline__ int up_slot(int k, int i) const { return __ldg(&n.up_ell[(size_t)k * n.N + i]); }
     __device__ __forceinline__ int i1dam(int i) const { return __ldg(&n.i1dam[i]); }
+};
+struct DownCell {
+    double rivelv, rivdph, rivdph_pre;
+};
+struct OwnG : OwnMaps {
+    static constexpr bool kResident = false;
+    const State &s;
+    unsigned fl;               // the cell's CellFlag bits
+    __device__ __forceinline__ OwnG(const Net &n_, const State &s_, unsigned fl_ = 0u) : OwnMaps{n_}, s(s_), fl(fl_) {}
+    __device__ __forceinline__ unsigned flags() const { return fl; }
     CMF_OWN_STATE(rivsto) CMF_OWN_STATE(fldsto) CMF_OWN_STATE(levsto) CMF_OWN_STATE(rivdph)
     CMF_OWN_STATE(rivdph_pre) CMF_OWN_STATE(rivout_pre) CMF_OWN_STATE(fldout_pre) CMF_OWN_STATE(fldsto_pre)
     CMF_OWN_STATE(flddph) CMF_OWN_STATE(fldfrc) CMF_OWN_STATE(storge) CMF_OWN_STATE(runoff)
     CMF_OWN_STATE(rivout_raw) CMF_OWN_STATE(fldout_raw) CMF_OWN_STATE(rate)
     CMF_OWN_STATE(a_rivvel) CMF_OWN_STATE(a_rivout) CMF_OWN_STATE(a_fldout) CMF_OWN_STATE(a_outflw)
     CMF_OWN_STATE(a_pthout) CMF_OWN_STATE(m_outflw) CMF_OWN_STATE(m_rivdph) CMF_OWN_STATE(m_storge)
+    __device__ __forceinline__ double nb(const double *p, size_t g) const { return p[g]; }
+    __device__ __forceinline__ DownCell down(size_t base, int j) const {
+        return {__ldg(&n.rivelv[j]), s.rivdph[base + j], s.rivdph_pre[base + j]};
+    }
+    __device__ __forceinline__ void put_raw(size_t g, int, double rout, double fout) const {
+        s.rivout_raw[g] = rout;
+        s.fldout_raw[g] = fout;
+    }
+    __device__ __forceinline__ void put_rate(size_t g, int, double, double, double rate) const { s.rate[g] = rate; }
+    __device__ __forceinline__ void put_a_rivvel(size_t g, double v) const { s.a_rivvel[g] = v; }
+    // CALC_VARS_PRE (src/cmf_ctrl_physics_mod.F90:254-277)
+    __device__ __forceinline__ void put_pre(size_t g, double rout, double fout, double dph, double fld) const {
+        s.rivout_pre[g] = rout;
+        s.fldout_pre[g] = fout;
+        s.rivdph_pre[g] = dph;
+        s.fldsto_pre[g] = fld;
+    }
+    template <class Out>
+    __device__ __forceinline__ void put_stage(size_t g, const Out &o, double storge) const {
+        s.rivsto[g] = o.rivsto;
+        s.fldsto[g] = o.fldsto;
+        s.rivdph[g] = o.rivdph;
+        s.flddph[g] = o.flddph;
+        s.fldfrc[g] = o.fldfrc;
+        if (n.llevee) {
+            s.levsto[g] = o.levsto;
+            s.levdph[g] = o.levdph;
+        }
+        s.storge[g] = storge;
+    }
+    // f(rivout, fldout) before the LSPAMAT rescale of every upstream cell, in I1UPST order: the CSR
+    // walk, since at k_rate's full occupancy the slot table's 16 B per cell cost more than its saved round
+    template <class F>
+    __device__ __forceinline__ void each_raw(size_t base, int i, F f) const {
+        const int u1 = up_hi(i);
+        for (int k = up_lo(i); k < u1; k++) {
+            const int j = __ldg(&n.up_idx[k]);
+            f(s.rivout_raw[base + j], s.fldout_raw[base + j]);
+        }
+    }
+    // f(rivout, fldout) after the rescale (:481-489); next(j) == i, so a reverse flow takes rate_i
+    template <class F>
+    __device__ __forceinline__ void each_out(size_t base, int i, double rate_i, F f) const;
 };
 #undef CMF_OWN_STATIC
 #undef CMF_OWN_STATE
 
-// f(j) for every upstream cell j of cell i, in I1UPST order (the order of every upstream sum)
+// f(j) for every upstream cell j of cell i, in I1UPST order.  The CSR walk past the slots reads four
+// indices at once (D8 networks have at most seven upstream cells), each f follows without another
+// dependent round.
 template <class Own, class F>
 __device__ __forceinline__ void for_each_upstream(const Net &n, const Own &w, int i, F f) {
     int slot[kUpSlots];
@@ -195,10 +272,25 @@ __device__ __forceinline__ void for_each_upstream(const Net &n, const Own &w, in
         f(last);
     } else if (last < -1) {                       // more than kUpSlots upstream cells
         const int k1 = __ldg(&n.up_ptr[i + 1]);
-        for (int k = -2 - last; k < k1; k++) f(__ldg(&n.up_idx[k]));
+        for (int k = -2 - last; k < k1; k += 4) {
+            int j[4];
+#pragma unroll
+            for (int e = 0; e < 4; e++) j[e] = k + e < k1 ? __ldg(&n.up_idx[k + e]) : -1;
+#pragma unroll
+            for (int e = 0; e < 4; e++)
+                if (j[e] >= 0) f(j[e]);
+        }
     }
 }
-
+template <class F>
+__device__ __forceinline__ void OwnG::each_out(size_t base, int i, double rate_i, F f) const {
+    const double *rate_m = s.rate + base;
+    for_each_upstream(n, *this, i, [&](int j) {
+        const double rj = s.rivout_raw[base + j], fj = s.fldout_raw[base + j];
+        const double r = (rj > 0.0) ? rate_m[j] : rate_i;
+        f(rj * r, fj * r);
+    });
+}
 
 // x**(-7._JPRB/3._JPRB) and x**(-4._JPRB/3._JPRB) of the local-inertial flux formulas
 // (src/cmf_calc_outflw_mod.F90:74,106,133,162; src/cmf_calc_pthout_mod.F90:67;
@@ -206,11 +298,13 @@ __device__ __forceinline__ void for_each_upstream(const Net &n, const Own &w, in
 // doubles y nearest -7/3 and -4/3, correctly rounded, for the positive depths these formulas take.
 // The exponent is y = -K/3 + d with d its rounding offset (d = -0x1.5555555555555p-53 for K = 7,
 // +0x1.5555555555555p-54 for K = 4), so x^y = (x^(-1/3))^K * x^d:
-//   c0 = rcbrt(x); one Newton step for the inverse cube root, c = c0 (1 + r/3), r = 1 - x c0^3,
-//     with c0^3 formed exactly by Dekker's FMA products (c carried as a double-double);
+//   c0: single-precision exp2(-log2(x)/3) (a few units of 2^-21) and one step of third order in double,
+//     c0 (1 + r/3 + 2 r^2/9), r = 1 - x c0^3, which leaves a few ulp; then one Newton step for the
+//     inverse cube root, c = c0 (1 + r/3), with c0^3 formed exactly by Dekker's FMA products (c carried
+//     as a double-double, relative error about 2^-100);
 //   c^K in double-double (Dekker products; relative error about 2^-100);
 //   x^d = 1 + d ln x to first order (|d ln x| < 3e-15, so ln x to single precision suffices).
-// The sum is rounded once.  Outside (1e-300, 1e300) the general pow is used.
+// The sum is rounded once.  Outside (1e-30, 1e30) the general pow is used.
 struct DD {
     double hi, lo;
 };
@@ -220,13 +314,16 @@ __device__ __forceinline__ DD dd_mul(DD a, DD b) {
     e = e + (a.hi * b.lo + a.lo * b.hi);
     return {p, e};
 }
+
 template <int K>
 __device__ __forceinline__ double pow_depth(double x) {
     static_assert(K == 7 || K == 4, "exponents -7/3 and -4/3 only");
     constexpr double y = -(double)K / 3.0;
     constexpr double d = (K == 7) ? -0x1.5555555555555p-53 : 0x1.5555555555555p-54;
-    if (!(x > 1e-300 && x < 1e300)) return pow(x, y);
-    const double c0 = rcbrt(x);
+    if (!(x > 1e-30 && x < 1e30)) return pow(x, y);
+    const double s0 = (double)exp2f(__log2f((float)x) * (-1.0f / 3.0f));
+    const double rs = fma(-x, s0 * s0 * s0, 1.0);
+    const double c0 = fma(s0 * rs, fma(rs, 2.0 / 9.0, 1.0 / 3.0), s0);
     const double p2 = c0 * c0, e2 = fma(c0, c0, -p2);
     const double p3 = p2 * c0, e3 = fma(p2, c0, -p3);
     const double t = fma(x, p3, -1.0);
@@ -267,202 +364,165 @@ struct StageOut {
     double rivsto, fldsto, levsto, rivdph, flddph, fldfrc, fldare, levdph;
 };
 
-// CMF_CALC_FLDSTG_DEF body, src/cmf_calc_fldstg_mod.F90:46-97
+// The floodplain layers a storage fills, from the channel up: I full layers (0-based layer in use, L: all),
+// the storage, width and depth below it, and its gradient.  Layers are read two at a time: the scan
+// costs one dependent round per two layers (four at a time spilled in k_store).
+struct Filled {
+    int I;
+    double sfil, wfil, dfil, grd;
+};
+__device__ __forceinline__ Filled fill_layers(const Net &n, int i, double pstoall, double rsm, double wth, double inc) {
+    constexpr int B = 2;
+    const int N = n.N, L = n.L;
+    Filled f{0, rsm, wth, 0.0, 0.0};
+    for (int l0 = 0; l0 < L; l0 += B) {
+        double smax[B], grd[B];
+#pragma unroll
+        for (int e = 0; e < B; e++)
+            if (l0 + e < L) {
+                smax[e] = __ldg(&n.fldstomax[(size_t)(l0 + e) * N + i]);
+                grd[e] = __ldg(&n.fldgrd[(size_t)(l0 + e) * N + i]);
+            }
+#pragma unroll
+        for (int e = 0; e < B; e++) {
+            if (l0 + e >= L) break;
+            if (!(pstoall > smax[e])) {
+                f.I = l0 + e;
+                f.grd = grd[e];
+                return f;
+            }
+            f.sfil = smax[e];
+            f.wfil = f.wfil + inc;
+            f.dfil = f.dfil + grd[e] * inc;
+        }
+    }
+    f.I = L;
+    return f;
+}
+
+// Stage scheme of one cell: CMF_CALC_FLDSTG_DEF (src/cmf_calc_fldstg_mod.F90:46-97), or with levees
+// CMF_LEVEE_FLDSTG (src/cmf_ctrl_levee_mod.F90:301-461).  The default scheme is case 1 of the levee
+// scheme for a cell without a levee, but for the bound of the river storage.
+struct StageMap {
+    double rsm, len, wth;
+};
 template <class Own>
-__device__ __forceinline__ StageOut stage_def(const Net &n, const Own &w, int i, double rivsto, double fldsto) {
+__device__ __forceinline__ StageMap stage_map(const Own &w, int i) { return {w.rivstomax(i), w.rivlen(i), w.rivwth(i)}; }
+template <class Own>
+__device__ __forceinline__ StageOut stage(const Net &n, const Own &w, int i, const StageMap &map, double rivsto, double fldsto,
+                                          double levsto) {
     StageOut o;
     const int N = n.N, L = n.L;
-    const double pstoall = rivsto + fldsto;
-    const double rsm = w.rivstomax(i);
+    const double riv_fld = rivsto + fldsto, pstoall = n.llevee ? riv_fld + levsto : riv_fld;
+    const double rsm = map.rsm, len = map.len, wth = map.wth;
     o.levsto = 0.0;
     o.levdph = 0.0;
-    if (pstoall > rsm) {
-        const double len = w.rivlen(i), wth = w.rivwth(i);
-        const double inc = (w.grarea(i) / len) * n.dfrcinc;
-        int I = 0;   // 0-based layer
-        double sfil = rsm, wfil = wth, dfil = 0.0;
-        while (I < L) {
-            const double smax = __ldg(&n.fldstomax[(size_t)I * N + i]);
-            if (!(pstoall > smax)) break;
-            sfil = smax;
-            wfil = wfil + inc;
-            dfil = dfil + __ldg(&n.fldgrd[(size_t)I * N + i]) * inc;
-            I++;
-        }
-        double wadd;
-        if (I >= L) {
-            wadd = 0.0;
-            o.flddph = dfil + ((pstoall - sfil) / wfil) / len;
-        } else {
-            const double gr = __ldg(&n.fldgrd[(size_t)I * N + i]);
-            const double sadd = pstoall - sfil;
-            wadd = -wfil + sqrt(wfil * wfil + ((2.0 * sadd) / len) / gr);
-            o.flddph = dfil + gr * wadd;
-        }
-        double rs = rsm + (len * wth) * o.flddph;
-        rs = dmin(rs, pstoall);
-        o.rivsto = rs;
-        o.rivdph = (rs / len) / wth;
-        o.fldsto = dmax(pstoall - rs, 0.0);
-        double frc = ((-wth + wfil) + wadd) / (inc * (double)L);
-        frc = dmax(frc, 0.0);
-        frc = dmin(frc, 1.0);
-        o.fldfrc = frc;
-        o.fldare = w.grarea(i) * frc;
-    } else {
+    if (!(pstoall > rsm)) {                                                         // case 0
         o.rivsto = pstoall;
-        o.rivdph = dmax((pstoall / w.rivlen(i)) / w.rivwth(i), 0.0);
+        o.rivdph = dmax((pstoall / len) / wth, 0.0);
         o.fldsto = 0.0;
         o.flddph = 0.0;
         o.fldfrc = 0.0;
         o.fldare = 0.0;
+        return o;
     }
-    return o;
-}
-
-// CMF_LEVEE_FLDSTG body, src/cmf_ctrl_levee_mod.F90:301-461
-template <class Own>
-__device__ __forceinline__ StageOut stage_levee(const Net &n, const Own &w, int i, double rivsto, double fldsto,
-                                                double levsto) {
-    StageOut o;
-    const int N = n.N, L = n.L;
-    const double pstoall = (rivsto + fldsto) + levsto;
-    const double rsm = w.rivstomax(i);
-    const double len = w.rivlen(i), wth = w.rivwth(i);
-    const double inc = (w.grarea(i) / len) * n.dfrcinc;
+    // read by out-of-bank cells only: the levee parameters and the layer width's quotient
+    const int lv = (n.llevee && (w.flags() & C_LEV)) ? __ldg(&n.lev_id[i]) : -1;
     const double grarea = w.grarea(i);
-    const int lv = __ldg(&n.lev_id[i]);
-    const double lbas = lv >= 0 ? __ldg(&n.levbassto[lv]) : 1.E18;
-    if (pstoall > rsm) {
-        if (pstoall < lbas) {                                                       // case 1
-            int I = 0;
-            double sfil = rsm, wfil = wth, dfil = 0.0, wadd;
-            while (I < L) {
-                const double smax = __ldg(&n.fldstomax[(size_t)I * N + i]);
-                if (!(pstoall > smax)) break;
-                sfil = smax; wfil = wfil + inc; dfil = dfil + __ldg(&n.fldgrd[(size_t)I * N + i]) * inc;
-                I++;
-            }
-            if (I < L) {
-                const double gr = __ldg(&n.fldgrd[(size_t)I * N + i]);
-                wadd = -wfil + sqrt(wfil * wfil + ((2.0 * (pstoall - sfil)) / len) / gr);
-                o.flddph = dfil + gr * wadd;
-            } else {
-                wadd = 0.0;
-                o.flddph = dfil + ((pstoall - sfil) / wfil) / len;
-            }
-            o.rivsto = rsm + (len * wth) * o.flddph;
-            o.rivdph = (o.rivsto / len) / wth;
+    const double inc = (grarea / len) * n.dfrcinc;
+    double lhgt = 0.0, lfrc = 0.0, bhgt = 0.0, ldst = 0.0, ltop = 0.0, lfil = 0.0;
+    int lcase = 1;
+    if (lv >= 0) {
+        const double lbas = __ldg(&n.levbassto[lv]);
+        lhgt = __ldg(&n.levhgt[lv]);
+        lfrc = __ldg(&n.levfrc[lv]);
+        bhgt = __ldg(&n.bashgt[lv]);
+        ldst = __ldg(&n.levdst[lv]);
+        ltop = __ldg(&n.levtopsto[lv]);
+        lfil = __ldg(&n.levfilsto[lv]);
+        lcase = pstoall < lbas ? 1 : pstoall < ltop ? 2 : pstoall < lfil ? 3 : 4;
+    }
+    if (lcase == 1 || lcase == 4) {
+        const Filled f = fill_layers(n, i, pstoall, rsm, wth, inc);
+        double wadd;
+        if (f.I < L) {
+            wadd = -f.wfil + sqrt(f.wfil * f.wfil + ((2.0 * (pstoall - f.sfil)) / len) / f.grd);
+            o.flddph = f.dfil + f.grd * wadd;
+        } else {
+            wadd = 0.0;
+            o.flddph = f.dfil + ((pstoall - f.sfil) / f.wfil) / len;
+        }
+        o.rivsto = rsm + (len * wth) * o.flddph;
+        if (!n.llevee) o.rivsto = dmin(o.rivsto, pstoall);
+        double frc = ((-wth + f.wfil) + wadd) / (inc * (double)L);
+        if (lcase == 1) {
             o.fldsto = dmax(pstoall - o.rivsto, 0.0);
-            double frc = ((-wth + wfil) + wadd) / (inc * (double)L);
+            frc = dmax(frc, 0.0);
+            frc = dmin(frc, 1.0);
+        } else {
+            const double sadd = ((o.flddph - lhgt) * (ldst + wth)) * len;
+            o.fldsto = dmax((ltop + sadd) - o.rivsto, 0.0);
+            o.levsto = dmax((pstoall - o.rivsto) - o.fldsto, 0.0);
+            o.levdph = o.flddph;
+        }
+        o.fldfrc = frc;
+        o.fldare = grarea * frc;
+    } else if (lcase == 2) {
+        const double sadd = pstoall - __ldg(&n.levbassto[lv]);
+        const double wadd = ldst + wth;
+        o.flddph = bhgt + (sadd / wadd) / len;
+        o.rivsto = rsm + (len * wth) * o.flddph;
+        o.fldsto = dmax(pstoall - o.rivsto, 0.0);
+        o.fldfrc = lfrc;
+        o.fldare = grarea * lfrc;
+    } else {                                                                        // case 3
+        o.flddph = lhgt;
+        o.rivsto = rsm + (len * wth) * o.flddph;
+        o.fldsto = dmax(ltop - o.rivsto, 0.0);
+        o.levsto = dmax((pstoall - o.rivsto) - o.fldsto, 0.0);
+        const int ilev = (int)(lfrc * (double)L) + 1;   // 1-based layer with the levee
+        double sfil = ltop, wfil = 0.0, dfil = 0.0, sadd;
+        int I = ilev;                                   // 1-based
+        while (I <= L) {
+            const double fhgt = __ldg(&n.fldhgt[(size_t)(I - 1) * N + i]), fmax = __ldg(&n.fldstomax[(size_t)(I - 1) * N + i]);
+            sadd = ((ldst + wth) * (lhgt - fhgt)) * len;
+            if (pstoall < fmax + sadd) break;
+            sfil = fmax + sadd;
+            wfil = inc * (double)I - ldst;
+            dfil = fhgt - bhgt;
+            I++;
+        }
+        if (I <= L) {
+            const double gr = __ldg(&n.fldgrd[(size_t)(I - 1) * N + i]);
+            const double wadd = -wfil + sqrt(wfil * wfil + ((2.0 * (pstoall - sfil)) / len) / gr);
+            const double dadd = wadd * gr;
+            o.levdph = (bhgt + dfil) + dadd;
+            double frc = (wfil + ldst) / (inc * (double)L);
             frc = dmax(frc, 0.0);
             frc = dmin(frc, 1.0);
             o.fldfrc = frc;
             o.fldare = grarea * frc;
-            o.levsto = 0.0;
-            o.levdph = 0.0;
         } else {
-            const double lhgt = __ldg(&n.levhgt[lv]), lfrc = __ldg(&n.levfrc[lv]), bhgt = __ldg(&n.bashgt[lv]), ldst = __ldg(&n.levdst[lv]);
-            const double ltop = __ldg(&n.levtopsto[lv]), lfil = __ldg(&n.levfilsto[lv]);
-            if (pstoall < ltop) {                                                   // case 2
-                const double sadd = pstoall - lbas;
-                const double wadd = ldst + wth;
-                o.flddph = bhgt + (sadd / wadd) / len;
-                o.rivsto = rsm + (len * wth) * o.flddph;
-                o.rivdph = (o.rivsto / len) / wth;
-                o.fldsto = dmax(pstoall - o.rivsto, 0.0);
-                o.fldfrc = lfrc;
-                o.fldare = grarea * lfrc;
-                o.levsto = 0.0;
-                o.levdph = 0.0;
-            } else if (pstoall < lfil) {                                            // case 3
-                o.flddph = lhgt;
-                o.rivsto = rsm + (len * wth) * o.flddph;
-                o.rivdph = (o.rivsto / len) / wth;
-                o.fldsto = dmax(ltop - o.rivsto, 0.0);
-                o.levsto = dmax((pstoall - o.rivsto) - o.fldsto, 0.0);
-                const int ilev = (int)(lfrc * (double)L) + 1;   // 1-based layer with the levee
-                double sfil = ltop, wfil = 0.0, dfil = 0.0, sadd;
-                int I = ilev;                                   // 1-based
-                while (I <= L) {
-                    sadd = ((ldst + wth) * (lhgt - __ldg(&n.fldhgt[(size_t)(I - 1) * N + i]))) * len;
-                    if (pstoall < __ldg(&n.fldstomax[(size_t)(I - 1) * N + i]) + sadd) break;
-                    sfil = __ldg(&n.fldstomax[(size_t)(I - 1) * N + i]) + sadd;
-                    wfil = inc * (double)I - ldst;
-                    dfil = __ldg(&n.fldhgt[(size_t)(I - 1) * N + i]) - bhgt;
-                    I++;
-                }
-                if (I <= L) {
-                    const double gr = __ldg(&n.fldgrd[(size_t)(I - 1) * N + i]);
-                    const double wadd = -wfil + sqrt(wfil * wfil + ((2.0 * (pstoall - sfil)) / len) / gr);
-                    const double dadd = wadd * gr;
-                    o.levdph = (bhgt + dfil) + dadd;
-                    double frc = (wfil + ldst) / (inc * (double)L);
-                    frc = dmax(frc, 0.0);
-                    frc = dmin(frc, 1.0);
-                    o.fldfrc = frc;
-                    o.fldare = grarea * frc;
-                } else {
-                    const double dadd = ((pstoall - sfil) / wfil) / len;
-                    o.levdph = (bhgt + dfil) + dadd;
-                    o.fldfrc = 1.0;
-                    o.fldare = grarea * 1.0;
-                }
-            } else {                                                                // case 4
-                int I = 0;
-                double sfil = rsm, wfil = wth, dfil = 0.0, wadd;
-                while (I < L) {
-                    const double smax = __ldg(&n.fldstomax[(size_t)I * N + i]);
-                    if (!(pstoall > smax)) break;
-                    sfil = smax; wfil = wfil + inc; dfil = dfil + __ldg(&n.fldgrd[(size_t)I * N + i]) * inc;
-                    I++;
-                }
-                if (I < L) {
-                    const double gr = __ldg(&n.fldgrd[(size_t)I * N + i]);
-                    wadd = -wfil + sqrt(wfil * wfil + ((2.0 * (pstoall - sfil)) / len) / gr);
-                    o.flddph = dfil + gr * wadd;
-                } else {
-                    wadd = 0.0;
-                    o.flddph = dfil + ((pstoall - sfil) / wfil) / len;
-                }
-                o.fldfrc = ((-wth + wfil) + wadd) / (inc * (double)L);
-                o.fldare = grarea * o.fldfrc;
-                o.rivsto = rsm + (len * wth) * o.flddph;
-                o.rivdph = (o.rivsto / len) / wth;
-                const double sadd = ((o.flddph - lhgt) * (ldst + wth)) * len;
-                o.fldsto = dmax((ltop + sadd) - o.rivsto, 0.0);
-                o.levsto = dmax((pstoall - o.rivsto) - o.fldsto, 0.0);
-                o.levdph = o.flddph;
-            }
+            const double dadd = ((pstoall - sfil) / wfil) / len;
+            o.levdph = (bhgt + dfil) + dadd;
+            o.fldfrc = 1.0;
+            o.fldare = grarea * 1.0;
         }
-    } else {                                                                        // case 0
-        o.rivsto = pstoall;
-        o.rivdph = dmax((pstoall / len) / wth, 0.0);
-        o.fldsto = 0.0; o.flddph = 0.0; o.fldfrc = 0.0; o.fldare = 0.0; o.levsto = 0.0; o.levdph = 0.0;
     }
+    o.rivdph = (o.rivsto / len) / wth;
     return o;
 }
 
-// diag_only: D2FLDARE and D2SFCELV are read by nothing inside the sub-step loop, so the sub-steps
-// write them on the last sub-step only (the values the caller observes are the same)
-__device__ __forceinline__ void store_stage(const Net &n, const State &s, size_t gi, int i, const StageOut &o,
+// D2FLDARE and D2SFCELV are read by nothing inside the sub-step loop, so the sub-steps write them on
+// the last sub-step only (diag_out; the values the caller observes are the same)
+template <class Own>
+__device__ __forceinline__ void store_stage(const Net &n, const State &s, const Own &w, size_t gi, int i, const StageOut &o,
                                             bool diag_out = true) {
-    s.rivsto[gi] = o.rivsto;
-    s.fldsto[gi] = o.fldsto;
-    s.rivdph[gi] = o.rivdph;
-    s.flddph[gi] = o.flddph;
-    s.fldfrc[gi] = o.fldfrc;
     if (diag_out) {
         s.fldare[gi] = o.fldare;
-        s.sfcelv[gi] = __ldg(&n.rivelv[i]) + o.rivdph;
+        s.sfcelv[gi] = w.rivelv(i) + o.rivdph;
     }
-    if (n.llevee) {
-        s.levsto[gi] = o.levsto;
-        s.levdph[gi] = o.levdph;
-        s.storge[gi] = (o.rivsto + o.fldsto) + o.levsto;
-    } else {
-        s.storge[gi] = o.rivsto + o.fldsto;
-    }
+    w.put_stage(gi, o, n.llevee ? (o.rivsto + o.fldsto) + o.levsto : o.rivsto + o.fldsto);
 }
 
 template <int NV>
@@ -495,10 +555,9 @@ __global__ void __launch_bounds__(kCellThreads, CMF_STAGE_MINB) k_stage(Net n, S
     double key = 1.0e308;
     if (i < n.N) {
         const size_t gi = (size_t)m * n.N + i;
-        const OwnG w{n, s};
-        const StageOut o = n.llevee ? stage_levee(n, w, i, s.rivsto[gi], s.fldsto[gi], s.levsto[gi])
-                                    : stage_def(n, w, i, s.rivsto[gi], s.fldsto[gi]);
-        store_stage(n, s, gi, i, o);
+        const OwnG w(n, s, __ldg(&n.cflag[i]));
+        const StageOut o = stage(n, w, i, stage_map(w, i), s.rivsto[gi], s.fldsto[gi], n.llevee ? s.levsto[gi] : 0.0);
+        store_stage(n, s, w, gi, i, o);
         if (n.ladpstp && __ldg(&n.i2mask[i]) == 0) key = cfl_key(n.pcadp, (i < n.R) ? __ldg(&n.nxtdst[i]) : n.pdstmth, n.pgrv, o.rivdph);
     }
     if (n.ladpstp) {
@@ -518,38 +577,48 @@ __global__ void __launch_bounds__(kCellThreads, CMF_STAGE_MINB) k_stage(Net n, S
 // ------------------------------------------------------------------------------------------
 // k_ntdt: NT and DT per member (src/cmf_ctrl_physics_mod.F90:205-206) and the loop bound
 // ------------------------------------------------------------------------------------------
+struct NtDt {
+    double dt_min, dt;
+    int nt;                        // 0: refused (NT cap)
+    bool near;                     // DT_DEF/DT_MIN - 0.01 next to an integer
+};
+__device__ __forceinline__ NtDt calc_ntdt(const Net &n, double dt_def, unsigned long long dtmin_bits) {
+    NtDt r{dt_def, dt_def, 1, false};
+    if (n.ladpstp) {
+        r.dt_min = dmin(dt_def, __longlong_as_double((long long)dtmin_bits));
+        const double x = dt_def * (1.0 / r.dt_min) - CMF_F(0.01);
+        if (!(x >= 0.0) || x > (double)(kNtCap - 1)) {
+            r.nt = 0;              // non-finite or oversized NT: refuse to loop
+        } else {
+            r.nt = (int)x + 1;
+            r.dt = dt_def * (double)(1.0f / (float)r.nt);
+            r.near = fabs(x - rint(x)) <= 1e-12 * dmax(x, 1.0);
+        }
+    }
+    return r;
+}
+__device__ __forceinline__ void put_ntdt(MemberCtl &c, LoopCtl *loop, const NtDt &r) {
+    c.dt_min = r.dt_min;
+    if (r.nt == 0) c.err = kErrNtCap;
+    c.nt = r.nt;
+    c.dt = r.dt;
+    c.it = 0;
+    c.nadd = 0.0;
+    atomicAdd((unsigned long long *)&loop->nt_hist[min(r.nt, kNtHist - 1)], 1ull);
+}
+
 __global__ void k_ntdt(Net n, State s, cudaGraphConditionalHandle h, int use_cond) {
     __shared__ int smax[32];
     int ntmax = 1;
     long long ntsum = 0, near = 0;
     for (int m = threadIdx.x; m < n.M; m += blockDim.x) {
         MemberCtl &c = s.ctl[m];
-        const double dt_def = c.dt_def;
-        int nt = 1;
-        double dt = dt_def;
-        if (n.ladpstp) {
-            const double dt_min = dmin(dt_def, __longlong_as_double((long long)c.dtmin_bits));
-            c.dt_min = dt_min;
-            const double x = dt_def * (1.0 / dt_min) - CMF_F(0.01);
-            if (!(x >= 0.0) || x > (double)(kNtCap - 1)) {
-                c.err = kErrNtCap;   // non-finite or oversized NT: refuse to loop
-                nt = 0;
-            } else {
-                nt = (int)x + 1;
-                dt = dt_def * (double)(1.0f / (float)nt);
-                if (fabs(x - rint(x)) <= 1e-12 * dmax(x, 1.0)) near++;
-            }
-            c.dtmin_bits = (unsigned long long)__double_as_longlong(dt_def);
-        } else {
-            c.dt_min = dt_def;
-        }
-        c.nt = nt;
-        c.dt = dt;
-        c.it = 0;
-        c.nadd = 0.0;
-        ntmax = max(ntmax, nt);
-        ntsum += nt;
-        atomicAdd((unsigned long long *)&s.loop->nt_hist[min(nt, kNtHist - 1)], 1ull);
+        const NtDt r = calc_ntdt(n, c.dt_def, c.dtmin_bits);
+        put_ntdt(c, s.loop, r);
+        if (n.ladpstp) c.dtmin_bits = (unsigned long long)__double_as_longlong(c.dt_def);
+        near += r.near;
+        ntmax = max(ntmax, r.nt);
+        ntsum += r.nt;
     }
     __shared__ long long ssum[32], snear[32];
     for (int o = 16; o > 0; o >>= 1) {
@@ -595,58 +664,147 @@ __device__ __forceinline__ double rate_min1(double a, double b) { return (a >= b
 
 // CMF_DIAG_AVEMAX_ADPSTP (src/cmf_calc_diag_mod.F90:104-161) of the sub-step before this one,
 // carried into this sub-step's phase A, which reads that sub-step's results anyway: its D2RIVOUT and
-// D2FLDOUT are this sub-step's D2*OUT_PRE, its D2RIVDPH and D2STORGE the state it left, its D2DAMINF
-// the inflow phase A is about to replace.  Every addition and maximum is the reference's, in its
-// order, so each accumulator holds the bits phase C of that sub-step would have stored.  Phase C
-// still forms the last sub-step's terms (and the division by NADD), and D2PTHOUT_aAVG, whose
-// per-cell path sum phase A does not see.  The accumulators are read after phase A's own stores:
-// read at its top they would hold 16 registers across the outflow arithmetic and spill (measured
-// slower).
-struct DiagPrev {
-    double rivout, fldout, outflw, daminf, dinf, mout, mdph, msto;
-};
-// `daminf` is the previous sub-step's D2DAMINF (phase A captures it before replacing it)
-__device__ __forceinline__ DiagPrev diag_carry_load(const Net &n, const State &s, size_t gi, bool first,
-                                                    double daminf) {
-    DiagPrev p;
-    p.rivout = first ? 0.0 : s.a_rivout[gi];
-    p.fldout = first ? 0.0 : s.a_fldout[gi];
-    p.outflw = first ? 0.0 : s.a_outflw[gi];
-    p.mout = first ? 0.0 : s.m_outflw[gi];
-    p.mdph = first ? 0.0 : s.m_rivdph[gi];
-    p.msto = first ? 0.0 : s.m_storge[gi];
-    p.dinf = daminf;
-    p.daminf = (first || !n.ldamout) ? 0.0 : s.a_daminf[gi];
-    return p;
-}
+// D2FLDOUT are this sub-step's D2*OUT_PRE, its D2RIVDPH and D2STORGE the state it left.  Every addition
+// and maximum is the reference's, in its order, so each accumulator holds the bits phase C of that
+// sub-step would have stored.  Phase C still forms the last sub-step's terms (and the division by
+// NADD), and D2PTHOUT_aAVG, whose per-cell path sum phase A does not see; D2DAMINF_aAVG is
+// accumulated by cell_dam and, for the cells without a dam rule, rebuilt on the last sub-step
+// (daminf_sum).  The accumulators are read after phase A's own stores: read at its top they would hold
+// registers across the outflow arithmetic and spill (measured slower).
 __device__ __forceinline__ bool same_bits(double a, double b) {
     return __double_as_longlong(a) == __double_as_longlong(b);
 }
-__device__ __forceinline__ void diag_carry_store(const Net &n, const State &s, size_t gi, double DT, bool first,
-                                                 const DiagPrev &p, double rivout, double fldout, double rivdph,
-                                                 double storge) {
+__device__ __forceinline__ void diag_carry(const State &s, size_t gi, double DT, bool first, double rivout, double fldout,
+                                           double rivdph, double storge) {
+    const double outflw = rivout + fldout;
+    const double pro = first ? 0.0 : s.a_rivout[gi], pfo = first ? 0.0 : s.a_fldout[gi];
+    const double pof = first ? 0.0 : s.a_outflw[gi], pmo = first ? 0.0 : s.m_outflw[gi];
+    const double pmd = first ? 0.0 : s.m_rivdph[gi], pms = first ? 0.0 : s.m_storge[gi];
     // a store is skipped when the sub-step leaves the accumulator's bits unchanged (a zero discharge
     // added to a running sum, a maximum that did not move): the array holds the same bits either way
     auto acc = [&](double prev, double *a, double v) {
         const double x = first ? v * DT : prev + v * DT;
         if (first || !same_bits(x, prev)) a[gi] = x;
     };
-    const double outflw = rivout + fldout;
-    acc(p.rivout, s.a_rivout, rivout);
-    acc(p.fldout, s.a_fldout, fldout);
-    acc(p.outflw, s.a_outflw, outflw);
-    if (n.ldamout) acc(p.daminf, s.a_daminf, p.dinf);
-    const double mo = dmax(p.mout, fabs(outflw));
-    const double md = dmax(p.mdph, rivdph);
-    const double ms = dmax(p.msto, storge);
-    if (first || !same_bits(mo, p.mout)) s.m_outflw[gi] = mo;
-    if (first || !same_bits(md, p.mdph)) s.m_rivdph[gi] = md;
-    if (first || !same_bits(ms, p.msto)) s.m_storge[gi] = ms;
+    acc(pro, s.a_rivout, rivout);
+    acc(pfo, s.a_fldout, fldout);
+    acc(pof, s.a_outflw, outflw);
+    const double mo = dmax(pmo, fabs(outflw));
+    const double md = dmax(pmd, rivdph);
+    const double ms = dmax(pms, storge);
+    if (first || !same_bits(mo, pmo)) s.m_outflw[gi] = mo;
+    if (first || !same_bits(md, pmd)) s.m_rivdph[gi] = md;
+    if (first || !same_bits(ms, pms)) s.m_storge[gi] = ms;
+}
+
+// D2DAMINF_aAVG before the last of `nt` sub-steps: accumulated where a dam rule renews D2DAMINF; elsewhere
+// D2DAMINF stays what the host set, and the running sum is rebuilt with the same additions (+0 stays +0)
+__device__ __forceinline__ double daminf_sum(const State &s, size_t gi, unsigned flags, double DT, int nt, double dinf) {
+    if (nt == 1) return 0.0;
+    if (flags & C_DAM) return s.a_daminf[gi];
+    if (__double_as_longlong(dinf) == 0) return 0.0;
+    double t = dinf * DT;
+    for (int k = 1; k < nt - 1; k++) t = t + dinf * DT;
+    return t;
+}
+
+// D2RIVVEL is observed after the last sub-step; its sub-step average is accumulated in phase A
+// (CMF_DIAG_AVEMAX_ADPSTP, src/cmf_calc_diag_mod.F90:104-161)
+template <class Own>
+__device__ __forceinline__ void vel_average(const Net &n, const State &s, const Own &w, size_t gi, double DT, int nt,
+                                            double dt_def, int k, double rvel) {
+    const bool first = (k == 0), last = (k == nt - 1);
+    if (last) s.rivvel[gi] = rvel;
+    if (!n.ldiag) return;
+    const double prev = first ? 0.0 : w.a_rivvel(gi);
+    double a = first ? rvel * DT : prev + rvel * DT;
+    if (last) {
+        a = a / (nadd_before(k, DT) + DT);
+        if (n.ldiag_out) s.o_rivvel[gi] = s.o_rivvel[gi] + a * dt_def;   // CMF_DIAG_AVEMAX_OUTPUT
+        s.a_rivvel[gi] = a;
+    } else if (first || !same_bits(a, prev)) {
+        w.put_a_rivvel(gi, a);          // unchanged bits (a dry cell adds +0): no store needed
+    }
+}
+
+// Reservoir operation, CMF_DAMOUT_CALC (src/cmf_ctrl_damout_mod.F90:316-498): the outflow of a cell with
+// I1DAM > 0, in place of cell_outflow's (which still forms the cell's diagnostics)
+template <class Own>
+__device__ __forceinline__ void cell_dam(const Net &n, const State &s, const Own &w, int m, int i, double DT, int nt,
+                                         double dt_def, int k) {
+    const size_t base = (size_t)m * n.N, gi = base + i;
+    double rout = 0.0, fout = 0.0, dinf = w.runoff(gi);
+    const int q = __ldg(&n.dam_pos[i]), d = __ldg(&n.dam_id[i]);
+    // UPDATE_INFLOW 1b: inflow from the dam's upstream cells, in ascending sequence
+    for (int e = __ldg(&n.dam_up_ptr[q]); e < __ldg(&n.dam_up_ptr[q + 1]); e++) {
+        const int j = __ldg(&n.dam_up_idx[e]);
+        const double fpre = n.lfldout ? w.nb(s.fldout_pre, base + j) : 0.0;
+        dinf = (dinf + w.nb(s.rivout_pre, base + j)) + fpre;
+    }
+    if (n.ldiag && k > 0) {              // the previous sub-step's D2DAMINF joins its average before it is replaced
+        const double prev = s.daminf[gi] * DT;
+        s.a_daminf[gi] = k == 1 ? prev : s.a_daminf[gi] + prev;
+    }
+    s.daminf[gi] = dinf;
+    if (w.flags() & C_KIN) {
+        // UPDATE_INFLOW 1c: kinematic outflow upstream of a dam; (1/n) sqrt(slope) of channel and
+        // floodplain are static
+        const double p23 = CMF_F(2. / 3.);
+        const double dph = w.rivdph(gi), wth = w.rivwth(i);
+        const double dvel = __ldg(&n.kin_vel[q]) * pow(dph, p23);
+        const double darea = wth * dph;
+        rout = dmin(darea * dvel, w.rivsto(gi) / DT);
+        const double fdph = w.flddph(gi), fsto = w.fldsto(gi);
+        if (fdph > 0.0 || fsto != 0.0) {        // else min(0 * 0, 0) = +0
+            const double dvel_f = __ldg(&n.kin_velf[q]) * pow(fdph, p23);
+            double dare_f = fsto * w.inv_rivlen(i);
+            dare_f = dmax(dare_f - fdph * wth, 0.0);
+            fout = dmin(dare_f * dvel_f, fsto / DT);
+        }
+        vel_average(n, s, w, gi, DT, nt, dt_def, k, dvel);
+    }
+    if (d >= 0 && __ldg(&n.dam_stat[d]) > 0) {
+        const double vol = s.damsto[gi];
+        const double qn = __ldg(&n.qn[d]), qf = __ldg(&n.qf[d]), qa = __ldg(&n.qa[d]), con = __ldg(&n.convol[d]), eme = __ldg(&n.emevol[d]);
+        double q = 0.0;
+        if (n.ldamh22) {
+            const double nor = __ldg(&n.norvol[d]);
+            if (vol <= nor) q = qn * (vol / con);
+            else if (nor < vol && vol <= con) {
+                if (qf <= dinf) q = qn * CMF_F(0.5) + ((vol - nor) / (con - nor)) * (qf - qn);
+                else { const double r = (vol - nor) / (eme - nor); q = qn * CMF_F(0.5) + (r * r) * (qf - qn); }
+            } else if (con < vol && vol < eme) {
+                if (qf <= dinf)
+                    q = qf + ((dmax(CMF_F(1.) - __ldg(&n.r_volupa[d]) / CMF_F(0.2), 0.0) * (vol - con)) / (eme - con)) * (dinf - qf);
+                else { const double r = (vol - nor) / (eme - nor); q = qn * CMF_F(0.5) + (r * r) * (qf - qn); }
+            } else q = dmax(dinf, qf);
+        } else {
+            // the regimes' volume fractions share one quotient and one power: a warp of dams in different
+            // regimes walks each once (sqrt, cube and tenth root in turn took 12 us of a sub-step)
+            const double adj = __ldg(&n.adjvol[d]);
+            const int regime = vol <= con ? 1 : vol <= adj ? 2 : (vol > adj && vol <= eme) ? 3 : vol > eme ? 4 : 0;
+            const double lo = regime == 1 ? 0.0 : regime == 2 ? con : adj;
+            const double x = (vol - lo) / (regime == 1 ? con : regime == 2 ? adj - con : eme - adj);
+            double f = 0.0;
+            if (regime == 2 || regime == 3) f = pow(x, regime == 2 ? 3.0 : CMF_F(0.1));
+            if (regime == 1) q = qn * sqrt(x);
+            else if (regime == 2) q = qn + f * (qa - qn);
+            else if (regime == 3) {
+                const double t = qa + f * (qf - qa);
+                q = dinf >= qf ? dmax(qn + ((vol - con) / (eme - con)) * (dinf - qn), t) : t;
+            } else if (regime == 4) q = (dinf >= qf) ? dinf : qf;
+        }
+        q = dmin(dmin(q, vol / DT), (w.rivsto(gi) + w.fldsto(gi)) / DT);
+        q = dmax(q, 0.0);
+        rout = q;
+        fout = 0.0;
+    }
+    w.put_raw(gi, i, rout, fout);
 }
 
 template <class Own>
 __device__ __forceinline__ void cell_outflow(const Net &n, const State &s, const Own &w, int m, int i, double DT,
-                                             const MemberCtl &c, int k, bool split) {
+                                             int nt, double dt_def, int k, bool split) {
     const size_t base = (size_t)m * n.N, gi = base + i;
     const double gdt = n.pgrv * DT;
     const double rivelv = w.rivelv(i);
@@ -659,192 +817,69 @@ __device__ __forceinline__ void cell_outflow(const Net &n, const State &s, const
     const double rivout_pre = w.rivout_pre(gi);
     const double rivout_old = split ? s.rivout_cur[gi] : rivout_pre;
     const double fldout_pre = w.fldout_pre(gi), storge = w.storge(gi);
-    const bool carry = n.ldiag && k > 0;   // diagnostics of sub-step k-1 (diag_carry_store)
-    bool dinf_taken = false;                 // D2DAMINF of sub-step k-1 read before the dam code replaced it
-    double dinf_prev = 0.0;
+    // river cells see the downstream cell's surface; a mouth the boundary elevation, over its own depth
+    const bool river = i < n.R;
+    double dwn, inv_dst, dsfc = sfc, dsfc_pre = sfc_pre, dflw = rivdph, dflw_pr = rivdph_pre;
+    if (river) {
+        const DownCell below = w.down(base, w.next(i));
+        dwn = below.rivelv + below.rivdph;
+        inv_dst = w.inv_nxtdst(i);
+        dsfc = dmax(sfc, dwn);
+        dsfc_pre = dmax(sfc_pre, below.rivelv + below.rivdph_pre);
+        dflw = dsfc - rivelv;
+        dflw_pr = dsfc_pre - rivelv;
+    } else {
+        dwn = __ldg(&n.dwnelv[i]);
+        inv_dst = 1.0 / n.pdstmth;
+    }
+    double dslp = (sfc - dwn) * inv_dst;
     double rout, fout = 0.0, rvel;
-    if (i < n.R) {
-        const int j = w.next(i);
-        const size_t gj = base + j;
-        const double rj = __ldg(&n.rivelv[j]);
-        const double dwn = rj + s.rivdph[gj];
-        const double dwn_pre = rj + s.rivdph_pre[gj];
-        const double inv_dst = w.inv_nxtdst(i);
-        // river
-        {
-            const double dsfc = dmax(sfc, dwn);
-            const double dslp = (sfc - dwn) * inv_dst;
-            const double dflw = dsfc - rivelv;
-            const double dare = dmax(wth * dflw, 1.E-10);
-            const double dflw_pr = dmax(sfc_pre, dwn_pre) - rivelv;
-            const double dflw_im = dmax(sqrt(dflw * dflw_pr), 1.E-6);
-            const double dout_pr = rivout_pre * inv_wth;
-            const double dout = (wth * (dout_pr + (gdt * dflw_im) * dslp))
-                              * (1.0 / (1.0 + ((gdt * (man * man)) * fabs(dout_pr)) * pow_depth<7>(dflw_im)));
-            const double dvel = rivout_old * (1.0 / dare);
-            const bool mask = (dflw_im > CMF_F(1.E-5) && dare > CMF_F(1.E-5));
-            rout = mask ? dout : 0.0;
-            rvel = mask ? dvel : 0.0;
+    {
+        const double dare = dmax(wth * dflw, 1.E-10);
+        const double dflw_im = dmax(sqrt(dflw * dflw_pr), 1.E-6);
+        const double dout_pr = rivout_pre * inv_wth;
+        const double dout = (wth * (dout_pr + (gdt * dflw_im) * dslp))
+                          * (1.0 / (1.0 + ((gdt * (man * man)) * fabs(dout_pr)) * pow_depth<7>(dflw_im)));
+        const double dvel = rivout_old * (1.0 / dare);
+        const bool mask = (dflw_im > CMF_F(1.E-5) && dare > CMF_F(1.E-5));
+        rout = mask ? dout : 0.0;
+        rvel = mask ? dvel : 0.0;
+    }
+    if (n.lfldout) {
+        // the reference's masks are a double at river cells and a default-real literal at mouths
+        const double eps = river ? 1.E-5 : CMF_F(1.E-5);
+        // without floodplain water the area is max(-FLDDPH * RIVWTH, 0) = 0: nothing more to read
+        const double fsto = w.fldsto(gi), inv_len = fsto != 0.0 ? w.inv_rivlen(i) : 0.0;
+        const double dare = fsto != 0.0 ? dmax(fsto * inv_len - w.flddph(gi) * wth, 0.0) : 0.0;
+        if (dare > eps) {
+            const double elv = w.elevtn(i);
+            dslp = dmax(-0.005, dmin(0.005, dslp));
+            const double df = river ? dmax(dsfc - elv, 0.0) : sfc - elv;
+            const double df_pr = dsfc_pre - elv;
+            const double dflw_im = dmax(sqrt(dmax(df * df_pr, 0.0)), 1.E-6);
+            const double flddph_pre = dmax(rivdph_pre - w.rivhgt(i), 0.0);
+            const double dare_pr = dmax(w.fldsto_pre(gi) * inv_len - flddph_pre * wth, 1.E-6);
+            const double dare_im = dmax(sqrt(dare * dare_pr), 1.E-6);
+            const double dout_pr = fldout_pre;
+            const double dout = (dout_pr + (gdt * dare_im) * dslp)
+                * (1.0 / (1.0 + (((gdt * (n.pmanfld * n.pmanfld)) * fabs(dout_pr)) * pow_depth<4>(dflw_im)) * (1.0 / dare_im)));
+            fout = (dflw_im > eps) ? dout : 0.0;
+            if (!(fout * rout > 0.0)) fout = 0.0;
         }
-        if (n.lfldout) {
-            const double inv_len = w.inv_rivlen(i);
-            double dare = w.fldsto(gi) * inv_len;
-            dare = dmax(dare - w.flddph(gi) * wth, 0.0);
-            if (dare > 1.E-5) {
-                const double elv = w.elevtn(i);
-                const double dsfc = dmax(sfc, dwn);
-                double dslp = (sfc - dwn) * inv_dst;
-                dslp = dmax(-0.005, dmin(0.005, dslp));
-                const double dflw = dmax(dsfc - elv, 0.0);
-                const double dflw_pr = dmax(sfc_pre, dwn_pre) - elv;
-                const double dflw_im = dmax(sqrt(dmax(dflw * dflw_pr, 0.0)), 1.E-6);
-                const double flddph_pre = dmax(rivdph_pre - w.rivhgt(i), 0.0);
-                double dare_pr = w.fldsto_pre(gi) * inv_len;
-                dare_pr = dmax(dare_pr - flddph_pre * wth, 1.E-6);
-                const double dare_im = dmax(sqrt(dare * dare_pr), 1.E-6);
-                const double dout_pr = fldout_pre;
-                const double dout = (dout_pr + (gdt * dare_im) * dslp)
-                    * (1.0 / (1.0 + (((gdt * (n.pmanfld * n.pmanfld)) * fabs(dout_pr)) * pow_depth<4>(dflw_im)) * (1.0 / dare_im)));
-                fout = (dflw_im > 1.E-5) ? dout : 0.0;
-                if (!(fout * rout > 0.0)) fout = 0.0;
-            }
-        }
+    }
+    if (river) {
         // storage-change limiter (v423), :176-182
         const double dlim = dmax((-rout - fout) * DT, CMF_F(1.E-10));
         const double rate = rate_min1(0.05 * storge, dlim);
         rout = rout * rate;
         fout = fout * rate;
-    } else {
-        const double inv_dst = 1.0 / n.pdstmth;
-        const double dwn = __ldg(&n.dwnelv[i]);
-        {
-            const double dslp = (sfc - dwn) * inv_dst;
-            const double dare = dmax(wth * rivdph, 1.E-10);
-            const double dflw_im = dmax(sqrt(rivdph * rivdph_pre), 1.E-6);
-            const double dout_pr = rivout_pre * inv_wth;
-            const double dout = (wth * (dout_pr + (gdt * dflw_im) * dslp))
-                              * (1.0 / (1.0 + ((gdt * (man * man)) * fabs(dout_pr)) * pow_depth<7>(dflw_im)));
-            const double dvel = rivout_old * (1.0 / dare);
-            const bool mask = (dflw_im > CMF_F(1.E-5) && dare > CMF_F(1.E-5));
-            rout = mask ? dout : 0.0;
-            rvel = mask ? dvel : 0.0;
-        }
-        if (n.lfldout) {
-            const double inv_len = w.inv_rivlen(i);
-            const double dare = dmax(w.fldsto(gi) * inv_len - w.flddph(gi) * wth, 0.0);
-            if (dare > CMF_F(1.E-5)) {
-                const double elv = w.elevtn(i);
-                double dslp = (sfc - dwn) * inv_dst;
-                dslp = dmax(-0.005, dmin(0.005, dslp));
-                const double dflw = sfc - elv;
-                const double dflw_pr = sfc_pre - elv;
-                const double dflw_im = dmax(sqrt(dmax(dflw * dflw_pr, 0.0)), 1.E-6);
-                const double flddph_pre = dmax(rivdph_pre - w.rivhgt(i), 0.0);
-                const double dare_pr = dmax(w.fldsto_pre(gi) * inv_len - flddph_pre * wth, 1.E-6);
-                const double dare_im = dmax(sqrt(dare * dare_pr), 1.E-6);
-                const double dout_pr = fldout_pre;
-                const double dout = (dout_pr + (gdt * dare_im) * dslp)
-                    * (1.0 / (1.0 + (((gdt * (n.pmanfld * n.pmanfld)) * fabs(dout_pr)) * pow_depth<4>(dflw_im)) * (1.0 / dare_im)));
-                fout = (dflw_im > CMF_F(1.E-5)) ? dout : 0.0;
-                if (!(fout * rout > 0.0)) fout = 0.0;
-            }
-        }
     }
-    // reservoir operation, CMF_DAMOUT_CALC (src/cmf_ctrl_damout_mod.F90:316-498)
-    if (n.ldamout) {
-        const int code = w.i1dam(i);
-        if (code > 0) {
-            rout = 0.0;
-            fout = 0.0;
-            double dinf = s.runoff[gi];
-            const int d = __ldg(&n.dam_id[i]);
-            if (d >= 0) {
-                // UPDATE_INFLOW 1b: inflow from the dam's upstream cells, in ascending sequence
-                for (int k = __ldg(&n.up_ptr[i]); k < __ldg(&n.up_ptr[i + 1]); k++) {
-                    const int j = __ldg(&n.up_idx[k]);
-                    const int cj = __ldg(&n.i1dam[j]);
-                    if (cj == 10 || cj == 11) {
-                        const double fpre = n.lfldout ? s.fldout_pre[base + j] : 0.0;
-                        dinf = (dinf + s.rivout_pre[base + j]) + fpre;
-                    }
-                }
-            }
-            if (carry) {
-                dinf_prev = s.daminf[gi];
-                dinf_taken = true;
-            }
-            s.daminf[gi] = dinf;
-            if (code == 10 && i < n.R) {
-                // UPDATE_INFLOW 1c: kinematic outflow upstream of a dam
-                const int j = __ldg(&n.next[i]);
-                const double p23 = CMF_F(2. / 3.);
-                double dslope = (__ldg(&n.elevtn[i]) - __ldg(&n.elevtn[j])) * (1.0 / __ldg(&n.nxtdst[i]));
-                dslope = dmax(dslope, n.pminslp);
-                const double dph = rivdph;
-                const double dvel = ((1.0 / man) * sqrt(dslope)) * pow(dph, p23);
-                const double darea = wth * dph;
-                rvel = dvel;
-                rout = dmin(darea * dvel, s.rivsto[gi] / DT);
-                const double slope_f = dmin(0.005, dslope);
-                const double fdph = s.flddph[gi];
-                const double dvel_f = ((1.0 / n.pmanfld) * sqrt(slope_f)) * pow(fdph, p23);
-                double dare_f = s.fldsto[gi] * (1.0 / __ldg(&n.rivlen[i]));
-                dare_f = dmax(dare_f - fdph * wth, 0.0);
-                fout = dmin(dare_f * dvel_f, s.fldsto[gi] / DT);
-            }
-            if (d >= 0 && __ldg(&n.dam_stat[d]) > 0) {
-                const double vol = s.damsto[gi];
-                const double qn = __ldg(&n.qn[d]), qf = __ldg(&n.qf[d]), qa = __ldg(&n.qa[d]), con = __ldg(&n.convol[d]), eme = __ldg(&n.emevol[d]);
-                double q = 0.0;
-                if (n.ldamh22) {
-                    const double nor = __ldg(&n.norvol[d]);
-                    if (vol <= nor) q = qn * (vol / con);
-                    else if (nor < vol && vol <= con) {
-                        if (qf <= dinf) q = qn * CMF_F(0.5) + ((vol - nor) / (con - nor)) * (qf - qn);
-                        else { const double r = (vol - nor) / (eme - nor); q = qn * CMF_F(0.5) + (r * r) * (qf - qn); }
-                    } else if (con < vol && vol < eme) {
-                        if (qf <= dinf)
-                            q = qf + ((dmax(CMF_F(1.) - __ldg(&n.r_volupa[d]) / CMF_F(0.2), 0.0) * (vol - con)) / (eme - con)) * (dinf - qf);
-                        else { const double r = (vol - nor) / (eme - nor); q = qn * CMF_F(0.5) + (r * r) * (qf - qn); }
-                    } else q = dmax(dinf, qf);
-                } else {
-                    const double adj = __ldg(&n.adjvol[d]);
-                    if (vol <= con) q = qn * sqrt(vol / con);
-                    else if (vol > con && vol <= adj) q = qn + pow((vol - con) / (adj - con), 3.0) * (qa - qn);
-                    else if (vol > adj && vol <= eme) {
-                        const double t = qa + pow((vol - adj) / (eme - adj), CMF_F(0.1)) * (qf - qa);
-                        if (dinf >= qf) q = dmax(qn + ((vol - con) / (eme - con)) * (dinf - qn), t);
-                        else q = t;
-                    } else if (vol > eme) q = (dinf >= qf) ? dinf : qf;
-                }
-                q = dmin(dmin(q, vol / DT), (s.rivsto[gi] + s.fldsto[gi]) / DT);
-                q = dmax(q, 0.0);
-                rout = q;
-                fout = 0.0;
-            }
-        }
+    if (!(w.flags() & C_DAM)) w.put_raw(gi, i, rout, fout);
+    if (n.ldiag && k > 0) {              // diagnostics of sub-step k-1
+        if constexpr (Own::kResident) w.carry(gi, DT, k == 1, rivout_pre, fldout_pre, rivdph, storge);
+        else diag_carry(s, gi, DT, k == 1, rivout_pre, fldout_pre, rivdph, storge);
     }
-    s.rivout_raw[gi] = rout;
-    s.fldout_raw[gi] = fout;
-    if (carry) {
-        const double dinf = dinf_taken ? dinf_prev : (n.ldamout ? s.daminf[gi] : 0.0);
-        diag_carry_store(n, s, gi, DT, k == 1, diag_carry_load(n, s, gi, k == 1, dinf), rivout_pre, fldout_pre,
-                         rivdph, storge);
-    }
-    // D2RIVVEL is observed after the last sub-step; its sub-step average is accumulated here
-    // (CMF_DIAG_AVEMAX_ADPSTP, src/cmf_calc_diag_mod.F90:104-161) instead of in phase C
-    const bool first = (k == 0), last = (k == c.nt - 1);
-    if (last) s.rivvel[gi] = rvel;
-    if (n.ldiag) {
-        const double prev = first ? 0.0 : w.a_rivvel(gi);
-        double a = first ? rvel * DT : prev + rvel * DT;
-        if (last) {
-            a = a / (nadd_before(k, DT) + DT);
-            if (n.ldiag_out) s.o_rivvel[gi] = s.o_rivvel[gi] + a * c.dt_def;   // CMF_DIAG_AVEMAX_OUTPUT
-        }
-        // unchanged bits (a dry cell adds +0): no store needed
-        if (first || last || __double_as_longlong(a) != __double_as_longlong(prev)) s.a_rivvel[gi] = a;
-    }
+    if (!(w.flags() & C_KIN)) vel_average(n, s, w, gi, DT, nt, dt_def, k, rvel);
 }
 
 // CMF_CALC_PTHOUT (src/cmf_calc_pthout_mod.F90:34-94) / CMF_LEVEE_OPT_PTHOUT (src/cmf_ctrl_levee_mod.F90:508-601)
@@ -854,89 +889,112 @@ __device__ __forceinline__ double path_flux(double wth, double pre, double gdt, 
     return (wth * (dout_pr + (gdt * dflw_im) * dslp)) / (1.0 + ((gdt * (man * man)) * fabs(dout_pr)) * pow_depth<7>(dflw_im));
 }
 
-__device__ __forceinline__ void path_outflow(const Net &n, const State &s, int m, int p, double DT) {
-    const int P = n.P, Lp = n.Lp;
-    const size_t pb = (size_t)m * Lp * P;
-    const size_t base = (size_t)m * n.N;
-    const double gdt = n.pgrv * DT;
-    const int skip = __ldg(&n.pth_skip[p]);
+// Coherent: the ends' values come past L1, which may hold an older sub-step's line (kernels that run
+// several phases)
+template <bool Coherent>
+__device__ __forceinline__ double ld_nb(const double *p, size_t g) { return Coherent ? __ldcg(p + g) : p[g]; }
+
+// Bifurcation paths by lanes: thread x of the path threads takes level l of path p, 32 / Lp paths per
+// warp, the lanes of a path consecutive from lane0 (one thread per path ran its levels' powers one after
+// the other, up to 5 times as long as a cell, and in the last blocks of the grid).  With more than 32
+// levels a warp takes one path, and lane l its levels l and l + 32.
+__host__ __device__ inline int paths_per_warp(int Lp) { return Lp > 0 && Lp <= 32 ? 32 / Lp : 1; }
+__host__ __device__ inline int path_threads(int P, int Lp) { return P > 0 ? (P + paths_per_warp(Lp) - 1) / paths_per_warp(Lp) * 32 : 0; }
+struct PathLane {
+    int p, l, lane0;
+    bool on;
+};
+__device__ __forceinline__ PathLane path_lane(const Net &n, int x) {
+    const int ppw = paths_per_warp(n.Lp), lane = x & 31, q = min(lane / n.Lp, ppw), l = lane - q * n.Lp;
+    const int p = (x >> 5) * ppw + q;
+    return {p, l, q * n.Lp, q < ppw && p < n.P && l < n.Lp};
+}
+// 0 + v(1) + v(2) + ... over the levels of a path, in their order; v[1] holds the levels past 32
+__device__ __forceinline__ double level_sum(int Lp, int lane0, const double (&v)[2]) {
     double sum = 0.0;
-    double flw[8];
-    const bool skipped = n.llevee ? (skip & 2) : (skip & 1);
-    if (skipped) {
-        for (int l = 0; l < Lp; l++) s.pthflw_raw[pb + (size_t)l * P + p] = 0.0;
-        s.pthsum_raw[(size_t)m * P + p] = 0.0;
-        return;
-    }
-    const int u = __ldg(&n.pth_up[p]), d = __ldg(&n.pth_dn[p]);
-    const double su = __ldg(&n.rivelv[u]) + s.rivdph[base + u], sd = __ldg(&n.rivelv[d]) + s.rivdph[base + d];
-    const double spu = __ldg(&n.rivelv[u]) + s.rivdph_pre[base + u], spd = __ldg(&n.rivelv[d]) + s.rivdph_pre[base + d];
-    double dslp = (su - sd) / __ldg(&n.pth_dst[p]);
-    dslp = dmax(-0.005, dmin(0.005, dslp));
-    if (!n.llevee) {
-        for (int l = 0; l < Lp; l++) {
-            const size_t o = (size_t)l * P + p;
-            const double elv = __ldg(&n.pth_elv[o]);
-            const double dflw = dmax(dmax(su, sd) - elv, 0.0);
-            const double dflw_pr = dmax(dmax(spu, spd) - elv, 0.0);
-            double dflw_im = sqrt(dflw * dflw_pr);
-            dflw_im = dmax(dflw_im, sqrt(dflw * 0.01));
-            const double f = (dflw_im > 1.E-5) ? path_flux(__ldg(&n.pth_wth[o]), s.pthflw_pre[pb + o], gdt, dflw_im, dslp, __ldg(&n.pth_man[l]), false) : 0.0;
-            if (l < 8) flw[l] = f;
-            s.pthflw_raw[pb + o] = f;
-        }
-    } else {
-        // level 1: river channel, semi-implicit depth
-        {
-            const double elv = __ldg(&n.pth_elv[p]);
-            const double dflw = dmax(dmax(su, sd) - elv, 0.0);
-            const double dflw_pr = dmax(dmax(spu, spd) - elv, 0.0);
-            double dflw_im = sqrt(dflw * dflw_pr);
-            if (dflw_im <= 0.0) dflw_im = dflw;
-            const double f = (dflw_im > 1.E-5) ? path_flux(__ldg(&n.pth_wth[p]), s.pthflw_pre[pb + p], gdt, dflw_im, dslp, __ldg(&n.pth_man[0]), false) : 0.0;
-            flw[0] = f;
-            s.pthflw_raw[pb + p] = f;
-        }
-        if (Lp > 1) {
-            const int lu = __ldg(&n.lev_id[u]), ld = __ldg(&n.lev_id[d]);
-            double slu = su, sld = sd;
-            if (lu >= 0 && __ldg(&n.levfrc[lu]) < 1.0) slu = dmin(__ldg(&n.elevtn[u]) + s.levdph[base + u], su);
-            if (ld >= 0 && __ldg(&n.levfrc[ld]) < 1.0) sld = dmin(__ldg(&n.elevtn[d]) + s.levdph[base + d], sd);
-            for (int l = 1; l < Lp; l++) {
-                const size_t o = (size_t)l * P + p;
-                const double dflw = dmax(dmax(slu, sld) - __ldg(&n.pth_elv[o]), 0.0);
-                const double f = (dflw > 1.E-5) ? path_flux(__ldg(&n.pth_wth[o]), s.pthflw_pre[pb + o], gdt, dflw, dslp, __ldg(&n.pth_man[l]), true) : 0.0;
-                if (l < 8) flw[l] = f;
-                s.pthflw_raw[pb + o] = f;
-            }
-        }
-    }
-    for (int l = 0; l < Lp; l++) sum = sum + (l < 8 ? flw[l] : s.pthflw_raw[pb + (size_t)l * P + p]);
-    if (sum != 0.0) {
-        const double rate = rate_min1(0.05 * dmin(s.storge[base + u], s.storge[base + d]), fabs(sum * DT));
-        for (int l = 0; l < Lp; l++) {
-            const size_t o = pb + (size_t)l * P + p;
-            s.pthflw_raw[o] = (l < 8 ? flw[l] : s.pthflw_raw[o]) * rate;
-        }
-        sum = sum * rate;
-    }
-    s.pthsum_raw[(size_t)m * P + p] = sum;
+    for (int k = 0; k < min(Lp, 32); k++) sum = sum + __shfl_sync(0xffffffffu, v[0], (lane0 + k) & 31);
+    for (int k = 32; k < Lp; k++) sum = sum + __shfl_sync(0xffffffffu, v[1], k - 32);
+    return sum;
 }
 
+// Phase A of one path lane (every lane of the warp calls it): the level's flux, and the limiter on the
+// sum over the levels
+template <bool Coherent>
+__device__ __forceinline__ void path_outflow(const Net &n, const State &s, int m, const PathLane &t, double DT) {
+    const int P = n.P, Lp = n.Lp, p = t.p;
+    const size_t base = (size_t)m * n.N, pb = (size_t)m * Lp * P;
+    const int skip = t.on ? __ldg(&n.pth_skip[p]) : 3;
+    const bool live = t.on && !(n.llevee ? (skip & 2) : (skip & 1));
+    double f[2] = {0.0, 0.0};
+    int u = 0, d = 0;
+    if (live) {
+        u = __ldg(&n.pth_up[p]);
+        d = __ldg(&n.pth_dn[p]);
+        const double gdt = n.pgrv * DT;
+        const double eu = __ldg(&n.rivelv[u]), ed = __ldg(&n.rivelv[d]);
+        const double su = eu + ld_nb<Coherent>(s.rivdph, base + u), sd = ed + ld_nb<Coherent>(s.rivdph, base + d);
+        double dslp = (su - sd) / __ldg(&n.pth_dst[p]);
+        dslp = dmax(-0.005, dmin(0.005, dslp));
+#pragma unroll 1
+        for (int h = 0, l = t.l; l < Lp; h++, l += 32) {
+            const size_t o = (size_t)l * P + p;
+            const double elv = __ldg(&n.pth_elv[o]), wth = __ldg(&n.pth_wth[o]), man = __ldg(&n.pth_man[l]);
+            const double pre = s.pthflw_pre[pb + o];
+            const bool channel = !n.llevee || l == 0;    // with levees: level 1, the river channel
+            double im;
+            if (channel) {
+                const double spu = eu + ld_nb<Coherent>(s.rivdph_pre, base + u), spd = ed + ld_nb<Coherent>(s.rivdph_pre, base + d);
+                const double dflw = dmax(dmax(su, sd) - elv, 0.0);
+                const double dflw_pr = dmax(dmax(spu, spd) - elv, 0.0);
+                im = sqrt(dflw * dflw_pr);
+                if (!n.llevee) im = dmax(im, sqrt(dflw * 0.01));
+                else if (im <= 0.0) im = dflw;           // semi-implicit depth
+            } else {
+                double slu = su, sld = sd;
+                if (skip & 4) slu = dmin(__ldg(&n.elevtn[u]) + ld_nb<Coherent>(s.levdph, base + u), su);
+                if (skip & 8) sld = dmin(__ldg(&n.elevtn[d]) + ld_nb<Coherent>(s.levdph, base + d), sd);
+                im = dmax(dmax(slu, sld) - elv, 0.0);
+            }
+            const double v = im > 1.E-5 ? path_flux(wth, pre, gdt, im, dslp, man, !channel) : 0.0;
+            if (h == 0) f[0] = v;
+            else f[1] = v;
+        }
+    }
+    double sum = level_sum(Lp, t.lane0, f);
+    if (!live) sum = 0.0;
+    if (sum != 0.0) {
+        const double rate = rate_min1(0.05 * dmin(ld_nb<Coherent>(s.storge, base + u), ld_nb<Coherent>(s.storge, base + d)), fabs(sum * DT));
+        f[0] = f[0] * rate;
+        f[1] = f[1] * rate;
+        sum = sum * rate;
+    }
+    if (t.on) {
+        s.pthflw_raw[pb + (size_t)t.l * P + p] = f[0];
+        if (t.l + 32 < Lp) s.pthflw_raw[pb + (size_t)(t.l + 32) * P + p] = f[1];
+        if (t.l == 0) s.pthsum_raw[(size_t)m * P + p] = sum;
+    }
+}
+
+// Blocks of phase A: cells, then (path, level) lanes, then dam cells
 template <int MinBlocks>
-__global__ void __launch_bounds__(kCellThreads, MinBlocks) k_flux(Net n, State s, int ncell_blocks) {
+__global__ void __launch_bounds__(kCellThreads, MinBlocks) k_flux(Net n, State s, int ncell_blocks, int npath_blocks) {
     const int m = blockIdx.y;
     const MemberCtl &c = s.ctl[m];
     const int k = s.loop->k;
     if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) s.loop->kcur = k;   // for k_rate and k_store
     if (k >= c.nt) return;
     const double DT = c.dt;
+    const int x = blockIdx.x * blockDim.x + threadIdx.x;
     if ((int)blockIdx.x < ncell_blocks) {
-        const int i = blockIdx.x * blockDim.x + threadIdx.x;
-        if (i < n.N) cell_outflow(n, s, OwnG{n, s}, m, i, DT, c, k, s.loop->split != 0);
+        if (x < n.N) cell_outflow(n, s, OwnG(n, s, __ldg(&n.cflag[x])), m, x, DT, c.nt, c.dt_def, k, s.loop->split != 0);
+    } else if ((int)blockIdx.x < ncell_blocks + npath_blocks) {
+        path_outflow<false>(n, s, m, path_lane(n, x - ncell_blocks * (int)blockDim.x), DT);
     } else {
-        const int p = (blockIdx.x - ncell_blocks) * blockDim.x + threadIdx.x;
-        if (p < n.P) path_outflow(n, s, m, p, DT);
+        const int d = x - (ncell_blocks + npath_blocks) * (int)blockDim.x;
+        if (d < n.ndam_cells) {
+            const int i = __ldg(&n.dam_cells[d]);
+            cell_dam(n, s, OwnG(n, s, __ldg(&n.cflag[i])), m, i, DT, c.nt, c.dt_def, k);
+        }
     }
 }
 
@@ -946,22 +1004,22 @@ __global__ void __launch_bounds__(kCellThreads, MinBlocks) k_flux(Net n, State s
 template <class Own>
 __device__ __forceinline__ void cell_rate(const Net &n, const State &s, const Own &w, int m, int i, double DT) {
     const size_t base = (size_t)m * n.N, gi = base + i;
-    double so = dmax(w.rivout_raw(gi), 0.0) + dmax(w.fldout_raw(gi), 0.0);
-    // the CSR walk: at full occupancy the slot table's 16 B per cell cost more than its saved round
-    const int u1 = w.up_hi(i);
-    for (int k = w.up_lo(i); k < u1; k++) {
-        const int j = __ldg(&n.up_idx[k]);
-        so = (so + dmax(-s.rivout_raw[base + j], 0.0)) + dmax(-s.fldout_raw[base + j], 0.0);
-    }
+    const double rout = w.rivout_raw(gi), fout = w.fldout_raw(gi);
+    double so = dmax(rout, 0.0) + dmax(fout, 0.0);
+    w.each_raw(base, i, [&](double rj, double fj) { so = (so + dmax(-rj, 0.0)) + dmax(-fj, 0.0); });
     so = so * DT;
-    if (n.lpthout) {
+    if (w.flags() & C_PATH) {
         const double *sum = s.pthsum_raw + (size_t)m * n.P;
-        for (int k = __ldg(&n.pout_ptr[i]); k < __ldg(&n.pout_ptr[i + 1]); k++) so = so + dmax(sum[__ldg(&n.pout_idx[k])], 0.0) * DT;
-        for (int k = __ldg(&n.pinf_ptr[i]); k < __ldg(&n.pinf_ptr[i + 1]); k++) so = so + dmax(-sum[__ldg(&n.pinf_idx[k])], 0.0) * DT;
+        const int q = __ldg(&n.path_pos[i]), e1 = __ldg(&n.pend_ptr[q + 1]);
+        for (int e = __ldg(&n.pend_ptr[q]); e < e1; e++) {
+            const int p = __ldg(&n.pend[e].x);
+            const double v = w.nb(sum, p >= 0 ? p : ~p);
+            so = so + dmax(p >= 0 ? v : -v, 0.0) * DT;
+        }
     }
     const double dout = dmax(so, 1.E-10);
     const double dsto = w.rivsto(gi) + w.fldsto(gi);
-    s.rate[gi] = rate_min1(dsto, dout);
+    w.put_rate(gi, i, rout, fout, rate_min1(dsto, dout));
 }
 
 // advance != 0: block (0,0) also moves the loop counter to the next sub-step and sets the WHILE
@@ -978,93 +1036,112 @@ __global__ void k_rate(Net n, State s, int advance, cudaGraphConditionalHandle h
     }
     if (k >= c.nt) return;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n.N) return;
-    cell_rate(n, s, OwnG{n, s}, m, i, c.dt);
+    if (i < n.N) cell_rate(n, s, OwnG(n, s, __ldg(&n.cflag[i])), m, i, c.dt);
 }
 
 // ------------------------------------------------------------------------------------------
 // phase C: rescale + inflow + dam balance + VARS_PRE + STONXT + stage + diagnostics
 // ------------------------------------------------------------------------------------------
+template <bool Coherent>
 __device__ __forceinline__ double scaled_pathsum(const Net &n, const double *sum_raw, const double *rate_m, int p) {
-    const double v = sum_raw[p];
+    const double v = ld_nb<Coherent>(sum_raw, p);
     if (__ldg(&n.pth_skip[p]) & 1) return v;
-    return v >= 0.0 ? v * rate_m[__ldg(&n.pth_up[p])] : v * rate_m[__ldg(&n.pth_dn[p])];
+    return v * ld_nb<Coherent>(rate_m, v >= 0.0 ? __ldg(&n.pth_up[p]) : __ldg(&n.pth_dn[p]));
 }
 
-// bifurcation paths in phase C: LSPAMAT path rescale (:494-517), CALC_VARS_PRE copy, diagnostics
-__device__ __forceinline__ void path_rescale(const Net &n, const State &s, int m, int p, double DT, bool first, bool last,
-                                             double nadd, double dt_def) {
-    const int P = n.P, Lp = n.Lp;
-    const size_t base = (size_t)m * n.N;
-    const size_t pb = (size_t)m * Lp * P;
+// one path lane in phase C (every lane of the warp calls it): LSPAMAT path rescale (:494-517),
+// CALC_VARS_PRE copy, diagnostics
+template <bool Coherent>
+__device__ __forceinline__ void path_rescale(const Net &n, const State &s, int m, const PathLane &t, double DT, bool first,
+                                             bool last, double nadd, double dt_def) {
+    const int P = n.P, Lp = n.Lp, p = t.p;
+    const size_t base = (size_t)m * n.N, pb = (size_t)m * Lp * P;
     const double *rate_m = s.rate + base;
-    const bool sk = __ldg(&n.pth_skip[p]) & 1;
-    const int u = __ldg(&n.pth_up[p]), d = __ldg(&n.pth_dn[p]);
-    double asum = 0.0;
-    for (int l = 0; l < Lp; l++) {
-        const size_t o = pb + (size_t)l * P + p;
-        double f = s.pthflw_raw[o];
-        if (!sk) f = (f >= 0.0) ? f * rate_m[u] : f * rate_m[d];
-        s.pthflw_pre[o] = f;
-        if (n.ldiag) {
-            double a = first ? f * DT : s.a_pthflw[o] + f * DT;
-            if (last) {
-                a = a / (nadd + DT);
-                asum = asum + a;
-                if (n.ldiag_out) s.o_pthflw[o] = s.o_pthflw[o] + a * dt_def;
+    double a[2] = {0.0, 0.0};
+    if (t.on) {
+        const bool sk = __ldg(&n.pth_skip[p]) & 1;
+#pragma unroll 1
+        for (int h = 0, l = t.l; l < Lp; h++, l += 32) {
+            const size_t o = pb + (size_t)l * P + p;
+            double f = s.pthflw_raw[o];
+            if (!sk) f = f * ld_nb<Coherent>(rate_m, f >= 0.0 ? __ldg(&n.pth_up[p]) : __ldg(&n.pth_dn[p]));
+            s.pthflw_pre[o] = f;
+            if (n.ldiag) {
+                double x = first ? f * DT : s.a_pthflw[o] + f * DT;
+                if (last) {
+                    x = x / (nadd + DT);
+                    if (n.ldiag_out) s.o_pthflw[o] = s.o_pthflw[o] + x * dt_def;
+                }
+                s.a_pthflw[o] = x;
+                if (h == 0) a[0] = x;
+                else a[1] = x;
             }
-            s.a_pthflw[o] = a;
         }
     }
-    s.pthsum[(size_t)m * P + p] = scaled_pathsum(n, s.pthsum_raw + (size_t)m * P, rate_m, p);
-    if (n.ldiag && last) s.a_pthsum[(size_t)m * P + p] = asum;
+    double asum = 0.0;
+    if (n.ldiag && last) asum = level_sum(Lp, t.lane0, a);
+    if (t.on && t.l == 0) {
+        s.pthsum[(size_t)m * P + p] = scaled_pathsum<Coherent>(n, s.pthsum_raw + (size_t)m * P, rate_m, p);
+        if (n.ldiag && last) s.a_pthsum[(size_t)m * P + p] = asum;
+    }
 }
 
 // one cell in phase C; `bput(k, v)` receives the last sub-step's budget term k
 template <class Own, class BPut>
 __device__ __forceinline__ void cell_store(const Net &n, const State &s, const Own &w, int m, int i, double DT,
-                                           bool first, bool last, double nadd, const MemberCtl &c, BPut bput) {
+                                           bool first, bool last, double nadd, int nt, double dt_def, BPut bput) {
     const size_t base = (size_t)m * n.N;
     const size_t gi = base + i;
     const double *rate_m = s.rate + base;
     // the cell's own state is read up front, before anything is stored: in the compiler's view a
     // store may alias any later load of another state array and would hold that load back
-    const double rate_i = w.rate(gi);
+    const auto rate_i = w.rate(gi);
     double rout = w.rivout_raw(gi), fout = w.fldout_raw(gi);
     const double runoff = w.runoff(gi);
     const double rivsto0 = w.rivsto(gi), fldsto0 = w.fldsto(gi), rivdph0 = w.rivdph(gi);
     const double frc = w.fldfrc(gi);
     const double levsto = n.llevee ? w.levsto(gi) : 0.0;
+    // with registers to spare (the resident kernel) the stage scheme's maps come with the gathers; read
+    // where they are used they cost a round of loads of their own
+    StageMap map;
+    if constexpr (Own::kResident) map = stage_map(w, i);
     // own outflow after the LSPAMAT rescale (:456-473)
-    if (i < n.R) {
-        const double r = (rout > 0.0) ? rate_i : rate_m[w.next(i)];
+    if (i < n.R && !(rout > 0.0)) {
+        const double r = w.nb(rate_m, w.next(i));
         rout = rout * r;
         fout = fout * r;
-    } else {
+    } else if constexpr (!Own::kResident) {      // phase B of the resident kernel has done it
         rout = rout * rate_i;
         fout = fout * rate_i;
     }
-    // inflow from the upstream cells, rescaled on the fly (:481-489); next(j) == i
+    // inflow from the upstream cells
     double rinf = 0.0, finf = 0.0;
-    for_each_upstream(n, w, i, [&](int j) {
-        const double rj = s.rivout_raw[base + j], fj = s.fldout_raw[base + j];
-        const double r = (rj > 0.0) ? rate_m[j] : rate_i;
-        rinf = rinf + rj * r;
-        finf = finf + fj * r;
+    w.each_out(base, i, rate_i, [&](double rj, double fj) {
+        rinf = rinf + rj;
+        finf = finf + fj;
     });
     double pout = 0.0;
-    bool has_path = false;
-    if (n.lpthout) {
+    const bool has_path = w.flags() & C_PATH;
+    if (has_path) {
         const double *sum = s.pthsum_raw + (size_t)m * n.P;
-        const int o0 = __ldg(&n.pout_ptr[i]), o1 = __ldg(&n.pout_ptr[i + 1]), f0 = __ldg(&n.pinf_ptr[i]), f1 = __ldg(&n.pinf_ptr[i + 1]);
-        has_path = (o1 > o0) || (f1 > f0);
-        for (int k = o0; k < o1; k++) pout = pout + scaled_pathsum(n, sum, rate_m, __ldg(&n.pout_idx[k]));
-        for (int k = f0; k < f1; k++) pout = pout - scaled_pathsum(n, sum, rate_m, __ldg(&n.pinf_idx[k]));
+        const int q = __ldg(&n.path_pos[i]), e1 = __ldg(&n.pend_ptr[q + 1]);
+        for (int e = __ldg(&n.pend_ptr[q]); e < e1; e++) {
+            const int2 t = __ldg(&n.pend[e]);
+            const bool up = t.x >= 0;              // this cell is the path's upstream end
+            double v = w.nb(sum, up ? t.x : ~t.x);
+            if (t.y == -2) {                       // listed at a cell that is not its end
+                v = scaled_pathsum<Own::kResident>(n, sum, rate_m, up ? t.x : ~t.x);
+            } else if (t.y >= 0) {
+                const double far = w.nb(rate_m, t.y);
+                v = v * ((v >= 0.0) == up ? (double)rate_i : far);
+            }
+            pout = up ? pout + v : pout - v;
+        }
     }
     // CMF_DAMOUT_WATBAL, src/cmf_ctrl_damout_mod.F90:516-535 (the new dam storage is stored below)
     double dmiss = 0.0, damsto1 = 0.0;
-    const int dam = n.ldamout ? __ldg(&n.dam_id[i]) : -1;
-    if (dam >= 0) {
+    const bool dam = w.flags() & C_DAMID;
+    if (dam) {
         const double inflow = (rinf + finf) + runoff;
         const double outflw = rout + fout;
         const double s0 = s.damsto[gi];
@@ -1087,17 +1164,15 @@ __device__ __forceinline__ void cell_store(const Net &n, const State &s, const O
     fs = fs + (runoff * frc) * DT;
     bput(2, n.llevee ? (rs + fs) + levsto : rs + fs);
     // stage scheme, :125
-    const StageOut o = n.llevee ? stage_levee(n, w, i, rs, fs, levsto) : stage_def(n, w, i, rs, fs);
+    if constexpr (!Own::kResident) map = stage_map(w, i);
+    const StageOut o = stage(n, w, i, map, rs, fs, levsto);
     // CALC_VARS_PRE, src/cmf_ctrl_physics_mod.F90:254-277, and the dam storage
-    s.rivout_pre[gi] = rout;
-    s.fldout_pre[gi] = fout;
-    s.rivdph_pre[gi] = rivdph0;
-    s.fldsto_pre[gi] = fldsto0;
-    if (dam >= 0) s.damsto[gi] = damsto1;
+    w.put_pre(gi, rout, fout, rivdph0, fldsto0);
+    if (dam) s.damsto[gi] = damsto1;
     // CMF_CheckNanB-style probe (src/cmf_utils_mod.F90:807-815) on the new storage: a NaN or
     // infinite runoff or state surfaces as a positive status instead of a silent NaN state
     if (!isfinite((o.rivsto + o.fldsto) + o.levsto)) s.ctl[m].err = kErrNonFinite;
-    store_stage(n, s, gi, i, o, last);
+    store_stage(n, s, w, gi, i, o, last);
     bput(5, n.llevee ? (rs + fs) + levsto : rs + fs);
     bput(6, n.llevee ? (o.rivsto + o.fldsto) + o.levsto : o.rivsto + o.fldsto);
     bput(7, o.rivsto);
@@ -1120,7 +1195,7 @@ __device__ __forceinline__ void cell_store(const Net &n, const State &s, const O
         // CMF_DIAG_AVEMAX_OUTPUT (src/cmf_calc_diag_mod.F90:272-318) on the last sub-step: the
         // output interval accumulates the finished sub-step average times DT_DEF
         const bool out = last && n.ldiag_out;
-        const double ddef = c.dt_def;
+        const double ddef = dt_def;
         auto acc = [&](double prev, double *a, double *oa, double v) {
             double x = first ? v * DT : prev + v * DT;
             if (last) x = x / na;
@@ -1134,7 +1209,8 @@ __device__ __forceinline__ void cell_store(const Net &n, const State &s, const O
             const double pof = first ? 0.0 : w.a_outflw(gi);
             const double pmo = first ? 0.0 : w.m_outflw(gi), pmd = first ? 0.0 : w.m_rivdph(gi);
             const double pms = first ? 0.0 : w.m_storge(gi);
-            const double dinf = n.ldamout ? s.daminf[gi] : 0.0, pdi = (first || !n.ldamout) ? 0.0 : s.a_daminf[gi];
+            const double dinf = n.ldamout ? s.daminf[gi] : 0.0;
+            const double pdi = n.ldamout ? daminf_sum(s, gi, w.flags(), DT, nt, dinf) : 0.0;
             acc(pro, s.a_rivout, s.o_rivout, rout);
             acc(pfo, s.a_fldout, s.o_fldout, fout);
             acc(pof, s.a_outflw, s.o_outflw, outflw);
@@ -1142,7 +1218,7 @@ __device__ __forceinline__ void cell_store(const Net &n, const State &s, const O
             // runoff*DT the accumulator would hold, rebuilt in registers on the last sub-step
             const double rdt = runoff * DT;
             double a = rdt;
-            for (int k = 1; k < c.nt; k++) a = a + rdt;
+            for (int k = 1; k < nt; k++) a = a + rdt;
             a = a / na;
             s.a_runoff[gi] = a;
             if (out) s.o_runoff[gi] = s.o_runoff[gi] + a * ddef;
@@ -1190,22 +1266,22 @@ __global__ void __launch_bounds__(kCellThreads, MinBlocks) k_store(Net n, State 
     const bool first = (kk == 0);
     const bool last = (kk == c.nt - 1);
     const double nadd = last ? nadd_before(kk, DT) : 0.0;   // only the averages of the last sub-step need it
+    const int x = blockIdx.x * blockDim.x + threadIdx.x;
     if ((int)blockIdx.x >= ncell_blocks) {
-        const int p = (blockIdx.x - ncell_blocks) * blockDim.x + threadIdx.x;
-        if (p < n.P) path_rescale(n, s, m, p, DT, first, last, nadd, c.dt_def);
+        path_rescale<false>(n, s, m, path_lane(n, x - ncell_blocks * (int)blockDim.x), DT, first, last, nadd, c.dt_def);
         return;
     }
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
     // budget terms of the last sub-step go to shared memory where they are computed (dynamic
     // shared memory, kBudgets x blockDim doubles), so they hold no registers across the stage scheme
     extern __shared__ double sbud[];
     double *bt = sbud + threadIdx.x;
     const int bstride = blockDim.x;
     auto bput = [&](int k, double v) { if (last) bt[k * bstride] = v; };
+    const int i = x;
     if (last && i >= n.N)
 #pragma unroll
         for (int k = 0; k < kBudgets; k++) bt[k * bstride] = 0.0;
-    if (i < n.N) cell_store(n, s, OwnG{n, s}, m, i, DT, first, last, nadd, c, bput);
+    if (i < n.N) cell_store(n, s, OwnG(n, s, __ldg(&n.cflag[i])), m, i, DT, first, last, nadd, c.nt, c.dt_def, bput);
     if (last) {
         double b[kBudgets];
 #pragma unroll

@@ -1,5 +1,6 @@
 // cmf_persist.cuh -- one persistent, cooperative launch per outer step (CMF_PHYSICS_ADVANCE,
-// src/cmf_ctrl_physics_mod.F90:21-153) on sm_100a.
+// src/cmf_ctrl_physics_mod.F90:21-153) on sm_100a, with the state in global memory: the persistent
+// schedule of members too large for the resident kernel (cmf_resident.cuh).
 //
 // The grid is exactly the set of CTAs that are resident at once (cudaLaunchCooperativeKernel); the
 // grid-wide dependencies of the step are software grid barriers:
@@ -49,21 +50,24 @@ struct GridBar {
         epoch++;
         __syncthreads();
         if (threadIdx.x == 0) {
-            __threadfence();
-            atomicAdd(count, 1u);
+            // release: the CTA's writes, ordered before it by the block barrier, are visible to every
+            // thread whose acquire below reads the full count
+            asm volatile("red.release.gpu.global.add.u32 [%0], 1;" :: "l"(count) : "memory");
             const unsigned target = nblocks * epoch;
-            const unsigned long long t0 = globaltimer_ns();
+            unsigned long long t0 = 0;
             int ok = 1;
-            while (ld_acquire(count) < target) {
+            // the error word and the clock are looked at once per 64 polls: they would triple a poll
+            for (int polls = 1; ld_acquire(count) < target; polls++) {
+                if (polls & 63) continue;
                 if (*(volatile int *)err) { ok = 0; break; }
-                if (globaltimer_ns() - t0 > wait_ns) {
+                const unsigned long long now = globaltimer_ns();
+                if (t0 == 0) t0 = now;
+                if (now - t0 > wait_ns) {
                     atomicExch(err, 1);
                     ok = 0;
                     break;
                 }
-                __nanosleep(64);
             }
-            __threadfence();
             *sflag = ok;
         }
         __syncthreads();
@@ -84,7 +88,7 @@ __device__ __forceinline__ TileGeom tile_geom(int t, int tpm, int N) {
 
 struct PersistArgs {
     int tpm;                    // cell tiles per member (ceil(N / kTile))
-    int ppm;                    // path tiles per member (ceil(P / kTile))
+    int ppm;                    // path tiles per member (ceil(path_threads / kTile))
     unsigned long long wait_ns; // bound of every device-side wait
     int selftest;               // 1: only run a barrier whose count can never complete (timeout check)
 };
@@ -118,32 +122,12 @@ __device__ __forceinline__ void ntdt_block(const Net &n, const State &s) {
     long long ntsum = 0, near = 0;
     for (int m = threadIdx.x; m < n.M; m += blockDim.x) {
         MemberCtl &c = s.ctl[m];
-        const double dt_def = c.dt_def;
-        int nt = 1;
-        double dt = dt_def;
-        if (n.ladpstp) {
-            const double dt_min = dmin(dt_def, __longlong_as_double((long long)c.dtmin_bits));
-            c.dt_min = dt_min;
-            const double x = dt_def * (1.0 / dt_min) - CMF_F(0.01);
-            if (!(x >= 0.0) || x > (double)(kNtCap - 1)) {
-                c.err = kErrNtCap;
-                nt = 0;
-            } else {
-                nt = (int)x + 1;
-                dt = dt_def * (double)(1.0f / (float)nt);
-                if (fabs(x - rint(x)) <= 1e-12 * dmax(x, 1.0)) near++;
-            }
-            c.dtmin_bits = (unsigned long long)__double_as_longlong(dt_def);
-        } else {
-            c.dt_min = dt_def;
-        }
-        c.nt = nt;
-        c.dt = dt;
-        c.it = 0;
-        c.nadd = 0.0;
-        ntmax = max(ntmax, nt);
-        ntsum += nt;
-        atomicAdd((unsigned long long *)&s.loop->nt_hist[min(nt, kNtHist - 1)], 1ull);
+        const NtDt r = calc_ntdt(n, c.dt_def, c.dtmin_bits);
+        put_ntdt(c, s.loop, r);
+        if (n.ladpstp) c.dtmin_bits = (unsigned long long)__double_as_longlong(c.dt_def);
+        near += r.near;
+        ntmax = max(ntmax, r.nt);
+        ntsum += r.nt;
     }
     for (int o = 16; o > 0; o >>= 1) {
         ntmax = max(ntmax, __shfl_down_sync(0xffffffffu, ntmax, o));
@@ -196,10 +180,9 @@ __global__ void __launch_bounds__(kTile, kPersistMinBlocks) k_persist(Net n, Sta
         double key = 1.0e308;
         if (i < tg.i1) {
             const size_t gi = (size_t)tg.m * N + i;
-            const OwnG w{n, s};
-            const StageOut o = n.llevee ? stage_levee(n, w, i, s.rivsto[gi], s.fldsto[gi], s.levsto[gi])
-                                        : stage_def(n, w, i, s.rivsto[gi], s.fldsto[gi]);
-            store_stage(n, s, gi, i, o);
+            const OwnG w(n, s, __ldg(&n.cflag[i]));
+            const StageOut o = stage(n, w, i, stage_map(w, i), s.rivsto[gi], s.fldsto[gi], n.llevee ? s.levsto[gi] : 0.0);
+            store_stage(n, s, w, gi, i, o);
             if (n.ladpstp && __ldg(&n.i2mask[i]) == 0) key = cfl_key(n.pcadp, (i < n.R) ? __ldg(&n.nxtdst[i]) : n.pdstmth, n.pgrv, o.rivdph);
         }
         if (n.ladpstp) {
@@ -229,10 +212,14 @@ __global__ void __launch_bounds__(kTile, kPersistMinBlocks) k_persist(Net n, Sta
                 const TileGeom tg = tile_geom(t, tpm, N);
                 const MemberCtl &c = s.ctl[tg.m];
                 const int i = tg.i0 + threadIdx.x;
-                if (k < c.nt && i < tg.i1) cell_outflow(n, s, OwnG{n, s}, tg.m, i, c.dt, c, k, split && k == 0);
+                if (k < c.nt && i < tg.i1) {
+                    const OwnG w(n, s, __ldg(&n.cflag[i]));
+                    cell_outflow(n, s, w, tg.m, i, c.dt, c.nt, c.dt_def, k, split && k == 0);
+                    if (w.flags() & C_DAM) cell_dam(n, s, w, tg.m, i, c.dt, c.nt, c.dt_def, k);
+                }
             } else {
-                const int q = t - T, m = q / ppm, p = (q - m * ppm) * kTile + threadIdx.x;
-                if (k < s.ctl[m].nt && p < n.P) path_outflow(n, s, m, p, s.ctl[m].dt);
+                const int q = t - T, m = q / ppm;
+                if (k < s.ctl[m].nt) path_outflow<false>(n, s, m, path_lane(n, (q - m * ppm) * kTile + threadIdx.x), s.ctl[m].dt);
             }
         }
         if (!gb.sync()) return;
@@ -240,7 +227,7 @@ __global__ void __launch_bounds__(kTile, kPersistMinBlocks) k_persist(Net n, Sta
         for (int t = b; t < T; t += G) {
             const TileGeom tg = tile_geom(t, tpm, N);
             const int i = tg.i0 + threadIdx.x;
-            if (k < s.ctl[tg.m].nt && i < tg.i1) cell_rate(n, s, OwnG{n, s}, tg.m, i, s.ctl[tg.m].dt);
+            if (k < s.ctl[tg.m].nt && i < tg.i1) cell_rate(n, s, OwnG(n, s, __ldg(&n.cflag[i])), tg.m, i, s.ctl[tg.m].dt);
         }
         if (!gb.sync()) return;
         // ---- phase C: rescale, inflow, STONXT, stage scheme, diagnostics; path rescale
@@ -259,7 +246,7 @@ __global__ void __launch_bounds__(kTile, kPersistMinBlocks) k_persist(Net n, Sta
                 if (last && i >= tg.i1)
 #pragma unroll
                     for (int q = 0; q < kBudgets; q++) bt[q * kTile] = 0.0;
-                if (i < tg.i1) cell_store(n, s, OwnG{n, s}, tg.m, i, DT, first, last, nadd, c, bput);
+                if (i < tg.i1) cell_store(n, s, OwnG(n, s, __ldg(&n.cflag[i])), tg.m, i, DT, first, last, nadd, c.nt, c.dt_def, bput);
                 if (last) {
                     double bl[kBudgets];
 #pragma unroll
@@ -267,12 +254,13 @@ __global__ void __launch_bounds__(kTile, kPersistMinBlocks) k_persist(Net n, Sta
                     warp_budget_partials(s, tg.m, i >> 5, budget_warps(N), bl);
                 }
             } else {
-                const int q = t - T, m = q / ppm, p = (q - m * ppm) * kTile + threadIdx.x;
+                const int q = t - T, m = q / ppm;
                 const MemberCtl &c = s.ctl[m];
-                if (k < c.nt && p < n.P) {
+                if (k < c.nt) {
                     const double DT = c.dt;
                     const bool last = (k == c.nt - 1);
-                    path_rescale(n, s, m, p, DT, k == 0, last, last ? nadd_before(k, DT) : 0.0, c.dt_def);
+                    path_rescale<false>(n, s, m, path_lane(n, (q - m * ppm) * kTile + threadIdx.x), DT, k == 0, last,
+                                        last ? nadd_before(k, DT) : 0.0, c.dt_def);
                 }
             }
         }
