@@ -242,10 +242,13 @@ int build_net(cmf_gpu_ctx *c, const cmf_map_ptrs *mp) {
         {&n.rivwth, mp->rivwth, (size_t)N}, {&n.rivhgt, mp->rivhgt, (size_t)N}, {&n.rivlen, mp->rivlen, (size_t)N},
         {&n.rivman, mp->rivman, (size_t)N}, {&n.grarea, mp->grarea, (size_t)N}, {&n.rivstomax, mp->rivstomax, (size_t)N},
         {&n.dwnelv, mp->dwnelv, (size_t)N}};
+    std::vector<double> below(N);
     for (auto &a : arrs) {
         if (!a.src) return set_err(CMF_E_ARG, "a required map pointer is NULL");
         if ((rc = c->upload_raw(a.dst, a.src, a.cnt))) return rc;
     }
+    for (int i = 0; i < N; i++) below[i] = mp->rivelv[next[i] >= 0 ? next[i] : i];
+    if ((rc = c->upload(&n.next_rivelv, below))) return rc;
     // reciprocals the outflow formulas take (x**(-1._JPRB)), correctly rounded once here
     {
         std::vector<double> inv(N);
@@ -480,7 +483,7 @@ int hot_maps_window(cmf_gpu_ctx *c) {
         {(const void **)&n.inv_rivwth, N * 8}, {(const void **)&n.inv_rivlen, N * 8},
         {(const void **)&n.next, N * 4}, {(const void **)&n.up_ptr, (N + 1) * 4}, {(const void **)&n.up_idx, c->E * 4},
         {(const void **)&n.up_ell, N * 4 * cmf::kUpSlots},
-        {(const void **)&n.cflag, N}};
+        {(const void **)&n.next_rivelv, N * 8}, {(const void **)&n.cflag, N}};
     size_t total = 0;
     for (const Item &it : items) total += (it.bytes + 255) & ~(size_t)255;
     int max_persist = 0, max_win = 0;
@@ -536,13 +539,15 @@ int alloc_state(cmf_gpu_ctx *c) {
     const size_t MP = (size_t)c->dims.nmembers * std::max(c->net.P, 1);
     const size_t MPL = (size_t)c->dims.nmembers * std::max(c->net.P * c->net.Lp, 1);
     const bool dg = c->opts.ldiag;
-    double **cell[] = {&s.rivsto, &s.fldsto, &s.rivout_raw, &s.fldout_raw, &s.rivout_pre, &s.fldout_pre,
+    double **cell[] = {&s.rivsto, &s.fldsto, &s.rivout_pre, &s.fldout_pre,
                        &s.rivout_cur, &s.fldout_cur, &s.rivdph_pre, &s.fldsto_pre, &s.rivdph, &s.flddph,
                        &s.fldfrc, &s.fldare, &s.sfcelv, &s.storge, &s.rivvel, &s.rivinf, &s.fldinf, &s.pthout,
                        &s.outflw, &s.rate, &s.runoff};
     int rc;
     for (double **p : cell)
         if ((rc = c->alloc(p, MN))) return rc;
+    if ((rc = c->alloc(&s.raw, MN)) || (rc = c->alloc(&s.out, MN)) || (rc = c->alloc(&s.dph, MN)) || (rc = c->alloc(&s.wet, MN)))
+        return rc;
     const size_t opt_cells[] = {c->opts.llevee ? MN : 1, c->opts.ldamout ? MN : 1};
     if ((rc = c->alloc(&s.levsto, opt_cells[0])) || (rc = c->alloc(&s.levdph, opt_cells[0]))) return rc;
     if ((rc = c->alloc(&s.damsto, opt_cells[1])) || (rc = c->alloc(&s.daminf, opt_cells[1]))) return rc;
@@ -596,9 +601,9 @@ void launch_store(cmf_gpu_ctx *c) {
         cmf::k_store<cmf::kStoreMinBlocksWide><<<g, q.bs, cmf::store_smem(q.bs), c->stream>>>(c->net, c->st, nc);
 }
 constexpr int kStageBlock = 256;   // stage + CFL kernel (once per outer step)
-void launch_stage(cmf_gpu_ctx *c) {
+void launch_stage(cmf_gpu_ctx *c, bool begin = true) {
     const dim3 g(nblk(c->dims.nseqall, kStageBlock), c->dims.nmembers);
-    cmf::k_stage<<<g, kStageBlock, 0, c->stream>>>(c->net, c->st);
+    cmf::k_stage<<<g, kStageBlock, 0, c->stream>>>(c->net, c->st, begin ? 1 : 0);
 }
 
 // Enqueue one sub-step (phases A, B, C).
@@ -856,7 +861,7 @@ int read_ctl(cmf_gpu_ctx *c) {
 int zero_state(cmf_gpu_ctx *c) {
     const size_t MN = (size_t)c->dims.nmembers * c->dims.nseqall;
     cmf::State &s = c->st;
-    for (double *p : {s.rivsto, s.fldsto, s.rivout_raw, s.fldout_raw, s.rivout_pre, s.fldout_pre, s.rivout_cur, s.fldout_cur,
+    for (double *p : {s.rivsto, s.fldsto, s.rivout_pre, s.fldout_pre, s.rivout_cur, s.fldout_cur,
                       s.rivdph_pre, s.fldsto_pre, s.rivdph, s.flddph, s.fldfrc, s.fldare, s.sfcelv, s.storge, s.rivvel,
                       s.rivinf, s.fldinf, s.pthout, s.outflw, s.rate})
         CUDA_TRY(cudaMemsetAsync(p, 0, MN * sizeof(double), c->stream));
@@ -1803,7 +1808,7 @@ int cmf_gpu_ctx_stage(cmf_gpu_ctx *c, double dt_def, double *dt_min_local) {
     CUDA_TRY(cudaSetDevice(c->device));
     int rc;
     if ((rc = sync_dt_def(c, dt_def))) return rc;
-    launch_stage(c);
+    launch_stage(c, false);
     CUDA_TRY(cudaGetLastError());
     c->launches += 1;
     if ((rc = read_ctl(c))) return rc;
@@ -1832,6 +1837,7 @@ int cmf_gpu_ctx_substeps(cmf_gpu_ctx *c, double dt_def, double dt_min_global, in
     }
     CUDA_TRY(cudaMemcpyAsync(c->st.ctl, c->hctl.data(), c->hctl.size() * sizeof(cmf::MemberCtl), cudaMemcpyHostToDevice, c->stream));
     c->dt_def_dev = dt_def;
+    cmf::k_begin<<<dim3(nblk(c->dims.nseqall, kStageBlock), c->dims.nmembers), kStageBlock, 0, c->stream>>>(c->net, c->st);
     cmf::k_ntdt<<<1, 256, 0, c->stream>>>(c->net, c->st, c->cond, 0);
     CUDA_TRY(cudaGetLastError());
     cmf::LoopCtl lc;
@@ -1840,7 +1846,7 @@ int cmf_gpu_ctx_substeps(cmf_gpu_ctx *c, double dt_def, double dt_min_global, in
     for (int k = 0; k < lc.ntmax; k++) enqueue_substep(c, 0);
     enqueue_epilogue(c);
     CUDA_TRY(cudaGetLastError());
-    c->launches += 2 + 3LL * lc.ntmax;
+    c->launches += 3 + 3LL * lc.ntmax;
     const int saved = c->opts.launch_mode;
     c->opts.launch_mode = 1;
     int rc = finish_outer(c, nt_out, dt_out, b);
@@ -1955,7 +1961,7 @@ __global__ void k_noalloc_stage(cmf::Net n, cmf::State s, double *blockmin) {
     if (i < n.N) {
         const cmf::OwnG w{n, s};
         const cmf::StageOut o = cmf::stage(n, w, i, cmf::stage_map(w, i), s.rivsto[i], s.fldsto[i], 0.0);
-        cmf::store_stage(n, s, w, i, i, o);
+        cmf::put_full_stage(n, s, i, i, o);
         if (n.ladpstp && n.i2mask[i] == 0)
             key = cmf::cfl_key(n.pcadp, (i < n.R) ? n.nxtdst[i] : n.pdstmth, n.pgrv, o.rivdph);
     }

@@ -31,13 +31,12 @@ namespace cmf {
 
 // Occupancy of the latency-bound cell kernels: at most kCellThreads threads per block and the
 // minimum resident blocks per SM (caps registers at 65536 / (threads x blocks)).  k_flux and
-// k_store come in two profiles, one of the dimensions the engine's autotuner searches: with many
-// cell-members in flight more resident warps beat the spills they cost (`wide`: 40/48 registers;
-// 16 config-1 members 22.2 vs 24.4 ms per coupling step), while a grid of about two waves runs
-// best with few spills (`small`: 64/64 registers, k_flux spill-free; one config-1 member 1.91 ms
-// vs 1.95 ms with k_flux at 48).  Both profiles execute the same arithmetic; only the register
-// allocation differs.
-constexpr int kFluxMinBlocksWide = 6, kStoreMinBlocksWide = 5;
+// k_store come in two profiles, one of the dimensions the engine's autotuner searches.  Measured per
+// launch (us; 16 members of 298,554 cells | one of 1,997,296): k_flux at 6 blocks 262 | 126, 5 blocks 223 |
+// 117, 4 blocks 228 | 120, 3 blocks 263 | 135; k_store at 5 blocks 270 | 130, 4 blocks 268 | 135, 3 blocks
+// 309 | 159; k_rate at 8 blocks 90 | 49, 6 blocks 88 | 49, 4 blocks 117 | 64.  Both profiles execute the
+// same arithmetic; only the register allocation differs.
+constexpr int kFluxMinBlocksWide = 5, kStoreMinBlocksWide = 5;
 constexpr int kFluxMinBlocksSmall = 4, kStoreMinBlocksSmall = 4;
 constexpr size_t kSmallCellMembers = size_t(1) << 19;   // untuned start: `small` up to this many cell-members
 #ifndef CMF_STAGE_MINB
@@ -100,6 +99,7 @@ struct Net {
     const double *__restrict__ rivelv, *__restrict__ elevtn, *__restrict__ nxtdst, *__restrict__ rivwth;
     const double *__restrict__ rivhgt, *__restrict__ rivlen, *__restrict__ rivman, *__restrict__ grarea;
     const double *__restrict__ rivstomax, *__restrict__ dwnelv;
+    const double *__restrict__ next_rivelv;  // [N] D2RIVELV of the downstream cell (its own at mouths)
     // D2NXTDST**(-1), D2RIVWTH**(-1), D2RIVLEN**(-1) of the outflow formulas, computed once at init
     // (the same correctly rounded reciprocal the reference evaluates every time)
     const double *__restrict__ inv_nxtdst, *__restrict__ inv_rivwth, *__restrict__ inv_rivlen;
@@ -148,10 +148,25 @@ enum CellFlag : unsigned {
     C_LEV = 16                 // levee parameters
 };
 
+// What the phase kernels keep per cell beside the arrays (State::wet): which of the arrays that are zero
+// in most cells hold something.  A clear bit means that they hold +0, so a dry cell neither reads nor
+// writes them (about 110 of 540 B per cell and sub-step); the averages' bits are of the running outer step.
+enum WetBit : unsigned {
+    W_STAGE = 1,               // fldsto, flddph, fldfrc, levsto, levdph
+    W_PRE = 2,                 // fldsto_pre
+    W_FOUT = 4,                // fldout_pre
+    W_AFLD = 8,                // a_fldout has been started (else 0)
+    W_AOUT = 16                // a_outflw has parted from a_rivout (else equal: fldout was +0 so far)
+};
+
 // Per-member state, member-major [M][N] (paths [M][Lp][P] / [M][P]).
 struct State {
     double *rivsto, *fldsto, *levsto, *damsto, *daminf;
-    double *rivout_raw, *fldout_raw;          // outflow before the LSPAMAT rescale (phase A -> C)
+    // (river, floodplain) outflow before the LSPAMAT rescale (phase A -> B), and after it where the cell's
+    // own rate applies (B -> C): one 16-byte element per neighbour gather
+    double2 *raw, *out;
+    double2 *dph;                             // (D2RIVDPH, D2RIVDPH_PRE) during the sub-steps of the phase kernels
+    unsigned char *wet;                       // WetBit
     double *rivout_pre, *fldout_pre;          // D2RIVOUT_PRE / D2FLDOUT_PRE (== D2RIVOUT / D2FLDOUT after a step)
     double *rivout_cur, *fldout_cur;          // host-set D2RIVOUT / D2FLDOUT while LoopCtl.split
     double *rivdph_pre, *fldsto_pre;
@@ -192,50 +207,80 @@ struct OwnMaps {
     __device__ __forceinline__ int up_slot(int k, int i) const { return __ldg(&n.up_ell[(size_t)k * n.N + i]); }
     __device__ __forceinline__ int i1dam(int i) const { return __ldg(&n.i1dam[i]); }
 };
+struct LazyRate;
 struct DownCell {
     double rivelv, rivdph, rivdph_pre;
 };
 struct OwnG : OwnMaps {
     static constexpr bool kResident = false;
     const State &s;
-    unsigned fl;               // the cell's CellFlag bits
-    __device__ __forceinline__ OwnG(const Net &n_, const State &s_, unsigned fl_ = 0u) : OwnMaps{n_}, s(s_), fl(fl_) {}
+    unsigned fl, wet;          // the cell's CellFlag and WetBit bits
+    __device__ __forceinline__ OwnG(const Net &n_, const State &s_, unsigned fl_ = 0u, unsigned wet_ = 0u)
+        : OwnMaps{n_}, s(s_), fl(fl_), wet(wet_) {}
     __device__ __forceinline__ unsigned flags() const { return fl; }
-    CMF_OWN_STATE(rivsto) CMF_OWN_STATE(fldsto) CMF_OWN_STATE(levsto) CMF_OWN_STATE(rivdph)
-    CMF_OWN_STATE(rivdph_pre) CMF_OWN_STATE(rivout_pre) CMF_OWN_STATE(fldout_pre) CMF_OWN_STATE(fldsto_pre)
-    CMF_OWN_STATE(flddph) CMF_OWN_STATE(fldfrc) CMF_OWN_STATE(storge) CMF_OWN_STATE(runoff)
-    CMF_OWN_STATE(rivout_raw) CMF_OWN_STATE(fldout_raw) CMF_OWN_STATE(rate)
-    CMF_OWN_STATE(a_rivvel) CMF_OWN_STATE(a_rivout) CMF_OWN_STATE(a_fldout) CMF_OWN_STATE(a_outflw)
+    CMF_OWN_STATE(rivsto) CMF_OWN_STATE(rivout_pre) CMF_OWN_STATE(runoff) CMF_OWN_STATE(a_rivvel) CMF_OWN_STATE(a_rivout)
     CMF_OWN_STATE(a_pthout) CMF_OWN_STATE(m_outflw) CMF_OWN_STATE(m_rivdph) CMF_OWN_STATE(m_storge)
+    __device__ __forceinline__ LazyRate rate(size_t g) const;
+#define CMF_OWN_SPARSE(name, bit) \
+    __device__ __forceinline__ double name(size_t g) const { return (wet & bit) ? s.name[g] : 0.0; }
+    CMF_OWN_SPARSE(fldsto, W_STAGE) CMF_OWN_SPARSE(flddph, W_STAGE) CMF_OWN_SPARSE(fldfrc, W_STAGE)
+    CMF_OWN_SPARSE(levsto, W_STAGE) CMF_OWN_SPARSE(fldsto_pre, W_PRE) CMF_OWN_SPARSE(fldout_pre, W_FOUT)
+    CMF_OWN_SPARSE(a_fldout, W_AFLD)
+#undef CMF_OWN_SPARSE
+    __device__ __forceinline__ double a_outflw(size_t g) const { return (wet & W_AOUT) ? s.a_outflw[g] : s.a_rivout[g]; }
+    __device__ __forceinline__ double rivdph(size_t g) const { return s.dph[g].x; }
+    __device__ __forceinline__ double rivdph_pre(size_t g) const { return s.dph[g].y; }
+    __device__ __forceinline__ double2 own_raw(size_t g) const { return s.raw[g]; }
+    __device__ __forceinline__ double2 own_out(size_t g) const { return s.out[g]; }
     __device__ __forceinline__ double nb(const double *p, size_t g) const { return p[g]; }
-    __device__ __forceinline__ DownCell down(size_t base, int j) const {
-        return {__ldg(&n.rivelv[j]), s.rivdph[base + j], s.rivdph_pre[base + j]};
+    __device__ __forceinline__ DownCell down(size_t base, int i, int j) const {
+        const double2 d = s.dph[base + j];
+        return {__ldg(&n.next_rivelv[i]), d.x, d.y};
     }
-    __device__ __forceinline__ void put_raw(size_t g, int, double rout, double fout) const {
-        s.rivout_raw[g] = rout;
-        s.fldout_raw[g] = fout;
-    }
-    __device__ __forceinline__ void put_rate(size_t g, int, double, double, double rate) const { s.rate[g] = rate; }
-    __device__ __forceinline__ void put_a_rivvel(size_t g, double v) const { s.a_rivvel[g] = v; }
-    // CALC_VARS_PRE (src/cmf_ctrl_physics_mod.F90:254-277)
-    __device__ __forceinline__ void put_pre(size_t g, double rout, double fout, double dph, double fld) const {
-        s.rivout_pre[g] = rout;
-        s.fldout_pre[g] = fout;
-        s.rivdph_pre[g] = dph;
-        s.fldsto_pre[g] = fld;
-    }
-    template <class Out>
-    __device__ __forceinline__ void put_stage(size_t g, const Out &o, double storge) const {
-        s.rivsto[g] = o.rivsto;
-        s.fldsto[g] = o.fldsto;
-        s.rivdph[g] = o.rivdph;
-        s.flddph[g] = o.flddph;
-        s.fldfrc[g] = o.fldfrc;
-        if (n.llevee) {
-            s.levsto[g] = o.levsto;
-            s.levdph[g] = o.levdph;
+    __device__ __forceinline__ void put_raw(size_t g, int, double rout, double fout) const { s.raw[g] = make_double2(rout, fout); }
+    // a positive outflow (and a mouth's) is rescaled by its own cell's rate here, and its gatherer takes
+    // the product; a reverse one keeps its value (not > 0) and is multiplied by the gatherer's rate
+    __device__ __forceinline__ void put_rate(size_t g, int i, double rout, double fout, double r) const {
+        s.rate[g] = r;
+        if (rout > 0.0 || i >= n.R) {
+            rout = rout * r;
+            fout = fout * r;
         }
-        s.storge[g] = storge;
+        s.out[g] = make_double2(rout, fout);
+    }
+    __device__ __forceinline__ void put_a_rivvel(size_t g, double v) const { s.a_rivvel[g] = v; }
+    // an array that holds +0 while `bit` is clear
+    __device__ __forceinline__ void put_sparse(unsigned bit, double *p, size_t g, double v) {
+        const bool some = __double_as_longlong(v) != 0;
+        if (some || (wet & bit)) p[g] = v;
+        wet = some ? wet | bit : wet & ~bit;
+    }
+    // CALC_VARS_PRE (src/cmf_ctrl_physics_mod.F90:254-277)
+    __device__ __forceinline__ void put_pre(size_t g, double rout, double fout, double dph, double fld, bool last) {
+        s.rivout_pre[g] = rout;
+        put_sparse(W_FOUT, s.fldout_pre, g, fout);
+        put_sparse(W_PRE, s.fldsto_pre, g, fld);
+        if (last) s.rivdph_pre[g] = dph;
+    }
+    // `dph`: the depth this one replaces (CALC_VARS_PRE's)
+    template <class Out>
+    __device__ __forceinline__ void put_stage(size_t g, const Out &o, double storge, double dph, bool last) {
+        s.rivsto[g] = o.rivsto;
+        s.dph[g] = make_double2(o.rivdph, dph);
+        const bool some = (__double_as_longlong(o.fldsto) | __double_as_longlong(o.flddph) | __double_as_longlong(o.fldfrc) |
+                           __double_as_longlong(o.levsto) | __double_as_longlong(o.levdph)) != 0;
+        if (some || (wet & W_STAGE)) {
+            s.fldsto[g] = o.fldsto;
+            s.flddph[g] = o.flddph;
+            s.fldfrc[g] = o.fldfrc;
+            if (n.llevee) {
+                s.levsto[g] = o.levsto;
+                s.levdph[g] = o.levdph;
+            }
+        }
+        wet = some ? wet | W_STAGE : wet & ~W_STAGE;
+        if (last) s.rivdph[g] = o.rivdph;
+        if (last || (fl & C_PATH)) s.storge[g] = storge;      // read by the paths at this cell
     }
     // f(rivout, fldout) before the LSPAMAT rescale of every upstream cell, in I1UPST order: the CSR
     // walk, since at k_rate's full occupancy the slot table's 16 B per cell cost more than its saved round
@@ -243,13 +288,19 @@ struct OwnG : OwnMaps {
     __device__ __forceinline__ void each_raw(size_t base, int i, F f) const {
         const int u1 = up_hi(i);
         for (int k = up_lo(i); k < u1; k++) {
-            const int j = __ldg(&n.up_idx[k]);
-            f(s.rivout_raw[base + j], s.fldout_raw[base + j]);
+            const double2 v = s.raw[base + __ldg(&n.up_idx[k])];
+            f(v.x, v.y);
         }
     }
     // f(rivout, fldout) after the rescale (:481-489); next(j) == i, so a reverse flow takes rate_i
-    template <class F>
-    __device__ __forceinline__ void each_out(size_t base, int i, double rate_i, F f) const;
+    template <class Rate, class F>
+    __device__ __forceinline__ void each_out(size_t base, int i, Rate rate_i, F f) const;
+};
+// the cell's rate, read only where a reverse flow or a path needs it
+struct LazyRate {
+    const double *p;
+    bool cg;                   // past L1: other CTAs of the same launch wrote it
+    __device__ __forceinline__ operator double() const { return cg ? __ldcg(p) : *p; }
 };
 #undef CMF_OWN_STATIC
 #undef CMF_OWN_STATE
@@ -282,15 +333,21 @@ __device__ __forceinline__ void for_each_upstream(const Net &n, const Own &w, in
         }
     }
 }
-template <class F>
-__device__ __forceinline__ void OwnG::each_out(size_t base, int i, double rate_i, F f) const {
-    const double *rate_m = s.rate + base;
-    for_each_upstream(n, *this, i, [&](int j) {
-        const double rj = s.rivout_raw[base + j], fj = s.fldout_raw[base + j];
-        const double r = (rj > 0.0) ? rate_m[j] : rate_i;
-        f(rj * r, fj * r);
-    });
+__device__ __forceinline__ LazyRate OwnG::rate(size_t g) const { return {s.rate + g, false}; }
+template <class Rate, class F>
+__device__ __forceinline__ void rescaled(double2 v, Rate rate_i, F f) {
+    if (!(v.x > 0.0) && !(v.x == 0.0 && v.y == 0.0)) {        // zeros stay zeros
+        const double r = rate_i;
+        v.x = v.x * r;
+        v.y = v.y * r;
+    }
+    f(v.x, v.y);
 }
+template <class Rate, class F>
+__device__ __forceinline__ void OwnG::each_out(size_t base, int i, Rate rate_i, F f) const {
+    for_each_upstream(n, *this, i, [&](int j) { rescaled(s.out[base + j], rate_i, f); });
+}
+
 
 // x**(-7._JPRB/3._JPRB) and x**(-4._JPRB/3._JPRB) of the local-inertial flux formulas
 // (src/cmf_calc_outflw_mod.F90:74,106,133,162; src/cmf_calc_pthout_mod.F90:67;
@@ -514,15 +571,44 @@ __device__ __forceinline__ StageOut stage(const Net &n, const Own &w, int i, con
 }
 
 // D2FLDARE and D2SFCELV are read by nothing inside the sub-step loop, so the sub-steps write them on
-// the last sub-step only (diag_out; the values the caller observes are the same)
+// the last sub-step only (the values the caller observes are the same)
 template <class Own>
-__device__ __forceinline__ void store_stage(const Net &n, const State &s, const Own &w, size_t gi, int i, const StageOut &o,
-                                            bool diag_out = true) {
-    if (diag_out) {
+__device__ __forceinline__ void store_stage(const Net &n, const State &s, Own &w, size_t gi, int i, const StageOut &o,
+                                            double dph, bool last) {
+    if (last) {
         s.fldare[gi] = o.fldare;
         s.sfcelv[gi] = w.rivelv(i) + o.rivdph;
     }
-    w.put_stage(gi, o, n.llevee ? (o.rivsto + o.fldsto) + o.levsto : o.rivsto + o.fldsto);
+    w.put_stage(gi, o, n.llevee ? (o.rivsto + o.fldsto) + o.levsto : o.rivsto + o.fldsto, dph, last);
+}
+
+// The stage scheme at the top of a step: every array, whatever the host or the emulator left in them
+__device__ __forceinline__ void put_full_stage(const Net &n, const State &s, size_t gi, int i, const StageOut &o) {
+    s.rivsto[gi] = o.rivsto;
+    s.fldsto[gi] = o.fldsto;
+    s.rivdph[gi] = o.rivdph;
+    s.flddph[gi] = o.flddph;
+    s.fldfrc[gi] = o.fldfrc;
+    s.fldare[gi] = o.fldare;
+    s.sfcelv[gi] = __ldg(&n.rivelv[i]) + o.rivdph;
+    if (n.llevee) {
+        s.levsto[gi] = o.levsto;
+        s.levdph[gi] = o.levdph;
+        s.storge[gi] = (o.rivsto + o.fldsto) + o.levsto;
+    } else {
+        s.storge[gi] = o.rivsto + o.fldsto;
+    }
+}
+// What the sub-steps of the phase kernels keep beside the arrays, from the arrays
+__device__ __forceinline__ void begin_cell(const Net &n, const State &s, size_t gi, double rivdph, double fldsto, double flddph,
+                                           double fldfrc, double levsto, double levdph) {
+    auto some = [](double v) { return __double_as_longlong(v) != 0; };
+    unsigned w = 0u;
+    if (some(fldsto) || some(flddph) || some(fldfrc) || some(levsto) || some(levdph)) w |= W_STAGE;
+    if (some(s.fldsto_pre[gi])) w |= W_PRE;
+    if (some(s.fldout_pre[gi])) w |= W_FOUT;
+    s.wet[gi] = (unsigned char)w;
+    s.dph[gi] = make_double2(rivdph, s.rivdph_pre[gi]);
 }
 
 template <int NV>
@@ -549,7 +635,8 @@ __device__ __forceinline__ void block_sum(double (&v)[NV], double *smem /* [32*N
 // ------------------------------------------------------------------------------------------
 // k_stage: stage scheme at the top of CMF_PHYSICS_ADVANCE + CALC_ADPSTP minimum
 // ------------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(kCellThreads, CMF_STAGE_MINB) k_stage(Net n, State s) {
+// begin: sub-steps of the phase kernels follow in the same step
+__global__ void __launch_bounds__(kCellThreads, CMF_STAGE_MINB) k_stage(Net n, State s, int begin) {
     const int m = blockIdx.y;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     double key = 1.0e308;
@@ -557,7 +644,8 @@ __global__ void __launch_bounds__(kCellThreads, CMF_STAGE_MINB) k_stage(Net n, S
         const size_t gi = (size_t)m * n.N + i;
         const OwnG w(n, s, __ldg(&n.cflag[i]));
         const StageOut o = stage(n, w, i, stage_map(w, i), s.rivsto[gi], s.fldsto[gi], n.llevee ? s.levsto[gi] : 0.0);
-        store_stage(n, s, w, gi, i, o);
+        put_full_stage(n, s, gi, i, o);
+        if (begin) begin_cell(n, s, gi, o.rivdph, o.fldsto, o.flddph, o.fldfrc, o.levsto, o.levdph);
         if (n.ladpstp && __ldg(&n.i2mask[i]) == 0) key = cfl_key(n.pcadp, (i < n.R) ? __ldg(&n.nxtdst[i]) : n.pdstmth, n.pgrv, o.rivdph);
     }
     if (n.ladpstp) {
@@ -572,6 +660,15 @@ __global__ void __launch_bounds__(kCellThreads, CMF_STAGE_MINB) k_stage(Net n, S
             if (lane == 0 && x < 1.0e308) atomicMin(&s.ctl[m].dtmin_bits, (unsigned long long)__double_as_longlong(x));
         }
     }
+}
+
+// begin_cell for sub-steps that follow a stage scheme of an earlier call
+__global__ void k_begin(Net n, State s) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n.N) return;
+    const size_t gi = (size_t)blockIdx.y * n.N + i;
+    begin_cell(n, s, gi, s.rivdph[gi], s.fldsto[gi], s.flddph[gi], s.fldfrc[gi], n.llevee ? s.levsto[gi] : 0.0,
+               n.llevee ? s.levdph[gi] : 0.0);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -674,11 +771,10 @@ __device__ __forceinline__ double rate_min1(double a, double b) { return (a >= b
 __device__ __forceinline__ bool same_bits(double a, double b) {
     return __double_as_longlong(a) == __double_as_longlong(b);
 }
-__device__ __forceinline__ void diag_carry(const State &s, size_t gi, double DT, bool first, double rivout, double fldout,
-                                           double rivdph, double storge) {
+__device__ __forceinline__ void diag_carry(const State &s, OwnG &w, size_t gi, double DT, bool first, double rivout,
+                                           double fldout, double rivdph, double storge) {
     const double outflw = rivout + fldout;
-    const double pro = first ? 0.0 : s.a_rivout[gi], pfo = first ? 0.0 : s.a_fldout[gi];
-    const double pof = first ? 0.0 : s.a_outflw[gi], pmo = first ? 0.0 : s.m_outflw[gi];
+    const double pro = first ? 0.0 : s.a_rivout[gi], pmo = first ? 0.0 : s.m_outflw[gi];
     const double pmd = first ? 0.0 : s.m_rivdph[gi], pms = first ? 0.0 : s.m_storge[gi];
     // a store is skipped when the sub-step leaves the accumulator's bits unchanged (a zero discharge
     // added to a running sum, a maximum that did not move): the array holds the same bits either way
@@ -686,9 +782,17 @@ __device__ __forceinline__ void diag_carry(const State &s, size_t gi, double DT,
         const double x = first ? v * DT : prev + v * DT;
         if (first || !same_bits(x, prev)) a[gi] = x;
     };
+    if (!same_bits(outflw, rivout) || (!first && (w.wet & W_AOUT))) {
+        const double prev = first ? 0.0 : (w.wet & W_AOUT) ? s.a_outflw[gi] : pro;
+        s.a_outflw[gi] = first ? outflw * DT : prev + outflw * DT;
+        w.wet |= W_AOUT;
+    }
     acc(pro, s.a_rivout, rivout);
-    acc(pfo, s.a_fldout, fldout);
-    acc(pof, s.a_outflw, outflw);
+    if (__double_as_longlong(fldout) != 0 || (!first && (w.wet & W_AFLD))) {
+        const double prev = first ? 0.0 : w.a_fldout(gi);
+        s.a_fldout[gi] = first ? fldout * DT : prev + fldout * DT;
+        w.wet |= W_AFLD;
+    }
     const double mo = dmax(pmo, fabs(outflw));
     const double md = dmax(pmd, rivdph);
     const double ms = dmax(pms, storge);
@@ -803,7 +907,7 @@ __device__ __forceinline__ void cell_dam(const Net &n, const State &s, const Own
 }
 
 template <class Own>
-__device__ __forceinline__ void cell_outflow(const Net &n, const State &s, const Own &w, int m, int i, double DT,
+__device__ __forceinline__ void cell_outflow(const Net &n, const State &s, Own &w, int m, int i, double DT,
                                              int nt, double dt_def, int k, bool split) {
     const size_t base = (size_t)m * n.N, gi = base + i;
     const double gdt = n.pgrv * DT;
@@ -816,12 +920,13 @@ __device__ __forceinline__ void cell_outflow(const Net &n, const State &s, const
     const double man = w.rivman(i);
     const double rivout_pre = w.rivout_pre(gi);
     const double rivout_old = split ? s.rivout_cur[gi] : rivout_pre;
-    const double fldout_pre = w.fldout_pre(gi), storge = w.storge(gi);
+    const double fldout_pre = w.fldout_pre(gi), fsto = w.fldsto(gi), riv_fld = w.rivsto(gi) + fsto;
+    const double storge = n.llevee ? riv_fld + w.levsto(gi) : riv_fld;      // D2STORGE of the stage scheme
     // river cells see the downstream cell's surface; a mouth the boundary elevation, over its own depth
     const bool river = i < n.R;
     double dwn, inv_dst, dsfc = sfc, dsfc_pre = sfc_pre, dflw = rivdph, dflw_pr = rivdph_pre;
     if (river) {
-        const DownCell below = w.down(base, w.next(i));
+        const DownCell below = w.down(base, i, w.next(i));
         dwn = below.rivelv + below.rivdph;
         inv_dst = w.inv_nxtdst(i);
         dsfc = dmax(sfc, dwn);
@@ -849,7 +954,7 @@ __device__ __forceinline__ void cell_outflow(const Net &n, const State &s, const
         // the reference's masks are a double at river cells and a default-real literal at mouths
         const double eps = river ? 1.E-5 : CMF_F(1.E-5);
         // without floodplain water the area is max(-FLDDPH * RIVWTH, 0) = 0: nothing more to read
-        const double fsto = w.fldsto(gi), inv_len = fsto != 0.0 ? w.inv_rivlen(i) : 0.0;
+        const double inv_len = fsto != 0.0 ? w.inv_rivlen(i) : 0.0;
         const double dare = fsto != 0.0 ? dmax(fsto * inv_len - w.flddph(gi) * wth, 0.0) : 0.0;
         if (dare > eps) {
             const double elv = w.elevtn(i);
@@ -877,7 +982,7 @@ __device__ __forceinline__ void cell_outflow(const Net &n, const State &s, const
     if (!(w.flags() & C_DAM)) w.put_raw(gi, i, rout, fout);
     if (n.ldiag && k > 0) {              // diagnostics of sub-step k-1
         if constexpr (Own::kResident) w.carry(gi, DT, k == 1, rivout_pre, fldout_pre, rivdph, storge);
-        else diag_carry(s, gi, DT, k == 1, rivout_pre, fldout_pre, rivdph, storge);
+        else diag_carry(s, w, gi, DT, k == 1, rivout_pre, fldout_pre, rivdph, storge);
     }
     if (!(w.flags() & C_KIN)) vel_average(n, s, w, gi, DT, nt, dt_def, k, rvel);
 }
@@ -893,6 +998,12 @@ __device__ __forceinline__ double path_flux(double wth, double pre, double gdt, 
 // several phases)
 template <bool Coherent>
 __device__ __forceinline__ double ld_nb(const double *p, size_t g) { return Coherent ? __ldcg(p + g) : p[g]; }
+
+template <bool Coherent>
+__device__ __forceinline__ double2 end_depth(const State &s, size_t g) {
+    if constexpr (Coherent) return make_double2(__ldcg(s.rivdph + g), __ldcg(s.rivdph_pre + g));
+    else return s.dph[g];
+}
 
 // Bifurcation paths by lanes: thread x of the path threads takes level l of path p, 32 / Lp paths per
 // warp, the lanes of a path consecutive from lane0 (one thread per path ran its levels' powers one after
@@ -932,7 +1043,8 @@ __device__ __forceinline__ void path_outflow(const Net &n, const State &s, int m
         d = __ldg(&n.pth_dn[p]);
         const double gdt = n.pgrv * DT;
         const double eu = __ldg(&n.rivelv[u]), ed = __ldg(&n.rivelv[d]);
-        const double su = eu + ld_nb<Coherent>(s.rivdph, base + u), sd = ed + ld_nb<Coherent>(s.rivdph, base + d);
+        const double2 du = end_depth<Coherent>(s, base + u), dd = end_depth<Coherent>(s, base + d);
+        const double su = eu + du.x, sd = ed + dd.x;
         double dslp = (su - sd) / __ldg(&n.pth_dst[p]);
         dslp = dmax(-0.005, dmin(0.005, dslp));
 #pragma unroll 1
@@ -943,7 +1055,7 @@ __device__ __forceinline__ void path_outflow(const Net &n, const State &s, int m
             const bool channel = !n.llevee || l == 0;    // with levees: level 1, the river channel
             double im;
             if (channel) {
-                const double spu = eu + ld_nb<Coherent>(s.rivdph_pre, base + u), spd = ed + ld_nb<Coherent>(s.rivdph_pre, base + d);
+                const double spu = eu + du.y, spd = ed + dd.y;
                 const double dflw = dmax(dmax(su, sd) - elv, 0.0);
                 const double dflw_pr = dmax(dmax(spu, spd) - elv, 0.0);
                 im = sqrt(dflw * dflw_pr);
@@ -975,6 +1087,21 @@ __device__ __forceinline__ void path_outflow(const Net &n, const State &s, int m
     }
 }
 
+__device__ __forceinline__ OwnG own_cell(const Net &n, const State &s, int m, int i) {
+    return OwnG(n, s, __ldg(&n.cflag[i]), s.wet[(size_t)m * n.N + i]);
+}
+__device__ __forceinline__ void put_wet(const Net &n, const State &s, int m, int i, unsigned before, unsigned now) {
+    if (now != before) s.wet[(size_t)m * n.N + i] = (unsigned char)now;
+}
+// one cell of phase A
+__device__ __forceinline__ void flux_cell(const Net &n, const State &s, int m, int i, double DT, int nt, double dt_def, int k,
+                                          bool split) {
+    OwnG w = own_cell(n, s, m, i);
+    const unsigned before = w.wet;
+    cell_outflow(n, s, w, m, i, DT, nt, dt_def, k, split);
+    put_wet(n, s, m, i, before, w.wet);
+}
+
 // Blocks of phase A: cells, then (path, level) lanes, then dam cells
 template <int MinBlocks>
 __global__ void __launch_bounds__(kCellThreads, MinBlocks) k_flux(Net n, State s, int ncell_blocks, int npath_blocks) {
@@ -986,14 +1113,14 @@ __global__ void __launch_bounds__(kCellThreads, MinBlocks) k_flux(Net n, State s
     const double DT = c.dt;
     const int x = blockIdx.x * blockDim.x + threadIdx.x;
     if ((int)blockIdx.x < ncell_blocks) {
-        if (x < n.N) cell_outflow(n, s, OwnG(n, s, __ldg(&n.cflag[x])), m, x, DT, c.nt, c.dt_def, k, s.loop->split != 0);
+        if (x < n.N) flux_cell(n, s, m, x, DT, c.nt, c.dt_def, k, s.loop->split != 0);
     } else if ((int)blockIdx.x < ncell_blocks + npath_blocks) {
         path_outflow<false>(n, s, m, path_lane(n, x - ncell_blocks * (int)blockDim.x), DT);
     } else {
         const int d = x - (ncell_blocks + npath_blocks) * (int)blockDim.x;
         if (d < n.ndam_cells) {
             const int i = __ldg(&n.dam_cells[d]);
-            cell_dam(n, s, OwnG(n, s, __ldg(&n.cflag[i])), m, i, DT, c.nt, c.dt_def, k);
+            cell_dam(n, s, own_cell(n, s, m, i), m, i, DT, c.nt, c.dt_def, k);
         }
     }
 }
@@ -1004,7 +1131,8 @@ __global__ void __launch_bounds__(kCellThreads, MinBlocks) k_flux(Net n, State s
 template <class Own>
 __device__ __forceinline__ void cell_rate(const Net &n, const State &s, const Own &w, int m, int i, double DT) {
     const size_t base = (size_t)m * n.N, gi = base + i;
-    const double rout = w.rivout_raw(gi), fout = w.fldout_raw(gi);
+    const double2 raw = w.own_raw(gi);
+    const double rout = raw.x, fout = raw.y;
     double so = dmax(rout, 0.0) + dmax(fout, 0.0);
     w.each_raw(base, i, [&](double rj, double fj) { so = (so + dmax(-rj, 0.0)) + dmax(-fj, 0.0); });
     so = so * DT;
@@ -1024,7 +1152,7 @@ __device__ __forceinline__ void cell_rate(const Net &n, const State &s, const Ow
 
 // advance != 0: block (0,0) also moves the loop counter to the next sub-step and sets the WHILE
 // condition (every k_flux block has read the counter; k_rate and k_store read `kcur`)
-__global__ void k_rate(Net n, State s, int advance, cudaGraphConditionalHandle h, int use_cond) {
+__global__ void __launch_bounds__(kCellThreads, 6) k_rate(Net n, State s, int advance, cudaGraphConditionalHandle h, int use_cond) {
     const int m = blockIdx.y;
     const MemberCtl &c = s.ctl[m];
     const int k = s.loop->kcur;
@@ -1036,7 +1164,7 @@ __global__ void k_rate(Net n, State s, int advance, cudaGraphConditionalHandle h
     }
     if (k >= c.nt) return;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n.N) cell_rate(n, s, OwnG(n, s, __ldg(&n.cflag[i])), m, i, c.dt);
+    if (i < n.N) cell_rate(n, s, own_cell(n, s, m, i), m, i, c.dt);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -1088,7 +1216,7 @@ __device__ __forceinline__ void path_rescale(const Net &n, const State &s, int m
 
 // one cell in phase C; `bput(k, v)` receives the last sub-step's budget term k
 template <class Own, class BPut>
-__device__ __forceinline__ void cell_store(const Net &n, const State &s, const Own &w, int m, int i, double DT,
+__device__ __forceinline__ void cell_store(const Net &n, const State &s, Own &w, int m, int i, double DT,
                                            bool first, bool last, double nadd, int nt, double dt_def, BPut bput) {
     const size_t base = (size_t)m * n.N;
     const size_t gi = base + i;
@@ -1096,7 +1224,8 @@ __device__ __forceinline__ void cell_store(const Net &n, const State &s, const O
     // the cell's own state is read up front, before anything is stored: in the compiler's view a
     // store may alias any later load of another state array and would hold that load back
     const auto rate_i = w.rate(gi);
-    double rout = w.rivout_raw(gi), fout = w.fldout_raw(gi);
+    const double2 own = w.own_out(gi);
+    double rout = own.x, fout = own.y;
     const double runoff = w.runoff(gi);
     const double rivsto0 = w.rivsto(gi), fldsto0 = w.fldsto(gi), rivdph0 = w.rivdph(gi);
     const double frc = w.fldfrc(gi);
@@ -1105,14 +1234,11 @@ __device__ __forceinline__ void cell_store(const Net &n, const State &s, const O
     // where they are used they cost a round of loads of their own
     StageMap map;
     if constexpr (Own::kResident) map = stage_map(w, i);
-    // own outflow after the LSPAMAT rescale (:456-473)
+    // own outflow after the LSPAMAT rescale (:456-473); phase B has done a positive one and a mouth's
     if (i < n.R && !(rout > 0.0)) {
         const double r = w.nb(rate_m, w.next(i));
         rout = rout * r;
         fout = fout * r;
-    } else if constexpr (!Own::kResident) {      // phase B of the resident kernel has done it
-        rout = rout * rate_i;
-        fout = fout * rate_i;
     }
     // inflow from the upstream cells
     double rinf = 0.0, finf = 0.0;
@@ -1167,12 +1293,12 @@ __device__ __forceinline__ void cell_store(const Net &n, const State &s, const O
     if constexpr (!Own::kResident) map = stage_map(w, i);
     const StageOut o = stage(n, w, i, map, rs, fs, levsto);
     // CALC_VARS_PRE, src/cmf_ctrl_physics_mod.F90:254-277, and the dam storage
-    w.put_pre(gi, rout, fout, rivdph0, fldsto0);
+    w.put_pre(gi, rout, fout, rivdph0, fldsto0, last);
     if (dam) s.damsto[gi] = damsto1;
     // CMF_CheckNanB-style probe (src/cmf_utils_mod.F90:807-815) on the new storage: a NaN or
     // infinite runoff or state surfaces as a positive status instead of a silent NaN state
     if (!isfinite((o.rivsto + o.fldsto) + o.levsto)) s.ctl[m].err = kErrNonFinite;
-    store_stage(n, s, w, gi, i, o, last);
+    store_stage(n, s, w, gi, i, o, rivdph0, last);
     bput(5, n.llevee ? (rs + fs) + levsto : rs + fs);
     bput(6, n.llevee ? (o.rivsto + o.fldsto) + o.levsto : o.rivsto + o.fldsto);
     bput(7, o.rivsto);
@@ -1239,6 +1365,15 @@ __device__ __forceinline__ void cell_store(const Net &n, const State &s, const O
     }
 }
 
+template <class BPut>
+__device__ __forceinline__ void store_cell(const Net &n, const State &s, int m, int i, double DT, bool first, bool last,
+                                           double nadd, int nt, double dt_def, BPut bput) {
+    OwnG w = own_cell(n, s, m, i);
+    const unsigned before = w.wet;
+    cell_store(n, s, w, m, i, DT, first, last, nadd, nt, dt_def, bput);
+    put_wet(n, s, m, i, before, w.wet);
+}
+
 // Budget partials of the last sub-step (the only one the caller observes), one per warp of 32
 // consecutive cells: a fixed butterfly over the warp, so the partials -- and the budgets k_budget
 // sums from them in a fixed order -- are the same whatever block size or schedule ran the cells.
@@ -1281,7 +1416,7 @@ __global__ void __launch_bounds__(kCellThreads, MinBlocks) k_store(Net n, State 
     if (last && i >= n.N)
 #pragma unroll
         for (int k = 0; k < kBudgets; k++) bt[k * bstride] = 0.0;
-    if (i < n.N) cell_store(n, s, OwnG(n, s, __ldg(&n.cflag[i])), m, i, DT, first, last, nadd, c.nt, c.dt_def, bput);
+    if (i < n.N) store_cell(n, s, m, i, DT, first, last, nadd, c.nt, c.dt_def, bput);
     if (last) {
         double b[kBudgets];
 #pragma unroll

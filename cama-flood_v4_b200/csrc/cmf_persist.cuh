@@ -182,7 +182,8 @@ __global__ void __launch_bounds__(kTile, kPersistMinBlocks) k_persist(Net n, Sta
             const size_t gi = (size_t)tg.m * N + i;
             const OwnG w(n, s, __ldg(&n.cflag[i]));
             const StageOut o = stage(n, w, i, stage_map(w, i), s.rivsto[gi], s.fldsto[gi], n.llevee ? s.levsto[gi] : 0.0);
-            store_stage(n, s, w, gi, i, o);
+            put_full_stage(n, s, gi, i, o);
+            begin_cell(n, s, gi, o.rivdph, o.fldsto, o.flddph, o.fldfrc, o.levsto, o.levdph);
             if (n.ladpstp && __ldg(&n.i2mask[i]) == 0) key = cfl_key(n.pcadp, (i < n.R) ? __ldg(&n.nxtdst[i]) : n.pdstmth, n.pgrv, o.rivdph);
         }
         if (n.ladpstp) {
@@ -213,9 +214,8 @@ __global__ void __launch_bounds__(kTile, kPersistMinBlocks) k_persist(Net n, Sta
                 const MemberCtl &c = s.ctl[tg.m];
                 const int i = tg.i0 + threadIdx.x;
                 if (k < c.nt && i < tg.i1) {
-                    const OwnG w(n, s, __ldg(&n.cflag[i]));
-                    cell_outflow(n, s, w, tg.m, i, c.dt, c.nt, c.dt_def, k, split && k == 0);
-                    if (w.flags() & C_DAM) cell_dam(n, s, w, tg.m, i, c.dt, c.nt, c.dt_def, k);
+                    flux_cell(n, s, tg.m, i, c.dt, c.nt, c.dt_def, k, split && k == 0);
+                    if (__ldg(&n.cflag[i]) & C_DAM) cell_dam(n, s, own_cell(n, s, tg.m, i), tg.m, i, c.dt, c.nt, c.dt_def, k);
                 }
             } else {
                 const int q = t - T, m = q / ppm;
@@ -227,7 +227,7 @@ __global__ void __launch_bounds__(kTile, kPersistMinBlocks) k_persist(Net n, Sta
         for (int t = b; t < T; t += G) {
             const TileGeom tg = tile_geom(t, tpm, N);
             const int i = tg.i0 + threadIdx.x;
-            if (k < s.ctl[tg.m].nt && i < tg.i1) cell_rate(n, s, OwnG(n, s, __ldg(&n.cflag[i])), tg.m, i, s.ctl[tg.m].dt);
+            if (k < s.ctl[tg.m].nt && i < tg.i1) cell_rate(n, s, own_cell(n, s, tg.m, i), tg.m, i, s.ctl[tg.m].dt);
         }
         if (!gb.sync()) return;
         // ---- phase C: rescale, inflow, STONXT, stage scheme, diagnostics; path rescale
@@ -246,7 +246,7 @@ __global__ void __launch_bounds__(kTile, kPersistMinBlocks) k_persist(Net n, Sta
                 if (last && i >= tg.i1)
 #pragma unroll
                     for (int q = 0; q < kBudgets; q++) bt[q * kTile] = 0.0;
-                if (i < tg.i1) cell_store(n, s, OwnG(n, s, __ldg(&n.cflag[i])), tg.m, i, DT, first, last, nadd, c.nt, c.dt_def, bput);
+                if (i < tg.i1) store_cell(n, s, tg.m, i, DT, first, last, nadd, c.nt, c.dt_def, bput);
                 if (last) {
                     double bl[kBudgets];
 #pragma unroll

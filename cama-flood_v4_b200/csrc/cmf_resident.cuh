@@ -101,23 +101,14 @@ struct OwnR : OwnMaps {
     __device__ __forceinline__ double fldsto_pre(size_t g) const { return sparse(B_FLDSTOPRE, s.fldsto_pre, g); }
     __device__ __forceinline__ double flddph(size_t g) const { return sparse(B_FLDDPH, s.flddph, g); }
     __device__ __forceinline__ double fldfrc(size_t g) const { return sparse(B_FLDFRC, s.fldfrc, g); }
-    __device__ __forceinline__ double storge(size_t g) const {
-        const double t = rivsto(g) + fldsto(g);
-        return n.llevee ? t + levsto(g) : t;
-    }
     __device__ __forceinline__ double runoff(size_t g) const { return s.runoff[g]; }
     // (F_ROUT, F_FOUT): the last sub-step's outflow until phase A, then before the rescale, and from
     // phase B on after it unless the flow is reverse.  A dam cell's outflow comes from a task of its own
     // in phase A, while the task of its diagnostics still reads the pair of the last sub-step, so it waits
     // in the phase kernels' arrays for phase B
-    __device__ __forceinline__ double rivout_raw(size_t g) const { return waiting ? s.rivout_raw[g] : get(F_ROUT); }
-    __device__ __forceinline__ double fldout_raw(size_t g) const { return waiting ? s.fldout_raw[g] : get(F_FOUT); }
-    // the cell's rate, read where a reverse flow or a path needs it
-    struct Rate {
-        const double *p;
-        __device__ __forceinline__ operator double() const { return __ldcg(p); }
-    };
-    __device__ __forceinline__ Rate rate(size_t g) const { return {s.rate + g}; }
+    __device__ __forceinline__ double2 own_raw(size_t g) const { return waiting ? s.raw[g] : own_out(g); }
+    __device__ __forceinline__ double2 own_out(size_t) const { return make_double2(get(F_ROUT), get(F_FOUT)); }
+    __device__ __forceinline__ LazyRate rate(size_t g) const { return {s.rate + g, true}; }
     __device__ __forceinline__ double a_rivvel(size_t) const { return get(F_ARIVVEL); }
     __device__ __forceinline__ double a_rivout(size_t) const { return get(F_ARIVOUT); }
     __device__ __forceinline__ double a_fldout(size_t g) const { return sparse(B_AFLDOUT, s.a_fldout, g); }
@@ -129,16 +120,15 @@ struct OwnR : OwnMaps {
     __device__ __forceinline__ double m_storge(size_t) const { return get(F_MSTORGE); }
     // values of other CTAs' cells: past L1, which may hold an older sub-step's line
     __device__ __forceinline__ double nb(const double *p, size_t g) const { return __ldcg(p + g); }
-    __device__ __forceinline__ DownCell down(size_t base, int j) const {
+    __device__ __forceinline__ DownCell down(size_t base, int i, int j) const {
         const double d = __ldcg(s.rivdph + base + j);
         const double pre = first_step ? __ldcg(s.rivdph_pre + base + j) : get(F_DWNPRE);
         put(F_DWNPRE, d);
-        return {__ldg(&n.rivelv[j]), d, pre};
+        return {__ldg(&n.next_rivelv[i]), d, pre};
     }
     __device__ __forceinline__ void put_raw(size_t g, int, double rout, double fout) const {
-        if (bits & C_DAM) {      // see rivout_raw
-            s.rivout_raw[g] = rout;
-            s.fldout_raw[g] = fout;
+        if (bits & C_DAM) {      // see own_raw
+            s.raw[g] = make_double2(rout, fout);
         } else {
             put(F_ROUT, rout);
             put(F_FOUT, fout);
@@ -158,7 +148,7 @@ struct OwnR : OwnMaps {
         if (x >= 0) out[x] = make_double2(rout, fout);
     }
     __device__ __forceinline__ void put_a_rivvel(size_t, double v) const { put(F_ARIVVEL, v); }
-    __device__ __forceinline__ void put_pre(size_t g, double rout, double fout, double dph, double fld) const {
+    __device__ __forceinline__ void put_pre(size_t g, double rout, double fout, double dph, double fld, bool) const {
         put(F_ROUT, rout);
         put(F_FOUT, fout);
         put(F_DPHPRE, dph);
@@ -170,7 +160,7 @@ struct OwnR : OwnMaps {
         if (bits & C_PATH) s.rivdph_pre[g] = dph;
     }
     template <class Out>
-    __device__ __forceinline__ void put_stage(size_t g, const Out &o, double sto) const {
+    __device__ __forceinline__ void put_stage(size_t g, const Out &o, double sto, double, bool) const {
         put(F_RIVSTO, o.rivsto);
         put(F_RIVDPH, o.rivdph);
         s.rivdph[g] = o.rivdph;
@@ -202,18 +192,11 @@ struct OwnR : OwnMaps {
     }
     template <class F>
     __device__ __forceinline__ void each_raw(size_t, int, F fn) const { each_pair(raw, fn); }
-    template <class F>
+    template <class Rate, class F>
     __device__ __forceinline__ void each_out(size_t, int, Rate rate_i, F fn) const {
-        each_pair(out, [&](double rj, double fj) {
-            if (!(rj > 0.0) && !(rj == 0.0 && fj == 0.0)) {      // zeros stay zeros
-                const double r = rate_i;
-                rj = rj * r;
-                fj = fj * r;
-            }
-            fn(rj, fj);
-        });
+        each_pair(out, [&](double rj, double fj) { rescaled(make_double2(rj, fj), rate_i, fn); });
     }
-    // the previous sub-step's averages and maxima (diag_carry_store with the sums held on the SM)
+    // the previous sub-step's averages and maxima (diag_carry with the sums held on the SM)
     __device__ __forceinline__ void carry(size_t g, double DT, bool first, double rout, double fout, double dph, double sto) const {
         const double outflw = rout + fout;
         const double pro = first ? 0.0 : get(F_ARIVOUT);
@@ -293,9 +276,9 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident(Net n, State s, Res
                 const int u0 = __ldg(&n.up_ptr[i]);
                 s_int[I_UP * stride + slot] = u0 | (__ldg(&n.up_ptr[i + 1]) - u0) << kResDegShift;
                 bits = __ldg(&n.cflag[i]) | (unsigned)ml << kResMemberShift;
-                const OwnR w(n, s, fields + slot, stride, s_int + slot, bits, a, ml, true);
+                OwnR w(n, s, fields + slot, stride, s_int + slot, bits, a, ml, true);
                 const StageOut o = stage(n, w, i, stage_map(w, i), s.rivsto[gi], s.fldsto[gi], n.llevee ? s.levsto[gi] : 0.0);
-                store_stage(n, s, w, gi, i, o);
+                store_stage(n, s, w, gi, i, o, 0.0, true);
                 w.put(F_ROUT, s.rivout_pre[gi]);
                 w.put(F_FOUT, s.fldout_pre[gi]);
                 w.put(F_DPHPRE, s.rivdph_pre[gi]);
@@ -346,7 +329,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident(Net n, State s, Res
                     const int ml = bits >> kResMemberShift;
                     if (bits >= kNoCell || !(bits & C_DAM) || k >= s_nt[ml]) continue;
                     const int i = s_cell[slot], m = m0 + ml;
-                    const OwnR w(n, s, fields + slot, stride, s_int + slot, bits, a, ml, k == 0);
+                    OwnR w(n, s, fields + slot, stride, s_int + slot, bits, a, ml, k == 0);
                     cell_dam(n, s, w, m, i, s_dt[ml], s_nt[ml], s.ctl[m].dt_def, k);
                 } else if (q < nd + npath) {
                     const int t = (q - nd) * (int)G + (int)b, ml = t / ptpm;
@@ -358,7 +341,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident(Net n, State s, Res
                     const int ml = bits >> kResMemberShift;
                     if (bits >= kNoCell || k >= s_nt[ml]) continue;
                     const int i = s_cell[slot], m = m0 + ml;
-                    const OwnR w(n, s, fields + slot, stride, s_int + slot, bits, a, ml, k == 0);
+                    OwnR w(n, s, fields + slot, stride, s_int + slot, bits, a, ml, k == 0);
                     cell_outflow(n, s, w, m, i, s_dt[ml], s_nt[ml], s.ctl[m].dt_def, k, split && k == 0);
                     s_bits[slot] = bits;
                 }
@@ -372,7 +355,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident(Net n, State s, Res
                 const int ml = bits >> kResMemberShift;
                 if (bits >= kNoCell || k >= s_nt[ml]) continue;
                 const int i = s_cell[slot];
-                const OwnR w(n, s, fields + slot, stride, s_int + slot, bits, a, ml, k == 0, true);
+                OwnR w(n, s, fields + slot, stride, s_int + slot, bits, a, ml, k == 0, true);
                 cell_rate(n, s, w, m0 + ml, i, s_dt[ml]);
             }
             if (!gb.sync()) return;
@@ -392,7 +375,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident(Net n, State s, Res
                     // sequence's order, whatever order the tiles have
                     double *term = a.terms + (size_t)ml * tpm * 32 + i;
                     auto bput = [&](int j, double v) { if (last) term[j * nterm] = v; };
-                    const OwnR w(n, s, fields + slot, stride, s_int + slot, bits, a, ml, k == 0);
+                    OwnR w(n, s, fields + slot, stride, s_int + slot, bits, a, ml, k == 0);
                     cell_store(n, s, w, m, i, DT, k == 0, last, nadd, nt, s.ctl[m].dt_def, bput);
                     s_bits[slot] = bits;
                 } else {
@@ -414,12 +397,13 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident(Net n, State s, Res
             unsigned bits = s_bits[slot];
             if (bits >= kNoCell) continue;
             const size_t gi = (size_t)(m0 + (bits >> kResMemberShift)) * N + s_cell[slot];
-            const OwnR w(n, s, fields + slot, stride, s_int + slot, bits, a, 0, false);
+            OwnR w(n, s, fields + slot, stride, s_int + slot, bits, a, 0, false);
             s.rivsto[gi] = w.get(F_RIVSTO);
             s.rivout_pre[gi] = w.get(F_ROUT);
             s.fldout_pre[gi] = w.get(F_FOUT);
             s.rivdph_pre[gi] = w.get(F_DPHPRE);
-            s.storge[gi] = w.storge(gi);
+            const double riv_fld = w.rivsto(gi) + w.fldsto(gi);
+            s.storge[gi] = n.llevee ? riv_fld + w.levsto(gi) : riv_fld;
             if (!(bits & B_FLDSTO)) s.fldsto[gi] = 0.0;
             if (!(bits & B_FLDSTOPRE)) s.fldsto_pre[gi] = 0.0;
             if (!(bits & B_FLDDPH)) s.flddph[gi] = 0.0;
