@@ -527,39 +527,43 @@ __global__ void k_emu_update(EmuNet n, const int *active, double dt, const doubl
 // ------------------------------------------------------------------------------------------
 // Fused inference on the 5th-generation tensor cores (tcgen05, sm_100a).
 //
-// One CTA per SM (a persistent grid) holds all four layers' weights in shared memory once, as
-// the MMAs' B operands, and runs four 128-row tiles at a time: warpgroup s (warps 4s..4s+3) owns
-// tile slot s -- its activation buffer (the next MMA's A operand) and 128 of the SM's 512
-// tensor-memory columns -- and a seventeenth warp issues the MMAs.  Both operands use the K-major
-// no-swizzle canonical layout: 16-byte rows of 8 bf16 grouped in 8-row core matrices, byte offset
-// (k/8)*(R*16) + (r/8)*128 + (r%8)*16 for an R-row operand.  Per layer of a slot: the warpgroup
-// writes the A operand, arrives on the slot's `ready` mbarrier; the MMA warp, polling all four
-// slots, issues that layer's tcgen05.mma chain (M=128, N=128 or 16, K=16 per instruction, fp32
-// accumulator in the slot's columns) and commits it to the slot's `done` mbarrier; the warpgroup
-// waits on it, reads its rows with tcgen05.ld (warp 4s+q owns TMEM lanes 32q..32q+31), adds the
-// bias, applies ReLU and the bf16 rounding in one cvt and writes the next A operand.  While one
-// slot runs its epilogue the tensor pipe serves the others.  The last layer (N=16, column 0 real)
-// adds b3 and writes y.  Every wait is bounded: a wait that runs out raises the CTA's abort flag,
-// every warpgroup leaves at its next vote, and the MMA warp drains the MMAs it issued (one more
-// commit, waited for with the full bound) before the tensor memory is released.  The rounding
-// points equal the layer-by-layer chain (bf16 inputs, fp32 accumulation, bf16 activations) and the
-// K=16 steps run in the same order, so the outputs equal that chain bit for bit.
+// One CTA per SM (a persistent grid) holds all four layers' weights in shared memory once, as the MMAs'
+// B operands, and runs two 128-row tiles at a time.  A tile's activations never touch shared memory:
+// slot s (warps 16s..16s+15) owns 192 of the SM's tensor-memory columns, 128 for the fp32 accumulator and 64
+// for the next layer's A operand (row = lane, two bf16 of consecutive k per column), which tcgen05.mma
+// reads from there.  With both operands in shared memory one 128x128x16 product reads 8 KB in the 64
+// cycles it takes, all of the SM's shared-memory bandwidth, next to the epilogue's stores; so it reads
+// 4 KB.  B is 128-byte swizzled (sw128_off).  Per layer of a slot: its warps (warp
+// 16s+4g+q: TMEM lanes 32q..32q+31, columns 32g..32g+31) wait for the layer's products, read the
+// accumulator with tcgen05.ld, add the bias, apply ReLU and the bf16 rounding in one cvt and write the
+// next A columns; after the slot's one barrier its first warp issues the next layer's tcgen05.mma chain
+// (one elected thread; M=128, N=128 or 16, K=16 per instruction) and commits it to the slot's mbarrier.  While one slot runs
+// its epilogue the tensor pipe serves the other; sixteen warps keep the epilogue to 32 columns per thread,
+// as a layer's time is the chain wait, load, convert, store, barrier, issue, product.  The last layer
+// (N=16, column 0 real) adds b3 and writes y, and the next tile's X goes in.  Tiles are dealt to the CTAs
+// first and to their slots second, so that a small call spreads over the SMs.  Every wait is bounded: a
+// wait that runs out ends the slot's loop at its next barrier (a vote), and its first warp drains the
+// MMAs it issued (one more commit, waited for with the full bound) before the tensor memory is released.
+// The rounding points equal the layer-by-layer chain (bf16 inputs, fp32 accumulation, bf16 activations) and
+// the K=16 steps run in the same order, so the outputs equal that chain bit for bit.
+// 4.2M rows: 511 us with four 128-thread slots, activations in shared memory and a polling issuer warp;
+// 582 us in this form with the MMAs issued under a branch on the thread index; 401 us as it stands, where the
+// products alone would take 202 us at the measured bf16 rate.  26.6k rows: 16.4 and 10.4 us.
 // ------------------------------------------------------------------------------------------
 constexpr int kTcRows = 128;
-constexpr int kTcSlots = 4;                           // tiles in flight per CTA
-constexpr int kTcEpi = 128 * kTcSlots;                // epilogue threads (4 warpgroups)
-constexpr int kTcThreads = kTcEpi + 32;               // + the MMA warp
+constexpr int kTcSlots = 2;                           // tiles in flight per CTA
+constexpr int kTcSlotThreads = 512;
+constexpr int kTcThreads = kTcSlotThreads * kTcSlots;
 constexpr int kTcW0 = 0;                              // byte offsets inside the packed image
-constexpr int kTcW1 = kTcW0 + 128 * 32 * 2;           // layer 0: N=128, K=32
+constexpr int kTcW1 = kTcW0 + 128 * 64 * 2;           // layer 0: N=128, K=32 (of a 64-column block)
 constexpr int kTcW2 = kTcW1 + 128 * 128 * 2;          // layers 1, 2: N=128, K=128
 constexpr int kTcW3 = kTcW2 + 128 * 128 * 2;          // layer 3: N=16, K=128
 constexpr int kTcWBytes = kTcW3 + 16 * 128 * 2;
-constexpr int kTcABytes = kTcRows * 128 * 2;          // one slot's activations: 128 rows x 128 k
-constexpr int kTcA = kTcWBytes;
-constexpr int kTcBias = kTcA + kTcSlots * kTcABytes;  // b0 b1 b2 (3 x 128 floats), b3[0]
-constexpr int kTcMisc = kTcBias + (3 * 128 + 4) * 4;  // ready[4], done[4], drain mbarriers; TMEM address; abort
-constexpr int kTcSmem = kTcMisc + (2 * kTcSlots + 1) * 8 + 16;
-constexpr int kTcCols = 128 * kTcSlots;               // tensor-memory columns of the CTA
+constexpr int kTcBias = kTcWBytes;                    // b0 b1 b2 (3 x 128 floats), b3[0]
+constexpr int kTcMisc = kTcBias + (3 * 128 + 4) * 4;  // done[2], drain[2] mbarriers; TMEM address
+constexpr int kTcSmem = kTcMisc + 2 * kTcSlots * 8 + 16;
+constexpr int kTcSlotCols = 192, kTcACol = 128;       // a slot's tensor-memory columns, the A operand's place
+constexpr int kTcCols = 512;                          // allocated (a power of two)
 #ifndef CMF_TC_WAIT_LIMIT
 #define CMF_TC_WAIT_LIMIT (1 << 20)
 #endif
@@ -574,6 +578,18 @@ __host__ __device__ constexpr uint64_t umma_smem_desc(uint32_t saddr, uint32_t l
     return (uint64_t)((saddr >> 4) & 0x3FFFu) | ((uint64_t)((lbo >> 4) & 0x3FFFu) << 16) |
            ((uint64_t)((sbo >> 4) & 0x3FFFu) << 32) | (1ull << 46);
 }
+// The layout of the inference image: 128-byte swizzled, a matrix of R rows cut into
+// blocks of 64 bf16 columns, block-major, a row's 128 bytes together, its 16-byte chunk c at c ^ (row % 8).
+__host__ __device__ constexpr uint32_t sw128_off(int r, int c, int R) {
+    return (uint32_t)((c >> 6) * (R * 128) + r * 128 + ((((c >> 3) & 7) ^ (r & 7)) << 4) + (c & 7) * 2);
+}
+__host__ __device__ constexpr uint64_t sw128_desc(uint32_t saddr, uint32_t lbo, uint32_t sbo) {
+    return umma_smem_desc(saddr, lbo, sbo) | (2ull << 61);
+}
+// K=16 step s of a matrix at `base` (1024-byte aligned)
+__device__ __forceinline__ uint64_t sw128_kmajor(uint32_t base, int R, int s) {
+    return sw128_desc(base + (s >> 2) * (R * 128) + (s & 3) * 32, 16, 1024);
+}
 __host__ __device__ constexpr uint32_t umma_idesc_bf16_f32(int M, int N) {
     // D fp32, A and B bf16, both K-major, N/8 and M/16
     return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
@@ -584,21 +600,22 @@ __host__ __device__ constexpr uint32_t canon_off(int r, int k, int R) {
     return (uint32_t)((k >> 3) * (R * 16) + (r >> 3) * 128 + (r & 7) * 16 + (k & 7) * 2);
 }
 
-// B operands of the four layers as one shared-memory image: element (n, k) = W[k][n]
+// B operands of the four layers as one shared-memory image: element (n, k) = W[k][n], columns 32.. of
+// layer 0 zero
 __global__ void k_mlp_tc_pack(const __nv_bfloat16 *__restrict__ W0, const __nv_bfloat16 *__restrict__ W1,
                               const __nv_bfloat16 *__restrict__ W2, const __nv_bfloat16 *__restrict__ W3, int ldw3,
                               __nv_bfloat16 *out) {
     const int e = blockIdx.x * blockDim.x + threadIdx.x;
-    const int n0 = 128 * 32, n1 = 128 * 128, n3 = 16 * 128;
+    const int n0 = 128 * 64, n1 = 128 * 128, n3 = 16 * 128;
     if (e >= n0 + 2 * n1 + n3) return;
     int n, k, R, base;
     const __nv_bfloat16 *W;
     int ldw;
-    if (e < n0) { n = e / 32; k = e % 32; R = 128; base = kTcW0; W = W0; ldw = 128; }
+    if (e < n0) { n = e / 64; k = e % 64; R = 128; base = kTcW0; W = W0; ldw = 128; }
     else if (e < n0 + n1) { const int q = e - n0; n = q / 128; k = q % 128; R = 128; base = kTcW1; W = W1; ldw = 128; }
     else if (e < n0 + 2 * n1) { const int q = e - n0 - n1; n = q / 128; k = q % 128; R = 128; base = kTcW2; W = W2; ldw = 128; }
     else { const int q = e - n0 - 2 * n1; n = q / 128; k = q % 128; R = 16; base = kTcW3; W = W3; ldw = ldw3; }
-    out[(base + canon_off(n, k, R)) / 2] = W[(size_t)k * ldw + n];
+    out[(base + sw128_off(n, k, R)) / 2] = (e < n0 && k >= 32) ? __float2bfloat16_rn(0.f) : W[(size_t)k * ldw + n];
 }
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -609,6 +626,24 @@ __device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t adesc, uint6
         "setp.ne.b32 p, %4, 0;\n\t"
         "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n"
         :: "r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(acc));
+}
+
+// one thread of a converged warp, chosen by the hardware: the form in which ptxas keeps the operands of
+// tcgen05 instructions in uniform registers (under a branch on the thread index each MMA took about 200
+// cycles to issue)
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred e;\n\telect.sync _|e, 0xffffffff;\n\tselp.u32 %0, 1, 0, e;\n\t}\n" : "=r"(p));
+    return p != 0;
+}
+
+// the same with A in tensor memory (K-major: lane = row, two consecutive k per 32-bit column)
+__device__ __forceinline__ void umma_bf16_ta(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t acc) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}\n"
+        :: "r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(acc));
 }
 
 __device__ __forceinline__ void umma_commit(uint32_t mbar) {
@@ -642,6 +677,18 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&v)[32]) {
 __device__ __forceinline__ void tmem_ld1(uint32_t taddr, uint32_t &v) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];" : "=r"(v) : "r"(taddr));
 }
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&v)[16]) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
+        :: "r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]),
+           "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15])
+        : "memory");
+}
+__device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint4 &a, const uint4 &b) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};"
+                 :: "r"(taddr), "r"(a.x), "r"(a.y), "r"(a.z), "r"(a.w), "r"(b.x), "r"(b.y), "r"(b.z), "r"(b.w) : "memory");
+}
+__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
@@ -655,35 +702,18 @@ __device__ __forceinline__ uint32_t relu_bf16x2(float lo, float hi) {
     return d;
 }
 
-// layer epilogue: bias + ReLU + bf16 of the 128 accumulator columns of row r into the next
-// layer's A operand (two 32-column loads in flight)
-__device__ __forceinline__ void tc_epilogue_hidden(uint32_t tmem_row, const float *bias, unsigned char *sA, int r) {
+// layer epilogue of 32 columns of one row: bias + ReLU + bf16 into 16 columns of the next A operand
+__device__ __forceinline__ void tc_epilogue_hidden(uint32_t tmem_d, const float *bias, uint32_t tmem_a) {
+    uint32_t v[32], w[16];
+    tmem_ld32(tmem_d, v);
+    tmem_wait_ld();
 #pragma unroll
-    for (int h = 0; h < 4; h += 2) {
-        uint32_t v[2][32];
-        tmem_ld32(tmem_row + 32 * h, v[0]);
-        tmem_ld32(tmem_row + 32 * (h + 1), v[1]);
-        tmem_wait_ld();
-#pragma unroll
-        for (int g = 0; g < 2; g++) {
-#pragma unroll
-            for (int q = 0; q < 4; q++) {
-                const int c = 32 * (h + g) + 8 * q;       // first of 8 columns = k chunk c/8 of the next layer
-                uint4 u;
-                uint32_t *w = reinterpret_cast<uint32_t *>(&u);
-#pragma unroll
-                for (int j = 0; j < 4; j++)
-                    w[j] = relu_bf16x2(__uint_as_float(v[g][8 * q + 2 * j]) + bias[c + 2 * j],
-                                       __uint_as_float(v[g][8 * q + 2 * j + 1]) + bias[c + 2 * j + 1]);
-                *reinterpret_cast<uint4 *>(sA + canon_off(r, c, kTcRows)) = u;
-            }
-        }
-    }
+    for (int j = 0; j < 16; j++)
+        w[j] = relu_bf16x2(__uint_as_float(v[2 * j]) + bias[2 * j], __uint_as_float(v[2 * j + 1]) + bias[2 * j + 1]);
+    tmem_st16(tmem_a, w);
+    tmem_wait_st();
 }
 
-__device__ __forceinline__ void named_bar(int id, int nthreads) {
-    asm volatile("bar.sync %0, %1;" :: "r"(id), "r"(nthreads) : "memory");
-}
 // named barrier with an OR over the participants' flags: every participant gets the same answer
 __device__ __forceinline__ bool named_bar_or(int id, int nthreads, bool v) {
     uint32_t r;
@@ -695,19 +725,6 @@ __device__ __forceinline__ bool named_bar_or(int id, int nthreads, bool v) {
         : "=r"(r) : "r"((uint32_t)v), "r"(id), "r"(nthreads) : "memory");
     return r != 0;
 }
-__device__ __forceinline__ void mbar_arrive(uint32_t mbar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" :: "r"(mbar) : "memory");
-}
-__device__ __forceinline__ bool mbar_try(uint32_t mbar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}\n"
-        : "=r"(ok) : "r"(mbar), "r"(parity) : "memory");
-    return ok != 0;
-}
-
 __global__ void __launch_bounds__(kTcThreads, 1) k_mlp_tc(const __nv_bfloat16 *__restrict__ X, int ldx, int rows,
                                                         const uint4 *__restrict__ wimg, const float *__restrict__ b0,
                                                         const float *__restrict__ b1, const float *__restrict__ b2,
@@ -715,20 +732,16 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_mlp_tc(const __nv_bfloat16 *_
                                                         int wait_limit) {
     extern __shared__ __align__(1024) unsigned char sm[];
     float *sb = reinterpret_cast<float *>(sm + kTcBias);
-    uint64_t *ready = reinterpret_cast<uint64_t *>(sm + kTcMisc);
-    uint64_t *done = ready + kTcSlots;
-    uint64_t *drain = done + kTcSlots;
-    uint32_t *tslot = reinterpret_cast<uint32_t *>(drain + 1);
-    volatile int *abort_flag = reinterpret_cast<volatile int *>(tslot + 1);
+    uint64_t *done = reinterpret_cast<uint64_t *>(sm + kTcMisc), *drain = done + kTcSlots;
+    uint32_t *tslot = reinterpret_cast<uint32_t *>(drain + kTcSlots);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     // weights and biases into shared memory
     for (int e = tid; e < kTcWBytes / 16; e += kTcThreads) reinterpret_cast<uint4 *>(sm)[e] = wimg[e];
     for (int e = tid; e < 128; e += kTcThreads) { sb[e] = b0[e]; sb[128 + e] = b1[e]; sb[256 + e] = b2[e]; }
     if (tid == 0) {
         sb[384] = b3[0];
-        for (int q = 0; q < 2 * kTcSlots + 1; q++)
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(smem_u32(ready + q)) : "memory");
-        *abort_flag = 0;
+        for (int q = 0; q < 2 * kTcSlots; q++)
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(smem_u32(done + q)) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 0) {   // one warp allocates the CTA's accumulator columns and releases the allocation permit
@@ -740,133 +753,87 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_mlp_tc(const __nv_bfloat16 *_
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = *tslot;
+    const uint32_t tmem = __shfl_sync(0xffffffffu, *tslot, 0);
     const int ntiles = (rows + kTcRows - 1) / kTcRows;
     const int stride = kTcSlots * (int)gridDim.x;             // tiles of slot s: first + j * stride
-    if (warp < kTcSlots * 4) {
-        // ---- epilogue warpgroup of slot s
-        const int sl = warp >> 2, q = warp & 3;
-        const int r = 32 * q + lane;                          // this thread's row == TMEM lane
-        unsigned char *sA = sm + kTcA + sl * kTcABytes;
-        const uint32_t trow = tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(128 * sl);
-        const uint32_t rd = smem_u32(ready + sl), dn = smem_u32(done + sl);
-        const int bar = 1 + sl;                               // named barrier of the warpgroup
-        uint32_t dphase = 0;
-        bool go = true;
-        int t = blockIdx.x * kTcSlots + sl;
-        uint4 xn[4];                                          // this row's X (32 bf16) of tile t
+    const int sl = __shfl_sync(0xffffffffu, warp >> 4, 0), g = (warp >> 2) & 3, q = warp & 3;
+    const int r = 32 * q + lane;                              // this thread's row == TMEM lane
+    const uint32_t td = tmem + (uint32_t)(kTcSlotCols * sl), trow = td + ((uint32_t)(32 * q) << 16);
+    const uint32_t dn = smem_u32(done + sl), sw = smem_u32(sm);
+    const bool lead = __shfl_sync(0xffffffffu, (warp & 15) == 0, 0);      // the slot's first warp
+    // issues layer L of the slot's tile (one thread of the lead warp): A from the slot's columns, B from
+    // the image
+    auto issue = [&](int L) {
+        tc_fence_after();
+        if (!elect_one()) return;
+        const uint32_t wb = sw + (L == 0 ? kTcW0 : L == 1 ? kTcW1 : L == 2 ? kTcW2 : kTcW3);
+        const uint32_t id = L == 3 ? umma_idesc_bf16_f32(128, 16) : umma_idesc_bf16_f32(128, 128);
+        const int ksteps = L == 0 ? 2 : 8, R = L == 3 ? 16 : 128;
 #pragma unroll
-        for (int kc = 0; kc < 4; kc++) xn[kc] = make_uint4(0u, 0u, 0u, 0u);
-        if (t < ntiles && t * kTcRows + r < rows)
-#pragma unroll
-            for (int kc = 0; kc < 4; kc++) xn[kc] = *reinterpret_cast<const uint4 *>(X + (size_t)(t * kTcRows + r) * ldx + kc * 8);
-        for (; t < ntiles && go; t += stride) {
-            const int row = t * kTcRows + r;
-#pragma unroll
-            for (int kc = 0; kc < 4; kc++) *reinterpret_cast<uint4 *>(sA + canon_off(r, kc * 8, kTcRows)) = xn[kc];
-            // the next tile's row of X, fetched while this tile's layers run
-            const int tn = t + stride;
-#pragma unroll
-            for (int kc = 0; kc < 4; kc++) xn[kc] = make_uint4(0u, 0u, 0u, 0u);
-            if (tn < ntiles && tn * kTcRows + r < rows)
-#pragma unroll
-                for (int kc = 0; kc < 4; kc++) xn[kc] = *reinterpret_cast<const uint4 *>(X + (size_t)(tn * kTcRows + r) * ldx + kc * 8);
-            fence_async_smem();
-            tc_fence_before();
-            named_bar(bar, 128);
-            if (r == 0) mbar_arrive(rd);
+        for (int st = 0; st < 8; st++)
+            if (st < ksteps) umma_bf16_ta(td, td + kTcACol + 8 * st, sw128_kmajor(wb, R, st), id, st > 0 ? 1u : 0u);
+        umma_commit(dn);
+    };
+    // this row's quarter pair of X (16 bf16: columns 16g..16g+15, g < 2) of a tile
+    uint4 xn[2];
+    auto load_x = [&](int tile) {
+        xn[0] = xn[1] = make_uint4(0u, 0u, 0u, 0u);
+        if (g < 2 && tile < ntiles && tile * kTcRows + r < rows) {
+            const uint4 *p = reinterpret_cast<const uint4 *>(X + (size_t)(tile * kTcRows + r) * ldx + 16 * g);
+            xn[0] = p[0];
+            xn[1] = p[1];
+        }
+    };
+    auto put_x = [&]() {
+        if (g < 2) tmem_st8(trow + kTcACol + 8 * g, xn[0], xn[1]);
+        tmem_wait_st();
+    };
+    bool ok = true, issued = false;
+    uint32_t phase = 0;
+    int t = blockIdx.x + sl * (int)gridDim.x;
+    if (t < ntiles) {
+        load_x(t);
+        put_x();
+        load_x(t + stride);                                   // fetched while the tile before it runs
+        tc_fence_before();
+        named_bar_or(1 + sl, kTcSlotThreads, false);
+        if (lead) { issue(0); issued = true; }
+    }
+    for (; t < ntiles && ok; t += stride) {
+        const int row = t * kTcRows + r;
 #pragma unroll 1
-            for (int layer = 0; layer < 4; layer++) {
-                // bounded wait for this layer's MMAs, then a warpgroup-uniform vote on the outcome
-                // (an OR over the warpgroup's flags, so no thread goes on to a barrier the others left)
-                bool fail = false;
-                int spins = 0;
-                while (!mbar_try(dn, dphase)) {
-                    if (*abort_flag) { fail = true; break; }
-                    if (++spins > wait_limit) { *abort_flag = 1; fail = true; break; }
-                }
-                if (named_bar_or(bar, 128, fail)) { go = false; break; }
-                dphase ^= 1u;
-                tc_fence_after();
-                if (layer < 3) {
-                    tc_epilogue_hidden(trow, sb + 128 * layer, sA, r);
-                    fence_async_smem();
-                    tc_fence_before();
-                    named_bar(bar, 128);
-                    if (r == 0) mbar_arrive(rd);
-                } else {
+        for (int layer = 0; layer < 4; layer++) {
+            const bool fail = !mbar_wait(dn, phase, wait_limit);
+            phase ^= 1u;
+            tc_fence_after();
+            if (layer < 3) {
+                tc_epilogue_hidden(trow + 32 * g, sb + 128 * layer + 32 * g, trow + kTcACol + 16 * g);
+            } else {
+                if (g == 0) {
                     uint32_t v;
                     tmem_ld1(trow, v);
                     tmem_wait_ld();
                     if (row < rows) y[row] = __uint_as_float(v) + sb[384];
-                    tc_fence_before();
-                    named_bar(bar, 128);   // the slot's columns and A buffer are free for the next tile
                 }
+                put_x();
+                load_x(t + 2 * stride);
             }
+            tc_fence_before();
+            ok = !named_bar_or(1 + sl, kTcSlotThreads, fail);
+            if (!ok) break;
+            if (lead && (layer < 3 || t + stride < ntiles)) issue((layer + 1) & 3);
         }
-    } else {
-      if (lane == 0) {
-        // ---- MMA warp: issues every layer of every slot as its A operand becomes ready
-        const uint32_t sw = smem_u32(sm);
-        const uint32_t id128 = umma_idesc_bf16_f32(128, 128), id16 = umma_idesc_bf16_f32(128, 16);
-        int left[kTcSlots], layer[kTcSlots];
-        uint32_t rphase[kTcSlots];
-        int remaining = 0;
-#pragma unroll
-        for (int sl = 0; sl < kTcSlots; sl++) {
-            const int t0 = blockIdx.x * kTcSlots + sl;
-            left[sl] = t0 < ntiles ? 4 * ((ntiles - 1 - t0) / stride + 1) : 0;
-            layer[sl] = 0;
-            rphase[sl] = 0u;
-            remaining += left[sl];
-        }
-        bool issued_any = false;
-        int spins = 0;
-        while (remaining > 0) {
-            bool progressed = false;
-#pragma unroll
-            for (int sl = 0; sl < kTcSlots; sl++) {
-                if (left[sl] == 0 || !mbar_try(smem_u32(ready + sl), rphase[sl])) continue;
-                rphase[sl] ^= 1u;
-                tc_fence_after();
-                const int L = layer[sl];
-                const int ksteps = L == 0 ? 2 : 8;
-                const uint32_t wb = sw + (L == 0 ? kTcW0 : L == 1 ? kTcW1 : L == 2 ? kTcW2 : kTcW3);
-                const uint32_t blbo = L == 3 ? 16 * 16 : 128 * 16;
-                const uint32_t sa = sw + kTcA + sl * kTcABytes;
-                for (int st = 0; st < ksteps; st++) {
-                    const uint64_t ad = umma_smem_desc(sa + 2 * st * (128 * 16), 128 * 16, 128);
-                    const uint64_t bd = umma_smem_desc(wb + 2 * st * blbo, blbo, 128);
-                    umma_bf16(tmem + 128 * sl, ad, bd, L == 3 ? id16 : id128, st > 0 ? 1u : 0u);
-                }
-                umma_commit(smem_u32(done + sl));
-                issued_any = true;
-                layer[sl] = (L + 1) & 3;
-                left[sl]--;
-                remaining--;
-                progressed = true;
-            }
-            if (progressed) {
-                spins = 0;
-            } else {
-                if (*abort_flag) break;
-                if (++spins > wait_limit) { *abort_flag = 1; break; }
-            }
-        }
-        if (issued_any) {
-            // every MMA this thread issued completes before the columns are released, also those
-            // whose completion no warpgroup waited for after an abort: one more commit tracks all
-            // of them, waited for with the full bound
-            umma_commit(smem_u32(drain));
-            mbar_wait(smem_u32(drain), 0u, kTcWaitLimit);
-        }
-      }
-      __syncwarp();
     }
+    if (issued) {
+        // every MMA this thread issued completes before the columns are released: one more commit
+        // tracks them all, waited for with the full bound
+        if (elect_one()) umma_commit(smem_u32(drain + sl));
+        mbar_wait(smem_u32(drain + sl), 0u, kTcWaitLimit);
+    }
+    if (lead && lane == 0 && !ok) atomicExch(&g_mlp_tc_status, 1);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    if (*abort_flag && tid == 0) atomicExch(&g_mlp_tc_status, 1);
     if (warp == 0)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem), "r"(kTcCols) : "memory");
 }
@@ -1645,7 +1612,7 @@ size_t cmf_emu_mlp_tc_pack_bytes(void) { return (size_t)kTcWBytes; }
 int cmf_emu_mlp_tc_pack(const void *W0, const void *W1, const void *W2, const void *W3, int ldw3, void *pack, void *stream) {
     if (!W0 || !W1 || !W2 || !W3 || !pack || ldw3 < 16 || ((uintptr_t)pack & 15))
         return emu_err(CMF_E_ARG, "cmf_emu_mlp_tc_pack: bad arguments (ldw3 >= 16, pack 16-byte aligned)");
-    const int n = 128 * 32 + 2 * 128 * 128 + 16 * 128;
+    const int n = 128 * 64 + 2 * 128 * 128 + 16 * 128;
     k_mlp_tc_pack<<<(n + 255) / 256, 256, 0, (cudaStream_t)stream>>>(
         (const __nv_bfloat16 *)W0, (const __nv_bfloat16 *)W1, (const __nv_bfloat16 *)W2, (const __nv_bfloat16 *)W3, ldw3,
         (__nv_bfloat16 *)pack);
@@ -1666,8 +1633,7 @@ int cmf_emu_mlp_tc(const void *X, int ldx, int rows, const void *pack, const flo
     EMU_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     EMU_TRY(cudaFuncSetAttribute(k_mlp_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem));
     const int ntiles = (rows + kTcRows - 1) / kTcRows;
-    const int want = (ntiles + kTcSlots - 1) / kTcSlots;
-    const int grid = want < sms ? want : sms;
+    const int grid = ntiles < sms ? ntiles : sms;
     k_mlp_tc<<<grid, kTcThreads, kTcSmem, (cudaStream_t)stream>>>((const __nv_bfloat16 *)X, ldx, rows, (const uint4 *)pack,
                                                                   b0, b1, b2, b3, y, g_tc_wait_limit);
     EMU_TRY(cudaGetLastError());

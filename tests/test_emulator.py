@@ -257,6 +257,32 @@ def test_tcgen05_inference_matches_mma_sync_and_reference(R):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("R", [1, 127, 129, 128 * 148 + 1, 128 * 296 + 16, 128 * 444 + 127, 128 * 740])
+def test_tcgen05_inference_does_not_depend_on_a_rows_tile(R):
+    """Rows dealt to another tile, slot, CTA and lane (a permutation, remainders of a tile, one to three
+    tiles per slot) give the same bits, and nothing is written past the last row."""
+    import torch
+
+    from cmf_b200.emulator import MLP, _emu_lib
+
+    dev = torch.device("cuda", 0)
+    rng = np.random.default_rng(R)
+    mlp = MLP(dev, seed=4)
+    W, b = _rand_params(rng, 0.2)
+    mlp.load({"W": W, "b": b})
+    X = torch.tensor(rng.standard_normal((R, 64)), device=dev).to(torch.bfloat16)
+    X[:, 30:] = 0
+    perm = torch.tensor(rng.permutation(R), device=dev)
+    out = torch.full((2, R + 128), float("nan"), dtype=torch.float32, device=dev)
+    mlp.infer_tc(X, out[0, :R])
+    mlp.infer_tc(X[perm].contiguous(), out[1, :R])
+    torch.cuda.synchronize()
+    assert _emu_lib().cmf_emu_mlp_tc_status() == 0
+    assert torch.isfinite(out[:, :R]).all() and torch.isnan(out[:, R:]).all()
+    assert torch.equal(out[0, :R][perm], out[1, :R])
+
+
+@pytest.mark.gpu
 def test_tcgen05_bounded_wait_reports_and_recovers():
     """With the MMA completion bound set to 0 every tcgen05 launch gives up at its first wait: the
     kernel still drains its MMA in flight and frees its tensor memory, returns, and the status
