@@ -418,15 +418,20 @@ __device__ __forceinline__ float manning_q(float area, float h, float s, float i
     return copysignf(area * __expf(0.6666667f * __logf(h)) * sqrtf(fabsf(s)) * inv_man, s);
 }
 
+// Bound by the latency of its 35 loads a cell, so six blocks per SM are asked for (54 registers and four
+// blocks without it); a row leaves through shared memory, four lanes writing its 64 bytes together, where a
+// lane per row wrote half a sector at a time.  32 x 299k cells, the hop pairs included: 1337 us as one row a
+// lane, 1313 us through shared memory, 1218 us with six blocks (seven: 1262 us).
 // features of cell i of member blockIdx.y; planes [2*(hops+1)][M*N] (0,1 = seeds; 2h+2, 2h+3 = hop h)
-__global__ void k_emu_assemble(EmuNet n, const double *__restrict__ rivsto, const double *__restrict__ fldsto,
+__global__ void __launch_bounds__(256, 6) k_emu_assemble(EmuNet n, const double *__restrict__ rivsto, const double *__restrict__ fldsto,
                                const double *__restrict__ levsto, const double *__restrict__ rivdph,
                                const double *__restrict__ flddph, const double *__restrict__ fldfrc,
                                const double *__restrict__ qprev, const double *__restrict__ runoff,
                                const float *__restrict__ planes, size_t plane, int hops, __nv_bfloat16 *X, int ldx,
                                int rows_per_member) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n.N) return;
+    __shared__ uint4 rows_s[8][128];
+    const int i0 = blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = min(i0, n.N - 1);
     // member blockIdx.y: state arrays are member-major [M][N], X rows [M][rows_per_member]
     const size_t mo = (size_t)blockIdx.y * n.N, gi = mo + i;
     const float qf = (float)n.qref[i];
@@ -469,7 +474,8 @@ __global__ void k_emu_assemble(EmuNet n, const double *__restrict__ rivsto, cons
     const float af = fmaxf((float)fldsto[gi] * __frcp_rn(len) - fdph * wth, 0.f);
     f[30] = fslog(manning_q(wth * rdph, rdph, slope, __frcp_rn((float)n.rivman[i])) * iq);
     f[31] = fslog(manning_q(af, fdph, fmaxf(-0.005f, fminf(0.005f, slope)), __frcp_rn((float)n.pmanfld)) * iq);
-    uint4 *row = reinterpret_cast<uint4 *>(X + ((size_t)blockIdx.y * rows_per_member + i) * ldx);
+    const int lane = threadIdx.x & 31;
+    uint4 *ws = rows_s[threadIdx.x >> 5];
 #pragma unroll
     for (int v = 0; v < 4; v++) {
         uint4 u;
@@ -477,7 +483,14 @@ __global__ void k_emu_assemble(EmuNet n, const double *__restrict__ rivsto, cons
         u.y = pack_bf16x2(f[8 * v + 2], f[8 * v + 3]);
         u.z = pack_bf16x2(f[8 * v + 4], f[8 * v + 5]);
         u.w = pack_bf16x2(f[8 * v + 6], f[8 * v + 7]);
-        row[v] = u;
+        ws[lane * 4 + (v ^ ((lane >> 1) & 3))] = u;
+    }
+    __syncwarp();
+    __nv_bfloat16 *xw = X + ((size_t)blockIdx.y * rows_per_member + (i0 - lane)) * ldx;
+#pragma unroll
+    for (int v = 0; v < 4; v++) {
+        const int r = 8 * v + (lane >> 2), c = lane & 3;
+        if (i0 - lane + r < n.N) *reinterpret_cast<uint4 *>(xw + (size_t)r * ldx + 8 * c) = ws[r * 4 + (c ^ ((r >> 1) & 3))];
     }
 }
 
