@@ -318,11 +318,10 @@ int build_net(cmf_gpu_ctx *c, const cmf_map_ptrs *mp) {
             for (int p : pi_idx) if (p < 0 || p >= P) return set_err(CMF_E_ARG, "I1P_INF out of range");
         }
         // the ends of paths by cell (Net::pend)
-        std::vector<int> pos(N, -1), ptr(1, 0);
-        std::vector<int2> ends;
+        std::vector<int2> range(N, make_int2(0, 0)), ends;
         for (int i = 0; i < N; i++) {
             if (po_ptr[i + 1] == po_ptr[i] && pi_ptr[i + 1] == pi_ptr[i]) continue;
-            pos[i] = (int)ptr.size() - 1;
+            range[i].x = (int)ends.size();
             for (int e = po_ptr[i]; e < po_ptr[i + 1]; e++) {
                 const int p = po_idx[e];
                 ends.push_back(make_int2(p, skip[p] & 1 ? -1 : pu[p] == i ? pd[p] : -2));
@@ -331,9 +330,9 @@ int build_net(cmf_gpu_ctx *c, const cmf_map_ptrs *mp) {
                 const int p = pi_idx[e];
                 ends.push_back(make_int2(~p, skip[p] & 1 ? -1 : pd[p] == i ? pu[p] : -2));
             }
-            ptr.push_back((int)ends.size());
+            range[i].y = (int)ends.size();
         }
-        if ((rc = c->upload(&n.path_pos, pos)) || (rc = c->upload(&n.pend_ptr, ptr)) || (rc = c->upload(&n.pend, ends))) return rc;
+        if ((rc = c->upload(&n.path_ends, range)) || (rc = c->upload(&n.pend, ends))) return rc;
         if ((rc = c->upload(&n.pth_up, pu)) || (rc = c->upload(&n.pth_dn, pd)) || (rc = c->upload(&n.pth_dst, dst)) || (rc = c->upload(&n.pth_elv, elv)) || (rc = c->upload(&n.pth_wth, wth)) ||
             (rc = c->upload(&n.pth_man, man)))
             return rc;

@@ -109,12 +109,11 @@ struct Net {
     const int *__restrict__ pth_skip;                        // [P] bit0 plain/LSPAMAT skip, bit1 levee skip, bits 2
                                                              // and 3: a levee fraction below 1 at the ends
     const double *__restrict__ pth_dst, *__restrict__ pth_elv, *__restrict__ pth_wth, *__restrict__ pth_man;
-    // the ends of paths: per cell with C_PATH its position (path_pos [N]), per position a range of entries,
-    // the cell's I1P_OUT paths and then its I1P_INF paths, each in list order.  An entry holds the path
+    // the ends of paths: per cell its range of entries (path_ends [N], read where C_PATH is set), the
+    // cell's I1P_OUT paths and then its I1P_INF paths, each in list order.  An entry holds the path
     // (x, ~path for I1P_INF) and the cell at its other end (y; -1: not rescaled, -2: the cell is
-    // not this path's end), so a path's flow and the
-    // rate it may need come one load after the entry.
-    const int *__restrict__ path_pos, *__restrict__ pend_ptr;
+    // not this path's end), so a path's flow and the rate it may need come one load after the entry.
+    const int2 *__restrict__ path_ends;
     const int2 *__restrict__ pend;
     // levee (compact per levee cell)
     const int *__restrict__ lev_id;     // [N] -1 when the cell carries the no-levee sentinels
@@ -1029,29 +1028,53 @@ __device__ __forceinline__ double level_sum(int Lp, int lane0, const double (&v)
 }
 
 // Phase A of one path lane (every lane of the warp calls it): the level's flux, and the limiter on the
-// sum over the levels
+// sum over the levels.  Its time is rounds of dependent loads, so there are two: what the lane's own
+// indices address, then what the path's ends do, read whether or not the branches below come to need it
+// (each read where it is used: five rounds; with path_rescale's two instead of four and the cells' own
+// range of path ends, a sub-step of 298,554 cells in the resident kernel 44.4 -> 43.1 us, of 2M cells by
+// phase kernels 304 -> 294 us).
 template <bool Coherent>
 __device__ __forceinline__ void path_outflow(const Net &n, const State &s, int m, const PathLane &t, double DT) {
     const int P = n.P, Lp = n.Lp, p = t.p;
     const size_t base = (size_t)m * n.N, pb = (size_t)m * Lp * P;
-    const int skip = t.on ? __ldg(&n.pth_skip[p]) : 3;
-    const bool live = t.on && !(n.llevee ? (skip & 2) : (skip & 1));
-    double f[2] = {0.0, 0.0};
-    int u = 0, d = 0;
-    if (live) {
+    int skip = 3, u = 0, d = 0;
+    double dst = 1.0, elv = 0.0, wth = 0.0, man = 0.0, pre = 0.0;
+    auto level = [&](int l) {
+        const size_t o = (size_t)l * P + p;
+        elv = __ldg(&n.pth_elv[o]);
+        wth = __ldg(&n.pth_wth[o]);
+        man = __ldg(&n.pth_man[l]);
+        pre = s.pthflw_pre[pb + o];
+    };
+    if (t.on) {
+        skip = __ldg(&n.pth_skip[p]);
         u = __ldg(&n.pth_up[p]);
         d = __ldg(&n.pth_dn[p]);
+        dst = __ldg(&n.pth_dst[p]);
+        level(t.l);
+    }
+    const bool live = t.on && !(n.llevee ? (skip & 2) : (skip & 1));
+    double f[2] = {0.0, 0.0}, sto = 0.0;
+    if (live) {
         const double gdt = n.pgrv * DT;
         const double eu = __ldg(&n.rivelv[u]), ed = __ldg(&n.rivelv[d]);
         const double2 du = end_depth<Coherent>(s, base + u), dd = end_depth<Coherent>(s, base + d);
+        const double stu = ld_nb<Coherent>(s.storge, base + u), std = ld_nb<Coherent>(s.storge, base + d);
+        const bool leveed = n.llevee && t.l > 0;
+        double lu = 0.0, ld = 0.0;
+        if (leveed && (skip & 4)) lu = __ldg(&n.elevtn[u]) + ld_nb<Coherent>(s.levdph, base + u);
+        if (leveed && (skip & 8)) ld = __ldg(&n.elevtn[d]) + ld_nb<Coherent>(s.levdph, base + d);
+        sto = dmin(stu, std);
         const double su = eu + du.x, sd = ed + dd.x;
-        double dslp = (su - sd) / __ldg(&n.pth_dst[p]);
+        double dslp = (su - sd) / dst;
         dslp = dmax(-0.005, dmin(0.005, dslp));
 #pragma unroll 1
         for (int h = 0, l = t.l; l < Lp; h++, l += 32) {
-            const size_t o = (size_t)l * P + p;
-            const double elv = __ldg(&n.pth_elv[o]), wth = __ldg(&n.pth_wth[o]), man = __ldg(&n.pth_man[l]);
-            const double pre = s.pthflw_pre[pb + o];
+            if (h > 0) {
+                level(l);
+                if (skip & 4) lu = __ldg(&n.elevtn[u]) + ld_nb<Coherent>(s.levdph, base + u);
+                if (skip & 8) ld = __ldg(&n.elevtn[d]) + ld_nb<Coherent>(s.levdph, base + d);
+            }
             const bool channel = !n.llevee || l == 0;    // with levees: level 1, the river channel
             double im;
             if (channel) {
@@ -1063,8 +1086,8 @@ __device__ __forceinline__ void path_outflow(const Net &n, const State &s, int m
                 else if (im <= 0.0) im = dflw;           // semi-implicit depth
             } else {
                 double slu = su, sld = sd;
-                if (skip & 4) slu = dmin(__ldg(&n.elevtn[u]) + ld_nb<Coherent>(s.levdph, base + u), su);
-                if (skip & 8) sld = dmin(__ldg(&n.elevtn[d]) + ld_nb<Coherent>(s.levdph, base + d), sd);
+                if (skip & 4) slu = dmin(lu, su);
+                if (skip & 8) sld = dmin(ld, sd);
                 im = dmax(dmax(slu, sld) - elv, 0.0);
             }
             const double v = im > 1.E-5 ? path_flux(wth, pre, gdt, im, dslp, man, !channel) : 0.0;
@@ -1075,7 +1098,7 @@ __device__ __forceinline__ void path_outflow(const Net &n, const State &s, int m
     double sum = level_sum(Lp, t.lane0, f);
     if (!live) sum = 0.0;
     if (sum != 0.0) {
-        const double rate = rate_min1(0.05 * dmin(ld_nb<Coherent>(s.storge, base + u), ld_nb<Coherent>(s.storge, base + d)), fabs(sum * DT));
+        const double rate = rate_min1(0.05 * sto, fabs(sum * DT));
         f[0] = f[0] * rate;
         f[1] = f[1] * rate;
         sum = sum * rate;
@@ -1138,8 +1161,8 @@ __device__ __forceinline__ void cell_rate(const Net &n, const State &s, const Ow
     so = so * DT;
     if (w.flags() & C_PATH) {
         const double *sum = s.pthsum_raw + (size_t)m * n.P;
-        const int q = __ldg(&n.path_pos[i]), e1 = __ldg(&n.pend_ptr[q + 1]);
-        for (int e = __ldg(&n.pend_ptr[q]); e < e1; e++) {
+        const int2 ends = __ldg(&n.path_ends[i]);
+        for (int e = ends.x; e < ends.y; e++) {
             const int p = __ldg(&n.pend[e].x);
             const double v = w.nb(sum, p >= 0 ? p : ~p);
             so = so + dmax(p >= 0 ? v : -v, 0.0) * DT;
@@ -1187,15 +1210,29 @@ __device__ __forceinline__ void path_rescale(const Net &n, const State &s, int m
     const double *rate_m = s.rate + base;
     double a[2] = {0.0, 0.0};
     if (t.on) {
-        const bool sk = __ldg(&n.pth_skip[p]) & 1;
+        // two rounds of loads: the path's own values, then the rates of both ends
+        const bool sk = __ldg(&n.pth_skip[p]) & 1, add = n.ldiag && !first;
+        const int u = __ldg(&n.pth_up[p]), d = __ldg(&n.pth_dn[p]);
+        size_t o = pb + (size_t)t.l * P + p;
+        double f = s.pthflw_raw[o], x0 = add ? s.a_pthflw[o] : 0.0;
+        const double sum = t.l == 0 ? ld_nb<Coherent>(s.pthsum_raw, (size_t)m * P + p) : 0.0;
+        double ru = 1.0, rd = 1.0;
+        if (!sk) {
+            ru = ld_nb<Coherent>(rate_m, u);
+            rd = ld_nb<Coherent>(rate_m, d);
+        }
+        if (t.l == 0) s.pthsum[(size_t)m * P + p] = sk ? sum : sum * (sum >= 0.0 ? ru : rd);
 #pragma unroll 1
         for (int h = 0, l = t.l; l < Lp; h++, l += 32) {
-            const size_t o = pb + (size_t)l * P + p;
-            double f = s.pthflw_raw[o];
-            if (!sk) f = f * ld_nb<Coherent>(rate_m, f >= 0.0 ? __ldg(&n.pth_up[p]) : __ldg(&n.pth_dn[p]));
+            if (h > 0) {
+                o = pb + (size_t)l * P + p;
+                f = s.pthflw_raw[o];
+                x0 = add ? s.a_pthflw[o] : 0.0;
+            }
+            if (!sk) f = f * (f >= 0.0 ? ru : rd);
             s.pthflw_pre[o] = f;
             if (n.ldiag) {
-                double x = first ? f * DT : s.a_pthflw[o] + f * DT;
+                double x = first ? f * DT : x0 + f * DT;
                 if (last) {
                     x = x / (nadd + DT);
                     if (n.ldiag_out) s.o_pthflw[o] = s.o_pthflw[o] + x * dt_def;
@@ -1206,11 +1243,9 @@ __device__ __forceinline__ void path_rescale(const Net &n, const State &s, int m
             }
         }
     }
-    double asum = 0.0;
-    if (n.ldiag && last) asum = level_sum(Lp, t.lane0, a);
-    if (t.on && t.l == 0) {
-        s.pthsum[(size_t)m * P + p] = scaled_pathsum<Coherent>(n, s.pthsum_raw + (size_t)m * P, rate_m, p);
-        if (n.ldiag && last) s.a_pthsum[(size_t)m * P + p] = asum;
+    if (n.ldiag && last) {
+        const double asum = level_sum(Lp, t.lane0, a);
+        if (t.on && t.l == 0) s.a_pthsum[(size_t)m * P + p] = asum;
     }
 }
 
@@ -1250,8 +1285,8 @@ __device__ __forceinline__ void cell_store(const Net &n, const State &s, Own &w,
     const bool has_path = w.flags() & C_PATH;
     if (has_path) {
         const double *sum = s.pthsum_raw + (size_t)m * n.P;
-        const int q = __ldg(&n.path_pos[i]), e1 = __ldg(&n.pend_ptr[q + 1]);
-        for (int e = __ldg(&n.pend_ptr[q]); e < e1; e++) {
+        const int2 ends = __ldg(&n.path_ends[i]);
+        for (int e = ends.x; e < ends.y; e++) {
             const int2 t = __ldg(&n.pend[e]);
             const bool up = t.x >= 0;              // this cell is the path's upstream end
             double v = w.nb(sum, up ? t.x : ~t.x);
