@@ -86,6 +86,7 @@ struct cmf_gpu_ctx {
     int persist_grid = 0;       // co-resident CTAs of the persistent kernel (0: it cannot run here)
     cmf::ResArgs res{};         // its resident form (group 0: a member does not fit the SMs)
     int res_threads = 0;
+    void (*res_kernel)(cmf::Net, cmf::State, cmf::ResArgs) = nullptr;   // k_resident with the registers its tasks leave
     bool l2_window = false;     // the hot maps sit under a persisting L2 access-policy window
     bool persist = false;       // outer steps run as one persistent cooperative launch
     Tuner tune;                 // online autotuner state
@@ -697,10 +698,13 @@ int persist_setup(cmf_gpu_ctx *c) {
         a.slots = (int)((tiles + grid - 1) / grid);
         // a warp per tile and per path tile, up to the CTA's limit
         const long long ptiles = group * (cmf::path_threads(c->net.P, c->net.Lp) / 32);
-        const int threads = 32 * (int)std::min<long long>(cmf::kResThreads / 32, a.slots + (ptiles + grid - 1) / grid + 1);
-        CUDA_TRY(cudaFuncSetAttribute(cmf::k_resident, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        const long long tasks = a.slots + (ptiles + grid - 1) / grid;
+        const bool few = tasks <= cmf::kResFewTasks;
+        const int threads = 32 * (int)std::min<long long>((few ? cmf::kResThreadsFew : cmf::kResThreadsMany) / 32, tasks + 1);
+        c->res_kernel = few ? cmf::k_resident<cmf::kResThreadsFew> : cmf::k_resident<cmf::kResThreadsMany>;
+        CUDA_TRY(cudaFuncSetAttribute(c->res_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       (int)cmf::res_smem(cmf::kResMaxSlots)));
-        CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, cmf::k_resident, threads, cmf::res_smem(a.slots)));
+        CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, c->res_kernel, threads, cmf::res_smem(a.slots)));
         if (per_sm >= 1) {
             a.tpm = (int)tpm;
             a.group = (int)group;
@@ -730,7 +734,7 @@ int launch_persist(cmf_gpu_ctx *c, unsigned long long selftest_ns = 0) {
         cmf::ResArgs a = c->res;
         if (selftest_ns) { a.wait_ns = selftest_ns; a.selftest = 1; }
         void *args[] = {&c->net, &c->st, &a};
-        CUDA_TRY(cudaLaunchCooperativeKernel((const void *)cmf::k_resident, dim3(c->persist_grid), dim3(c->res_threads), args,
+        CUDA_TRY(cudaLaunchCooperativeKernel((const void *)c->res_kernel, dim3(c->persist_grid), dim3(c->res_threads), args,
                                              cmf::res_smem(a.slots), c->stream));
     } else {
         cmf::PersistArgs a{};

@@ -421,14 +421,16 @@ struct StageOut {
 };
 
 // The floodplain layers a storage fills, from the channel up: I full layers (0-based layer in use, L: all),
-// the storage, width and depth below it, and its gradient.  Layers are read two at a time: the scan
-// costs one dependent round per two layers (four at a time spilled in k_store).
+// the storage, width and depth below it, and its gradient.  Layers are read B at a time, one dependent
+// round per B layers: two in the phase kernels (four at a time spilled in k_store), one in the resident
+// kernel, where the registers of a second layer spilled past its little L1 (298,554 cells: 42.4 us per
+// sub-step with two, 38.4 us with one).
 struct Filled {
     int I;
     double sfil, wfil, dfil, grd;
 };
+template <int B>
 __device__ __forceinline__ Filled fill_layers(const Net &n, int i, double pstoall, double rsm, double wth, double inc) {
-    constexpr int B = 2;
     const int N = n.N, L = n.L;
     Filled f{0, rsm, wth, 0.0, 0.0};
     for (int l0 = 0; l0 < L; l0 += B) {
@@ -499,7 +501,7 @@ __device__ __forceinline__ StageOut stage(const Net &n, const Own &w, int i, con
         lcase = pstoall < lbas ? 1 : pstoall < ltop ? 2 : pstoall < lfil ? 3 : 4;
     }
     if (lcase == 1 || lcase == 4) {
-        const Filled f = fill_layers(n, i, pstoall, rsm, wth, inc);
+        const Filled f = fill_layers<Own::kResident ? 1 : 2>(n, i, pstoall, rsm, wth, inc);
         double wadd;
         if (f.I < L) {
             wadd = -f.wfil + sqrt(f.wfil * f.wfil + ((2.0 * (pstoall - f.sfil)) / len) / f.grd);
@@ -936,6 +938,22 @@ __device__ __forceinline__ void cell_outflow(const Net &n, const State &s, Own &
         dwn = __ldg(&n.dwnelv[i]);
         inv_dst = 1.0 / n.pdstmth;
     }
+    // the floodplain's maps and state, read where a first test passes; the resident kernel knows from the
+    // cell's bits that there is water on it and reads them with everything else
+    double inv_len = 0.0, fdph = 0.0, elv = 0.0, hgt = 0.0, fsto_pre = 0.0;
+    auto read_area = [&] { inv_len = w.inv_rivlen(i); fdph = w.flddph(gi); };
+    auto read_flow = [&] { elv = w.elevtn(i); hgt = w.rivhgt(i); fsto_pre = w.fldsto_pre(gi); };
+    if constexpr (Own::kResident)
+        if (n.lfldout && w.flooded()) {
+            read_area();
+            read_flow();
+        }
+    // diagnostics of sub-step k-1: here, so that their sums come with the downstream depth and hold no
+    // registers across the flow equations
+    if (n.ldiag && k > 0) {
+        if constexpr (Own::kResident) w.carry(gi, DT, k == 1, rivout_pre, fldout_pre, rivdph, storge);
+        else diag_carry(s, w, gi, DT, k == 1, rivout_pre, fldout_pre, rivdph, storge);
+    }
     double dslp = (sfc - dwn) * inv_dst;
     double rout, fout = 0.0, rvel;
     {
@@ -953,16 +971,17 @@ __device__ __forceinline__ void cell_outflow(const Net &n, const State &s, Own &
         // the reference's masks are a double at river cells and a default-real literal at mouths
         const double eps = river ? 1.E-5 : CMF_F(1.E-5);
         // without floodplain water the area is max(-FLDDPH * RIVWTH, 0) = 0: nothing more to read
-        const double inv_len = fsto != 0.0 ? w.inv_rivlen(i) : 0.0;
-        const double dare = fsto != 0.0 ? dmax(fsto * inv_len - w.flddph(gi) * wth, 0.0) : 0.0;
+        if constexpr (!Own::kResident)
+            if (fsto != 0.0) read_area();
+        const double dare = fsto != 0.0 ? dmax(fsto * inv_len - fdph * wth, 0.0) : 0.0;
         if (dare > eps) {
-            const double elv = w.elevtn(i);
+            if constexpr (!Own::kResident) read_flow();
             dslp = dmax(-0.005, dmin(0.005, dslp));
             const double df = river ? dmax(dsfc - elv, 0.0) : sfc - elv;
             const double df_pr = dsfc_pre - elv;
             const double dflw_im = dmax(sqrt(dmax(df * df_pr, 0.0)), 1.E-6);
-            const double flddph_pre = dmax(rivdph_pre - w.rivhgt(i), 0.0);
-            const double dare_pr = dmax(w.fldsto_pre(gi) * inv_len - flddph_pre * wth, 1.E-6);
+            const double flddph_pre = dmax(rivdph_pre - hgt, 0.0);
+            const double dare_pr = dmax(fsto_pre * inv_len - flddph_pre * wth, 1.E-6);
             const double dare_im = dmax(sqrt(dare * dare_pr), 1.E-6);
             const double dout_pr = fldout_pre;
             const double dout = (dout_pr + (gdt * dare_im) * dslp)
@@ -979,10 +998,6 @@ __device__ __forceinline__ void cell_outflow(const Net &n, const State &s, Own &
         fout = fout * rate;
     }
     if (!(w.flags() & C_DAM)) w.put_raw(gi, i, rout, fout);
-    if (n.ldiag && k > 0) {              // diagnostics of sub-step k-1
-        if constexpr (Own::kResident) w.carry(gi, DT, k == 1, rivout_pre, fldout_pre, rivdph, storge);
-        else diag_carry(s, w, gi, DT, k == 1, rivout_pre, fldout_pre, rivdph, storge);
-    }
     if (!(w.flags() & C_KIN)) vel_average(n, s, w, gi, DT, nt, dt_def, k, rvel);
 }
 
@@ -1324,22 +1339,11 @@ __device__ __forceinline__ void cell_store(const Net &n, const State &s, Own &w,
     rs = rs + (runoff * (1.0 - frc)) * DT;       // D2GDWRTN is zero without groundwater delay
     fs = fs + (runoff * frc) * DT;
     bput(2, n.llevee ? (rs + fs) + levsto : rs + fs);
-    // stage scheme, :125
-    if constexpr (!Own::kResident) map = stage_map(w, i);
-    const StageOut o = stage(n, w, i, map, rs, fs, levsto);
-    // CALC_VARS_PRE, src/cmf_ctrl_physics_mod.F90:254-277, and the dam storage
+    bput(5, n.llevee ? (rs + fs) + levsto : rs + fs);
+    // What the new storage does not change leaves before the stage scheme, so that it holds no registers
+    // across it.  CALC_VARS_PRE, src/cmf_ctrl_physics_mod.F90:254-277, and the dam storage:
     w.put_pre(gi, rout, fout, rivdph0, fldsto0, last);
     if (dam) s.damsto[gi] = damsto1;
-    // CMF_CheckNanB-style probe (src/cmf_utils_mod.F90:807-815) on the new storage: a NaN or
-    // infinite runoff or state surfaces as a positive status instead of a silent NaN state
-    if (!isfinite((o.rivsto + o.fldsto) + o.levsto)) s.ctl[m].err = kErrNonFinite;
-    store_stage(n, s, w, gi, i, o, rivdph0, last);
-    bput(5, n.llevee ? (rs + fs) + levsto : rs + fs);
-    bput(6, n.llevee ? (o.rivsto + o.fldsto) + o.levsto : o.rivsto + o.fldsto);
-    bput(7, o.rivsto);
-    bput(8, o.fldsto);
-    bput(9, o.fldare);
-    bput(10, o.levsto);
     if (last) {   // diagnostics read by nothing inside the sub-step loop
         s.rivinf[gi] = rinf;
         s.fldinf[gi] = finf;
@@ -1351,11 +1355,11 @@ __device__ __forceinline__ void cell_store(const Net &n, const State &s, Own &w,
     // D2PTHOUT_aAVG: D2PTHINF is never written by the reference (always 0), and a cell without
     // bifurcation channels adds +0 every sub-step, so its average (and output average) stays at the
     // +0 the arrays were created with; cells with channels accumulate it here every sub-step.
+    // CMF_DIAG_AVEMAX_OUTPUT (src/cmf_calc_diag_mod.F90:272-318) on the last sub-step: the output
+    // interval accumulates the finished sub-step average times DT_DEF.
+    const bool out = last && n.ldiag_out;
     if (n.ldiag && (last || has_path)) {
         const double na = nadd + DT;
-        // CMF_DIAG_AVEMAX_OUTPUT (src/cmf_calc_diag_mod.F90:272-318) on the last sub-step: the
-        // output interval accumulates the finished sub-step average times DT_DEF
-        const bool out = last && n.ldiag_out;
         const double ddef = dt_def;
         auto acc = [&](double prev, double *a, double *oa, double v) {
             double x = first ? v * DT : prev + v * DT;
@@ -1367,9 +1371,7 @@ __device__ __forceinline__ void cell_store(const Net &n, const State &s, Own &w,
         if (last) {
             // every previous accumulator is read before the first of them is stored
             const double pro = first ? 0.0 : w.a_rivout(gi), pfo = first ? 0.0 : w.a_fldout(gi);
-            const double pof = first ? 0.0 : w.a_outflw(gi);
-            const double pmo = first ? 0.0 : w.m_outflw(gi), pmd = first ? 0.0 : w.m_rivdph(gi);
-            const double pms = first ? 0.0 : w.m_storge(gi);
+            const double pof = first ? 0.0 : w.a_outflw(gi), pmo = first ? 0.0 : w.m_outflw(gi);
             const double dinf = n.ldamout ? s.daminf[gi] : 0.0;
             const double pdi = n.ldamout ? daminf_sum(s, gi, w.flags(), DT, nt, dinf) : 0.0;
             acc(pro, s.a_rivout, s.o_rivout, rout);
@@ -1384,18 +1386,32 @@ __device__ __forceinline__ void cell_store(const Net &n, const State &s, Own &w,
             s.a_runoff[gi] = a;
             if (out) s.o_runoff[gi] = s.o_runoff[gi] + a * ddef;
             if (n.ldamout) acc(pdi, s.a_daminf, s.o_daminf, dinf);
-            const double stg = n.llevee ? (o.rivsto + o.fldsto) + o.levsto : o.rivsto + o.fldsto;
             const double mo = dmax(pmo, fabs(outflw));
-            const double md = dmax(pmd, o.rivdph);
-            const double ms = dmax(pms, stg);
             s.m_outflw[gi] = mo;
-            s.m_rivdph[gi] = md;
-            s.m_storge[gi] = ms;
-            if (out) {
-                s.om_outflw[gi] = dmax(s.om_outflw[gi], fabs(mo));
-                s.om_rivdph[gi] = dmax(s.om_rivdph[gi], md);
-                s.om_storge[gi] = dmax(s.om_storge[gi], ms);
-            }
+            if (out) s.om_outflw[gi] = dmax(s.om_outflw[gi], fabs(mo));
+        }
+    }
+    // stage scheme, :125
+    if constexpr (!Own::kResident) map = stage_map(w, i);
+    const StageOut o = stage(n, w, i, map, rs, fs, levsto);
+    // CMF_CheckNanB-style probe (src/cmf_utils_mod.F90:807-815) on the new storage: a NaN or
+    // infinite runoff or state surfaces as a positive status instead of a silent NaN state
+    if (!isfinite((o.rivsto + o.fldsto) + o.levsto)) s.ctl[m].err = kErrNonFinite;
+    store_stage(n, s, w, gi, i, o, rivdph0, last);
+    bput(6, n.llevee ? (o.rivsto + o.fldsto) + o.levsto : o.rivsto + o.fldsto);
+    bput(7, o.rivsto);
+    bput(8, o.fldsto);
+    bput(9, o.fldare);
+    bput(10, o.levsto);
+    if (n.ldiag && last) {
+        const double pmd = first ? 0.0 : w.m_rivdph(gi), pms = first ? 0.0 : w.m_storge(gi);
+        const double stg = n.llevee ? (o.rivsto + o.fldsto) + o.levsto : o.rivsto + o.fldsto;
+        const double md = dmax(pmd, o.rivdph), ms = dmax(pms, stg);
+        s.m_rivdph[gi] = md;
+        s.m_storge[gi] = ms;
+        if (out) {
+            s.om_rivdph[gi] = dmax(s.om_rivdph[gi], md);
+            s.om_storge[gi] = dmax(s.om_storge[gi], ms);
         }
     }
 }

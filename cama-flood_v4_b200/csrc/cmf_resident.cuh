@@ -16,11 +16,10 @@
 // Why: a sub-step of the phase kernels moves about 530 B per cell through L2 or HBM, and its time is
 // dependent rounds of loads in three launches.  Here a phase of a cell is one round: static values and
 // neighbours' results, addressed from shared memory.  Measured per sub-step (B200): 298,554 cells with
-// channels, levees and dams 43 us (phase kernels 57; one persistent kernel over global memory 82),
-// 2 x 26,691 cells 27 us (31; 36), 10,000 plain cells 12.5 us (21; 21).  What is left: about 1.3 us per
-// barrier, the longest tile of each phase (out-of-bank cells with levees, ends of paths), and at full
-// size 16 warps per SM, each at the latency of its tile (128 registers; 24 warps at 80 spill past the
-// little L1 that is left, and gain nothing).
+// channels, levees and dams 38 us (one persistent kernel over global memory 82), 2 x 26,691 cells 20 us (36),
+// 10,000 plain cells 12.1 us (21).  What is left: about 1.3 us per barrier, the longest tile of each phase
+// (out-of-bank cells with levees, ends of paths), and at full size 16 warps per SM, each at the latency of
+// its tile.  A spilled register costs more here than a load of its own: there is little L1 left.
 #pragma once
 #include "cmf_persist.cuh"
 
@@ -34,10 +33,12 @@ enum ResBit : unsigned { B_FLDSTO = 1 << 8, B_FLDSTOPRE = 1 << 9, B_FLDDPH = 1 <
                          B_LEVDPH = 1 << 13, B_AFLDOUT = 1 << 14, B_AOUTFLW = 1 << 15 };
 constexpr int kResMemberShift = 16;
 constexpr unsigned kNoCell = 0xffffu << kResMemberShift;
-#ifndef CMF_RES_THREADS
-#define CMF_RES_THREADS 512
-#endif
-constexpr int kResThreads = CMF_RES_THREADS;
+// Threads of a CTA at most, and so the registers a thread may have: 16 warps of 128 registers, or, while
+// a CTA has no more than kResFewTasks tiles and path tiles, so that a phase is two rounds of warps either
+// way, 12 of 168.  Per sub-step, 16 and 12 warps: 10,000 plain cells 12.7 and 12.1 us, 2 x 26,691 cells
+// 21.1 and 20.4, 2 x 40,000 (22 tasks) 24.1 and 23.1; 2 x 60,000 (33 tasks) 25.8 and 27.0, 298,554 cells
+// 38.2 and 42.7.  Eighteen warps or more spill: 52 us or more at 298,554 cells.
+constexpr int kResThreadsMany = 512, kResThreadsFew = 384, kResFewTasks = 2 * (kResThreadsFew / 32);
 constexpr int kResMaxGroup = 64;                  // members of one group (their NT/DT sit in shared memory)
 // What a cell needs of the network, also on the SM: its index, its downstream cell, its element of the
 // exchange arrays, and its upstream cells' range there (first element, count above kResDegShift).  The
@@ -94,6 +95,7 @@ struct OwnR : OwnMaps {
     __device__ __forceinline__ double rivsto(size_t) const { return get(F_RIVSTO); }
     __device__ __forceinline__ double fldsto(size_t g) const { return sparse(B_FLDSTO, s.fldsto, g); }
     __device__ __forceinline__ double levsto(size_t g) const { return sparse(B_LEVSTO, s.levsto, g); }
+    __device__ __forceinline__ bool flooded() const { return bits & B_FLDSTO; }
     __device__ __forceinline__ double rivdph(size_t) const { return get(F_RIVDPH); }
     __device__ __forceinline__ double rivdph_pre(size_t) const { return get(F_DPHPRE); }
     __device__ __forceinline__ double rivout_pre(size_t) const { return get(F_ROUT); }
@@ -218,7 +220,8 @@ struct OwnR : OwnMaps {
     }
 };
 
-__global__ void __launch_bounds__(kResThreads, 1) k_resident(Net n, State s, ResArgs a) {
+template <int Threads>
+__global__ void __launch_bounds__(Threads, 1) k_resident(Net n, State s, ResArgs a) {
     extern __shared__ double fields[];
     __shared__ int sflag, s_nt[kResMaxGroup], s_ntmax, s_q[3], s_nd, s_dam[kResMaxSlots];
     __shared__ double s_dt[kResMaxGroup], s_bud[kBudgetThreads / 32];
