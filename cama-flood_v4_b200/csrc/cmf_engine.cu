@@ -895,15 +895,11 @@ int d2h(cmf_gpu_ctx *c, T *dst, const T *src, size_t n) {
 // state arrays of the boundary are [M][NSEQMAX]; the device keeps [M][NSEQALL] (== NSEQMAX here)
 // NT, DT, budgets and statuses of the step whose control blocks are in c->hctl
 int process_ctl(cmf_gpu_ctx *c, int32_t *nt_out, double *dt_out, cmf_budget *b) {
-    if (c->persist) {
-        int berr = 0;
-        CUDA_TRY(cudaMemcpyAsync(&berr, &c->st.loop->bar_err, sizeof berr, cudaMemcpyDeviceToHost, c->stream));
+    if (c->hctl[0].bar_err) {       // comes with the control blocks: a read of its own would wait for the steps behind
+        c->hctl[0].bar_err = 0;
+        CUDA_TRY(cudaMemsetAsync(&c->st.ctl[0].bar_err, 0, sizeof(int), c->stream));
         CUDA_TRY(cudaStreamSynchronize(c->stream));
-        if (berr) {
-            CUDA_TRY(cudaMemsetAsync(&c->st.loop->bar_err, 0, sizeof(int), c->stream));
-            CUDA_TRY(cudaStreamSynchronize(c->stream));
-            return set_err(CMF_E_BARRIER, "persistent kernel: a grid barrier did not complete within its bound");
-        }
+        return set_err(CMF_E_BARRIER, "persistent kernel: a grid barrier did not complete within its bound");
     }
     int err = 0;
     int ntmax = 0;
@@ -1296,11 +1292,11 @@ int cmf_gpu_ctx_persist_selftest(cmf_gpu_ctx *c, int64_t wait_ns) {
     int rc = launch_persist(c, (unsigned long long)wait_ns);
     if (rc) return rc;
     int berr = 0;
-    CUDA_TRY(cudaMemcpyAsync(&berr, &c->st.loop->bar_err, sizeof berr, cudaMemcpyDeviceToHost, c->stream));
+    CUDA_TRY(cudaMemcpyAsync(&berr, &c->st.ctl[0].bar_err, sizeof berr, cudaMemcpyDeviceToHost, c->stream));
     CUDA_TRY(cudaStreamSynchronize(c->stream));
     CUDA_TRY(cudaGetLastError());
     if (!berr) return set_err(CMF_E_STATE, "persistent self-test: the barrier completed although it could not");
-    CUDA_TRY(cudaMemsetAsync(&c->st.loop->bar_err, 0, sizeof(int), c->stream));
+    CUDA_TRY(cudaMemsetAsync(&c->st.ctl[0].bar_err, 0, sizeof(int), c->stream));
     CUDA_TRY(cudaStreamSynchronize(c->stream));
     return set_err(CMF_E_BARRIER, "persistent self-test: the grid barrier ran out its bound and the kernel returned");
 }

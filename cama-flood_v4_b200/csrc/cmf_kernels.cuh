@@ -62,7 +62,7 @@ struct MemberCtl {
     int nt;                        // sub-steps of this outer step
     int it;                        // index of the next sub-step
     int err;
-    int pad;
+    int bar_err;                   // member 0: a bounded wait of the persistent kernel ran out
     double budget[kBudgets];       // last finished sub-step
 };
 
@@ -81,7 +81,6 @@ struct LoopCtl {
                                  // 1e-12 (relative) of an integer: NT there hangs on DT_MIN's last bits
     long long nt_hist[kNtHist];  // (outer step, member) pairs by NT
     unsigned bar;                // grid-barrier arrival count of the persistent kernel (zeroed per launch)
-    int bar_err;                 // set when a bounded wait of the persistent kernel ran out
 };
 
 // Static data shared by all members (device pointers).

@@ -11,7 +11,7 @@
 // (cmf_kernels.cuh, global-memory accessor), so the results are identical bit for bit.
 //
 // Barriers spin on a counter in global memory with a bound: a CTA that waits longer than the bound
-// sets LoopCtl.bar_err and every CTA leaves the kernel at its next barrier, so a wait that cannot end
+// sets MemberCtl.bar_err of member 0 and every CTA leaves the kernel at its next barrier, so a wait that cannot end
 // returns an error status to the host instead of holding the GPU.
 #pragma once
 #include "cmf_kernels.cuh"
@@ -161,7 +161,7 @@ __global__ void __launch_bounds__(kTile, kPersistMinBlocks) k_persist(Net n, Sta
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ int sflag;
     const unsigned G = gridDim.x, b = blockIdx.x;
-    GridBar gb{&s.loop->bar, &s.loop->bar_err, G, 0u, pa.wait_ns, &sflag};
+    GridBar gb{&s.loop->bar, &s.ctl[0].bar_err, G, 0u, pa.wait_ns, &sflag};
     if (pa.selftest) {
         // barrier timeout check: the count target includes one arrival that never comes
         gb.nblocks = G + 1;

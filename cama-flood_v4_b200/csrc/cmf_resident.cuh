@@ -228,7 +228,7 @@ __global__ void __launch_bounds__(Threads, 1) k_resident(Net n, State s, ResArgs
     __shared__ unsigned long long s_min[kResMaxGroup];
     const unsigned G = gridDim.x, b = blockIdx.x;
     const int tid = threadIdx.x, nw = blockDim.x >> 5, warp = tid >> 5, lane = tid & 31;
-    GridBar gb{&s.loop->bar, &s.loop->bar_err, G, 0u, a.wait_ns, &sflag};
+    GridBar gb{&s.loop->bar, &s.ctl[0].bar_err, G, 0u, a.wait_ns, &sflag};
     if (a.selftest) {           // the count target includes one arrival that never comes
         gb.nblocks = G + 1;
         gb.sync();
