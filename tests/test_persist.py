@@ -10,6 +10,7 @@ import numpy as np
 import pytest
 
 from conftest import rel_close, runoff_series
+from cmf_b200 import synth
 
 pytestmark = pytest.mark.gpu
 
@@ -63,6 +64,43 @@ def test_persistent_equals_graph_bit_for_bit(case_dirs, name, members, nsteps):
     for f in DIAG_KEYS:
         assert _same(ga[f], gb[f]), f
     assert a.kernel_launches < b.kernel_launches
+
+
+# (scale of the config-1 grid, members, path levels): a net of a few cells in its last tile, more members
+# than a group holds, paths of more levels than a warp has lanes, 23 tasks per SM (the form with more
+# registers) and 25 (the other), two groups of a large member, and a member that does not
+# fit the SMs (the kernel over global memory)
+@pytest.mark.parametrize("scale,members,levels", [(0.012, 1, 5), (0.012, 70, 33), (0.05, 1, 64), (0.1, 29, 5), (0.1, 30, 5),
+                                                  (0.6, 4, 3), (1.05, 1, 5)])
+def test_resident_edges_equal_graph_bit_for_bit(tmp_path, scale, members, levels):
+    """Three flooded steps of nets at the edges of the resident kernel's tiles, groups and register forms
+    leave the same bits as the graph of phase kernels."""
+    from cmf_b200 import HostModel, PhysicsGPU
+
+    spec = synth.spec_config1(seed=3, scale=scale)
+    spec.npthlev = levels
+    spec.rivhgt_scale = 0.3
+    synth.write_case(synth.make_case(spec), str(tmp_path / "c"))
+    h = HostModel(str(tmp_path / "c"))
+    series = np.stack(list(runoff_series(h.map("grarea"), "stress", 3, hourly=True)))
+    weight = np.random.default_rng(2).uniform(0.5, 2.0, (members, 1))
+    a = PhysicsGPU(h, nmembers=members, launch_mode=2, ldiag_output=True)
+    b = PhysicsGPU(h, nmembers=members, launch_mode=0, block_size=256, ldiag_output=True)
+    for r in series:
+        steps = []
+        for g in (a, b):
+            g.put_runoff(weight * r)
+            steps.append(g.advance())
+        (na, da, ba), (nb, db, bb) = steps
+        assert np.array_equal(na, nb) and _same(da, db)
+        for m in range(members):
+            assert all(_same(np.float64(v), np.float64(bb[m][f])) for f, v in ba[m].items()), m
+    sa, sb = a.get_state(), b.get_state()
+    ga, gb = a.get_diag(), b.get_diag()
+    for f in STATE_KEYS:
+        assert _same(sa[f], sb[f]), f
+    for f in DIAG_KEYS:
+        assert _same(ga[f], gb[f]), f
 
 
 def test_persistent_vs_oracle(case_dirs):
