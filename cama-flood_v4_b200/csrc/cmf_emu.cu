@@ -345,25 +345,36 @@ struct EmuNet {
 };
 
 
-// hop-0 inputs: last-step mean outflow and runoff of every member, as fp32 planes
-__global__ void k_emu_seed(EmuNet n, const double *__restrict__ qprev, const double *__restrict__ runoff, float *pa, float *pb) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n.N) return;
-    const size_t gi = (size_t)blockIdx.y * n.N + i;
-    pa[gi] = (float)qprev[gi];
-    pb[gi] = (float)runoff[gi];
-}
-
-// one hop of upstream message passing: out[i] = sum over upstream j of in[j], ascending upstream order
-__global__ void k_emu_hop(EmuNet n, const float *__restrict__ in_a, const float *__restrict__ in_b, float *out_a, float *out_b) {
+// one hop of upstream message passing: out[i] = sum over upstream j of in[j], ascending upstream order.  The
+// first hop reads the fp64 last-step outflow and runoff (rounded to fp32), the later ones the hop before's
+// planes.  Bound by its gathers through L1, so a hop of its own: two hops in one pass gather a cell's second
+// ring anew, through two more index loads, for a third less memory traffic.  Two upstream cells are in flight
+// at a time.  Eight hops and the assembly for 32 x 299k cells: 1215 us with two hops a pass, 1081 us with one.
+template <bool FromState>
+__global__ void __launch_bounds__(256) k_emu_hop(EmuNet n, const float *__restrict__ in_a, const float *__restrict__ in_b,
+                                                 const double *__restrict__ qa, const double *__restrict__ qb, float *out_a,
+                                                 float *out_b) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n.N) return;
     const size_t mo = (size_t)blockIdx.y * n.N;
+    auto va = [&](int j) { return FromState ? (float)qa[mo + j] : in_a[mo + j]; };
+    auto vb = [&](int j) { return FromState ? (float)qb[mo + j] : in_b[mo + j]; };
     float a = 0.f, b = 0.f;
-    for (int k = n.up_ptr[i]; k < n.up_ptr[i + 1]; k++) {
-        const int j = n.up_idx[k];
-        a += in_a[mo + j];
-        b += in_b[mo + j];
+    const int k1 = n.up_ptr[i + 1];
+    for (int k = n.up_ptr[i]; k < k1; k += 2) {
+        const int j0 = n.up_idx[k], j1 = k + 1 < k1 ? n.up_idx[k + 1] : -1;
+        const float a0 = va(j0), b0 = vb(j0);
+        float a1 = 0.f, b1 = 0.f;
+        if (j1 >= 0) {
+            a1 = va(j1);
+            b1 = vb(j1);
+        }
+        a += a0;
+        b += b0;
+        if (j1 >= 0) {
+            a += a1;
+            b += b1;
+        }
     }
     out_a[mo + i] = a;
     out_b[mo + i] = b;
@@ -379,39 +390,6 @@ __device__ __forceinline__ float fslog(float x) {
     return copysignf(a < 1e-3f ? a * (1.f - 0.5f * a) : __logf(1.f + a), x);
 }
 
-// two hops in one pass: out1[i] = sum over upstream j of in[j]; out2[i] = sum over upstream j of
-// (sum over upstream k of j of in[k]) -- the same fp32 sums, in the same ascending order, as two
-// single-hop passes.  The first pair reads the fp64 last-step outflow and runoff directly (the
-// single-hop chain converts them to fp32 planes first: the same values).
-template <bool FromState>
-__global__ void k_emu_hop2(EmuNet n, const float *__restrict__ in_a, const float *__restrict__ in_b,
-                           const double *__restrict__ qa, const double *__restrict__ qb, float *o1a, float *o1b,
-                           float *o2a, float *o2b) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n.N) return;
-    const size_t mo = (size_t)blockIdx.y * n.N;
-    auto va = [&](int j) { return FromState ? (float)qa[mo + j] : in_a[mo + j]; };
-    auto vb = [&](int j) { return FromState ? (float)qb[mo + j] : in_b[mo + j]; };
-    float a1 = 0.f, b1 = 0.f, a2 = 0.f, b2 = 0.f;
-    for (int k = n.up_ptr[i]; k < n.up_ptr[i + 1]; k++) {
-        const int j = n.up_idx[k];
-        a1 += va(j);
-        b1 += vb(j);
-        float sa = 0.f, sb = 0.f;
-        for (int q = n.up_ptr[j]; q < n.up_ptr[j + 1]; q++) {
-            const int g = n.up_idx[q];
-            sa += va(g);
-            sb += vb(g);
-        }
-        a2 += sa;
-        b2 += sb;
-    }
-    o1a[mo + i] = a1;
-    o1b[mo + i] = b1;
-    o2a[mo + i] = a2;
-    o2b[mo + i] = b2;
-}
-
 // Manning discharge of a rectangular section of area A, hydraulic depth h and friction slope s
 __device__ __forceinline__ float manning_q(float area, float h, float s, float inv_man) {
     if (!(area > 0.f) || !(h > 0.f)) return 0.f;
@@ -420,9 +398,9 @@ __device__ __forceinline__ float manning_q(float area, float h, float s, float i
 
 // Bound by the latency of its 35 loads a cell, so six blocks per SM are asked for (54 registers and four
 // blocks without it); a row leaves through shared memory, four lanes writing its 64 bytes together, where a
-// lane per row wrote half a sector at a time.  32 x 299k cells, the hop pairs included: 1337 us as one row a
-// lane, 1313 us through shared memory, 1218 us with six blocks (seven: 1262 us).
-// features of cell i of member blockIdx.y; planes [2*(hops+1)][M*N] (0,1 = seeds; 2h+2, 2h+3 = hop h)
+// lane per row wrote half a sector at a time.  32 x 299k cells, four passes of two hops included: 1337 us as
+// one row a lane, 1313 us through shared memory, 1218 us with six blocks (seven: 1262 us).
+// features of cell i of member blockIdx.y; planes [2*(hops+1)][M*N] (0, 1 unused; 2h+2, 2h+3 = hop h)
 __global__ void __launch_bounds__(256, 6) k_emu_assemble(EmuNet n, const double *__restrict__ rivsto, const double *__restrict__ fldsto,
                                const double *__restrict__ levsto, const double *__restrict__ rivdph,
                                const double *__restrict__ flddph, const double *__restrict__ fldfrc,
@@ -1681,19 +1659,9 @@ int cmf_emu_features(const cmf_emu_net *net, const cmf_emu_member *mb, int nmemb
     const dim3 blocks((n.N + 255) / 256, nmembers);
     const size_t plane = (size_t)nmembers * n.N;
     auto pl = [&](int k) { return planes + (size_t)k * plane; };   // hop h: planes 2h+2 (outflow), 2h+3 (runoff)
-    int h = 0;
-    if (hops >= 2) {
-        k_emu_hop2<true><<<blocks, 256, 0, st>>>(n, nullptr, nullptr, mb->qprev, mb->runoff, pl(2), pl(3), pl(4), pl(5));
-        h = 2;
-    } else if (hops == 1) {
-        k_emu_seed<<<blocks, 256, 0, st>>>(n, mb->qprev, mb->runoff, pl(0), pl(1));
-        k_emu_hop<<<blocks, 256, 0, st>>>(n, pl(0), pl(1), pl(2), pl(3));
-        h = 1;
-    }
-    for (; h + 2 <= hops; h += 2)
-        k_emu_hop2<false><<<blocks, 256, 0, st>>>(n, pl(2 * h), pl(2 * h + 1), nullptr, nullptr, pl(2 * h + 2),
-                                                  pl(2 * h + 3), pl(2 * h + 4), pl(2 * h + 5));
-    if (h < hops) k_emu_hop<<<blocks, 256, 0, st>>>(n, pl(2 * h), pl(2 * h + 1), pl(2 * h + 2), pl(2 * h + 3));
+    if (hops >= 1) k_emu_hop<true><<<blocks, 256, 0, st>>>(n, nullptr, nullptr, mb->qprev, mb->runoff, pl(2), pl(3));
+    for (int h = 1; h < hops; h++)
+        k_emu_hop<false><<<blocks, 256, 0, st>>>(n, pl(2 * h), pl(2 * h + 1), nullptr, nullptr, pl(2 * h + 2), pl(2 * h + 3));
     k_emu_assemble<<<blocks, 256, 0, st>>>(n, mb->rivsto, mb->fldsto, mb->levsto, mb->rivdph, mb->flddph, mb->fldfrc,
                                            mb->qprev, mb->runoff, planes, plane, hops, (__nv_bfloat16 *)X, ldx,
                                            rows_per_member);
