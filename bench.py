@@ -221,8 +221,9 @@ def phase_bytes(N: int, E: int, L_bar: float, P: int, Lp: int, nlev: int, ndam: 
                (the last sub-step's own accumulators, once per outer step, are not counted)
                + levee: index 4/cell + 7 params + LEVSTO r/w + LEVDPH w per levee cell
                + dams: 112 B per dam, paths: FLW r/w 16 x Lp + FLWSUM 16 per path
-    k_store walks the upstream lists through a 4-slot table (16 B per cell, one dependent load
-    fewer); the count keeps the CSR's compulsory bytes, so the fraction it gives is conservative."""
+    This is the pass of a network with water on every floodplain: the kernels skip, cell by cell, the
+    arrays that hold zero there (floodplain and levee state, D2FLDOUT's averages), and exchange
+    outflows and depths as 16-byte pairs.  The count stays the same so that the fractions compare."""
     flux = N * (140 + (128 if ldiag else 0)) + P * (8 + 8 + 4 + 32 * Lp + 8) + ndam * 112
     rate = N * 48 + (E - N) * 4 + P * 2 * (8 + 8)
     store = N * (188 + 16 * L_bar) + N * 4 + nlev * (7 * 8 + 16 + 8) + ndam * 112 + P * (16 * Lp + 16)
@@ -487,7 +488,7 @@ def gpu_arm(args) -> int:
                         "l2": "256 MiB buffer written before every timed step", "nt_mean": member_sub / max(K * M, 1),
                         "nt_histogram": nthist, "nt_near_integer_steps": int(s1["near_boundary"] - s0["near_boundary"]),
                         "schedule": sched,
-                        "launch": ("one CUDA graph per coupling step, device-side sub-step loop" if args.launch_mode == 0
+                        "launch": ("one launch per coupling step (see schedule), device-side sub-step loop" if args.launch_mode == 0
                                    else "host-driven kernel launches")},
             "e2e": {"value": e2e_value, "unit": UNIT, "h2d_bytes_per_step": M * N * 8,
                     "d2h_bytes_per_step": M * N * 8 + M * 160,
@@ -851,7 +852,7 @@ def cfg4_arm(args) -> int:
                                f"levees 10%, {h.dims.ndam} dams, {Mmax} members, hourly AR(1) forcing",
                    "members": Mmax, "nt_mean": top["nt_mean"], "L_bar": Lbar, "case_generation_s": round(t_gen, 1),
                    "l2": "working set far above L2 (no flush needed)",
-                   "launch": "one CUDA graph per coupling step, device-side sub-step loop"},
+                   "launch": "one launch per coupling step (see schedule), device-side sub-step loop"},
         "roofline": {"bound": "hbm", "achieved": top["kst"], "peak": peaks["hbm_gbs"], "unit": "GB/s",
                      "frac": top["kst"] / peaks["hbm_gbs"], "traffic": None, "kernel": "k_store",
                      "peak_source": peaks["source"] + " (hbm_gbs, burst copy)",

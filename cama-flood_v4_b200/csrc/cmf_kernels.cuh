@@ -1350,7 +1350,7 @@ __device__ __forceinline__ void cell_store(const Net &n, const State &s, Own &w,
         s.outflw[gi] = outflw;
     }
     // CMF_DIAG_AVEMAX_ADPSTP / GETAVE_ADPSTP, src/cmf_calc_diag_mod.F90:104-221.  The sub-steps
-    // before the last one are accumulated by the next sub-step's phase A (diag_carry_store), except
+    // before the last one are accumulated by the next sub-step's phase A (diag_carry), except
     // D2PTHOUT_aAVG: D2PTHINF is never written by the reference (always 0), and a cell without
     // bifurcation channels adds +0 every sub-step, so its average (and output average) stays at the
     // +0 the arrays were created with; cells with channels accumulate it here every sub-step.

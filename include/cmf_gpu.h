@@ -81,7 +81,8 @@ typedef struct cmf_opts {
     int32_t launch_mode; /* 0: one CUDA graph per coupling step with a device-side sub-step loop;
                             1: host-driven launches (reads NT back before the sub-steps);
                             2: one persistent cooperative kernel per coupling step (grid barriers
-                               between the phases, cell tiles interleaved over the CTAs)          */
+                               between the phases, cell tiles interleaved over the CTAs, the state
+                               of members that fit the SMs held there through the sub-steps)      */
     int32_t device;      /* CUDA device ordinal                                                   */
     int32_t block_size;  /* 0: the online autotuner picks the schedule (launch_mode 0); else
                             threads per block of the phase kernels (64..256)                     */
