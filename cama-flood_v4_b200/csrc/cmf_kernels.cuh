@@ -206,6 +206,19 @@ struct OwnMaps {
     __device__ __forceinline__ int i1dam(int i) const { return __ldg(&n.i1dam[i]); }
 };
 struct LazyRate;
+// What phase B leaves of an outflow: a positive one (and a mouth's) is rescaled by its own cell's rate here, and
+// its gatherer takes the product; a reverse one keeps its value (not > 0) and is multiplied by the gatherer's
+// rate.  Where the own rate takes a positive outflow to zero or below it (the rate of an overdrawn cell, which
+// net runoff below zero makes, is negative) the product would pass for a reverse flow: NaN stands there, and
+// whose sums come out NaN takes them again from the pairs before the rescale, by their signs (each_by_sign).
+__device__ __forceinline__ double2 rescale_own(double rout, double fout, double r, bool mouth) {
+    if (rout > 0.0 || mouth) {
+        rout = rout * r;
+        fout = fout * r;
+        if (!(rout > 0.0) && !mouth) rout = __longlong_as_double(0x7ff8000000000000ll);
+    }
+    return make_double2(rout, fout);
+}
 struct DownCell {
     double rivelv, rivdph, rivdph_pre;
 };
@@ -236,15 +249,9 @@ struct OwnG : OwnMaps {
         return {__ldg(&n.next_rivelv[i]), d.x, d.y};
     }
     __device__ __forceinline__ void put_raw(size_t g, int, double rout, double fout) const { s.raw[g] = make_double2(rout, fout); }
-    // a positive outflow (and a mouth's) is rescaled by its own cell's rate here, and its gatherer takes
-    // the product; a reverse one keeps its value (not > 0) and is multiplied by the gatherer's rate
     __device__ __forceinline__ void put_rate(size_t g, int i, double rout, double fout, double r) const {
         s.rate[g] = r;
-        if (rout > 0.0 || i >= n.R) {
-            rout = rout * r;
-            fout = fout * r;
-        }
-        s.out[g] = make_double2(rout, fout);
+        s.out[g] = rescale_own(rout, fout, r, i >= n.R);
     }
     __device__ __forceinline__ void put_a_rivvel(size_t g, double v) const { s.a_rivvel[g] = v; }
     // an array that holds +0 while `bit` is clear
@@ -293,6 +300,9 @@ struct OwnG : OwnMaps {
     // f(rivout, fldout) after the rescale (:481-489); next(j) == i, so a reverse flow takes rate_i
     template <class Rate, class F>
     __device__ __forceinline__ void each_out(size_t base, int i, Rate rate_i, F f) const;
+    // the same from the pairs before the rescale (see rescale_own)
+    template <class F>
+    __device__ __forceinline__ void each_by_sign(size_t base, int i, double rate_i, F f) const;
 };
 // the cell's rate, read only where a reverse flow or a path needs it
 struct LazyRate {
@@ -344,6 +354,19 @@ __device__ __forceinline__ void rescaled(double2 v, Rate rate_i, F f) {
 template <class Rate, class F>
 __device__ __forceinline__ void OwnG::each_out(size_t base, int i, Rate rate_i, F f) const {
     for_each_upstream(n, *this, i, [&](int j) { rescaled(s.out[base + j], rate_i, f); });
+}
+// f(rivout, fldout) of one flow by the rate its sign before the rescale names: its own cell's or the gatherer's
+template <class F>
+__device__ __forceinline__ void by_sign(double2 raw, double own, double below, F f) {
+    const double r = raw.x > 0.0 ? own : below;
+    f(raw.x * r, raw.y * r);
+}
+template <class F>
+__device__ __forceinline__ void OwnG::each_by_sign(size_t base, int i, double rate_i, F f) const {
+    for (int k = up_lo(i); k < up_hi(i); k++) {
+        const size_t g = base + __ldg(&n.up_idx[k]);
+        by_sign(s.raw[g], s.rate[g], rate_i, f);
+    }
 }
 
 
@@ -1295,6 +1318,18 @@ __device__ __forceinline__ void cell_store(const Net &n, const State &s, Own &w,
         rinf = rinf + rj;
         finf = finf + fj;
     });
+    if (rout != rout || rinf != rinf) {            // see rescale_own
+        if (i < n.R && rout != rout)
+            by_sign(s.raw[gi], rate_i, w.nb(rate_m, w.next(i)), [&](double r, double f) {
+                rout = r;
+                fout = f;
+            });
+        rinf = finf = 0.0;
+        w.each_by_sign(base, i, rate_i, [&](double rj, double fj) {
+            rinf = rinf + rj;
+            finf = finf + fj;
+        });
+    }
     double pout = 0.0;
     const bool has_path = w.flags() & C_PATH;
     if (has_path) {

@@ -137,17 +137,13 @@ struct OwnR : OwnMaps {
         }
         if (x >= 0) raw[x] = make_double2(rout, fout);
     }
-    // a positive outflow (and a mouth's) is rescaled by its own cell's rate here, and its gatherer takes
-    // the product; a reverse one keeps its value (not > 0) and is multiplied by the gatherer's rate
     __device__ __forceinline__ void put_rate(size_t g, int i, double rout, double fout, double r) const {
         s.rate[g] = r;
-        if (rout > 0.0 || i >= n.R) {
-            rout = rout * r;
-            fout = fout * r;
-        }
-        put(F_ROUT, rout);
-        put(F_FOUT, fout);
-        if (x >= 0) out[x] = make_double2(rout, fout);
+        const double2 v = rescale_own(rout, fout, r, i >= n.R);
+        if (v.x != v.x) s.raw[g] = make_double2(rout, fout);       // for this cell's phase C
+        put(F_ROUT, v.x);
+        put(F_FOUT, v.y);
+        if (x >= 0) out[x] = v;
     }
     __device__ __forceinline__ void put_a_rivvel(size_t, double v) const { put(F_ARIVVEL, v); }
     __device__ __forceinline__ void put_pre(size_t g, double rout, double fout, double dph, double fld, bool) const {
@@ -197,6 +193,11 @@ struct OwnR : OwnMaps {
     template <class Rate, class F>
     __device__ __forceinline__ void each_out(size_t, int, Rate rate_i, F fn) const {
         each_pair(out, [&](double rj, double fj) { rescaled(make_double2(rj, fj), rate_i, fn); });
+    }
+    template <class F>
+    __device__ __forceinline__ void each_by_sign(size_t base, int, double rate_i, F fn) const {
+        const int first = up & ((1 << kResDegShift) - 1), end = first + (int)((unsigned)up >> kResDegShift);
+        for (int e = first; e < end; e++) by_sign(__ldcg(raw + e), __ldcg(s.rate + base + __ldg(&n.up_idx[e])), rate_i, fn);
     }
     // the previous sub-step's averages and maxima (diag_carry with the sums held on the SM)
     __device__ __forceinline__ void carry(size_t g, double DT, bool first, double rout, double fout, double dph, double sto) const {

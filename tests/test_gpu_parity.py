@@ -109,6 +109,64 @@ def test_parity_resynced_each_step(case_dirs, name, nsteps):
     print(f"{name}: worst per-step relative deviation {worst_seen:.3e}")
 
 
+def _oracle_view(o, name):
+    """The oracle's own array (a step from a state made by hand)."""
+    import ctypes as C
+
+    n = C.c_int(0)
+    return np.ctypeslib.as_array(o.lib.orc_darray(o.h, name.encode(), C.byref(n)), shape=(n.value,))
+
+
+@pytest.mark.parametrize("mode", [0, 2])
+@pytest.mark.parametrize("name,seeds", [("cfg0", 2), ("cfg1s", 6), ("stress", 6)])
+def test_overdrawn_cells_take_one_rate(case_dirs, name, seeds, mode):
+    """Net runoff below zero overdraws cells, so their storage and LSPAMAT rate turn negative and the
+    storage limiter turns reverse flows positive: every outflow is still rescaled by one rate, chosen by
+    the sign it had before the rescale (src/cmf_calc_outflw_mod.F90:456-489), also where the rate of the
+    cell below is less than 1.  One step from such a state, graph of phase kernels and persistent kernel."""
+    h, g, o = _models(case_dirs[name], launch_mode=mode, **({} if mode else {"block_size": 128}))
+    area, nxt = h.map("grarea"), h.map("i1next") - 1
+    river = np.flatnonzero(nxt >= 0)
+    series = list(runoff_series(area, name, 8, hourly=True))
+    for r in series:
+        o.put_runoff(r)
+        o.advance()
+    start = {f: o.d(f) for f in ORACLE_STATE if o.d(f).size == g._state_sizes(f)}
+    seen = [0]
+
+    def count(_it):
+        rate = _oracle_view(o, "rate")
+        own = (rate[river] < 0.0) & (_oracle_view(o, "rivout")[river] != 0.0)
+        seen[0] += int((own & (rate[nxt[river]] != 1.0)).sum())
+
+    o.on_substep(count)
+    for seed in range(seeds):
+        rng = np.random.default_rng(seed)
+        st = {f: v.copy() for f, v in start.items()}
+        empty = rng.random(nxt.size) < 0.3
+        st["rivsto"][empty] *= -1e-3
+        # what flowed last would empty the other cells several times over
+        st["rivout_pre"] = np.where(empty, st["rivout_pre"], rng.uniform(2, 40, nxt.size) * np.maximum(st["rivsto"], 1.0) / 3600.0)
+        st["rivout"] = st["rivout_pre"].copy()
+        r = np.where(rng.random(nxt.size) < 0.3, -1e-3 * area / 3600.0, series[0])
+        for f, v in st.items():
+            _oracle_view(o, f)[:] = v
+        g.set_state(st)
+        o.put_runoff(r)
+        g.put_runoff(r)
+        nt_o, dt_o = o.advance()
+        nt_g, dt_g, _ = g.advance()
+        assert nt_g[0] == nt_o and dt_g[0] == dt_o, f"seed {seed}"
+        out = g.get_state()
+        for f in ("rivsto", "fldsto", "rivout", "fldout", "levsto", "damsto", "pthflw"):
+            if f not in st:
+                continue
+            ok, worst, bad = rel_close(out[f][0], o.d(f), RTOL)
+            assert ok, f"seed {seed} {f}: worst {worst:.3e}, {bad} cells above {RTOL}"
+    o.on_substep(None)
+    assert seen[0], "no outflow of an overdrawn cell met a rate-limited cell below"
+
+
 def test_graph_and_stream_launch_bit_identical(case_dirs):
     """The device-side conditional loop and the host-driven loop produce identical bits."""
     from cmf_b200 import HostModel, PhysicsGPU
