@@ -399,13 +399,16 @@ int build_net(cmf_gpu_ctx *c, const cmf_map_ptrs *mp) {
         std::vector<unsigned char> fl(N, 0);
         std::vector<int> dams, rules, order, pos(N, -1), dup_ptr, dup_idx;
         std::vector<double> vel, velf;
+        for (int p = 0; p < n.P; p++)
+            for (int e : {h_pu[p], h_pd[p]})
+                if (e >= 0) fl[e] |= cmf::C_END;
         for (int i = 0; i < N; i++) {
             unsigned f = 0;
             if (h_i1dam[i] > 0) f |= cmf::C_DAM | (h_i1dam[i] == 10 && i < R ? cmf::C_KIN : 0);
             if (h_dam_id[i] >= 0) f |= cmf::C_DAMID;
             if (h_po_ptr[i + 1] > h_po_ptr[i] || h_pi_ptr[i + 1] > h_pi_ptr[i]) f |= cmf::C_PATH;
             if (h_lev_id[i] >= 0) f |= cmf::C_LEV;
-            fl[i] = (unsigned char)f;
+            fl[i] |= (unsigned char)f;
             if (f & cmf::C_DAM) (f & cmf::C_KIN ? dams : rules).push_back(i);
         }
         dams.insert(dams.end(), rules.begin(), rules.end());

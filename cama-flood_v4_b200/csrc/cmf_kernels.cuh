@@ -142,8 +142,9 @@ enum CellFlag : unsigned {
     C_DAM = 1,                 // I1DAM > 0: outflow by cell_dam
     C_KIN = 2,                 // I1DAM == 10 on a river cell: kinematic outflow upstream of a dam
     C_DAMID = 4,               // a dam's storage stands here
-    C_PATH = 8,                // an end of a bifurcation path
-    C_LEV = 16                 // levee parameters
+    C_PATH = 8,                // paths in the cell's lists (I1P_OUT, I1P_INF)
+    C_LEV = 16,                // levee parameters
+    C_END = 32                 // an end of a path (PTH_UPST, PTH_DOWN): the path reads its storage and depths
 };
 
 // What the phase kernels keep per cell beside the arrays (State::wet): which of the arrays that are zero
@@ -285,7 +286,7 @@ struct OwnG : OwnMaps {
         }
         wet = some ? wet | W_STAGE : wet & ~W_STAGE;
         if (last) s.rivdph[g] = o.rivdph;
-        if (last || (fl & C_PATH)) s.storge[g] = storge;      // read by the paths at this cell
+        if (last || (fl & C_END)) s.storge[g] = storge;      // read by the paths at this cell
     }
     // f(rivout, fldout) before the LSPAMAT rescale of every upstream cell, in I1UPST order: the CSR
     // walk, since at k_rate's full occupancy the slot table's 16 B per cell cost more than its saved round

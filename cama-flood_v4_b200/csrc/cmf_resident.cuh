@@ -155,7 +155,7 @@ struct OwnR : OwnMaps {
             s.rivout_pre[g] = rout;
             s.fldout_pre[g] = fout;
         }
-        if (bits & C_PATH) s.rivdph_pre[g] = dph;
+        if (bits & C_END) s.rivdph_pre[g] = dph;
     }
     template <class Out>
     __device__ __forceinline__ void put_stage(size_t g, const Out &o, double sto, double, bool) const {
@@ -169,7 +169,7 @@ struct OwnR : OwnMaps {
             put_sparse(B_LEVSTO, s.levsto, g, o.levsto);
             put_sparse(B_LEVDPH, s.levdph, g, o.levdph);
         }
-        if (bits & C_PATH) {     // read by the paths at this cell
+        if (bits & C_END) {      // read by the paths at this cell
             s.storge[g] = sto;
             if (n.llevee) s.levdph[g] = o.levdph;
         }

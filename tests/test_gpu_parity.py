@@ -167,6 +167,43 @@ def test_overdrawn_cells_take_one_rate(case_dirs, name, seeds, mode):
     assert seen[0], "no outflow of an overdrawn cell met a rate-limited cell below"
 
 
+@pytest.mark.parametrize("mode", [0, 2])
+def test_paths_missing_from_their_cells_lists(case_dirs, mode):
+    """The boundary takes the paths' ends (PTH_UPST, PTH_DOWN) and the cells' lists of paths beside each
+    other: where a cell's list is empty its paths still flow by the storage, depths and levee depth of
+    every sub-step (src/cmf_ctrl_levee_mod.F90:508-601).  Per-step parity from the oracle's state."""
+    import ctypes as C
+
+    from cmf_b200 import HostModel, PhysicsGPU
+    from oracle import Oracle
+
+    h = HostModel(case_dirs["stress"])
+    o = Oracle(case_dirs["stress"])
+    drop = h.i1seqx % 2 == 0
+    for name in ("i1p_outn", "i1p_infn"):
+        n = C.c_int(0)
+        mine = np.ctypeslib.as_array(getattr(h.maps, name), shape=(h.dims.nseqall,))
+        theirs = np.ctypeslib.as_array(o.lib.orc_iarray(o.h, name.encode(), C.byref(n)), shape=(n.value,))
+        assert np.array_equal(mine, theirs) and np.any(mine[drop])
+        mine[drop] = 0
+        theirs[drop] = 0
+    g = PhysicsGPU(h, launch_mode=mode, **({} if mode else {"block_size": 128}))
+    flowed = 0.0
+    for k, r in enumerate(runoff_series(h.map("grarea"), "stress", 30)):
+        g.set_state({f: o.d(f) for f in ORACLE_STATE if o.d(f).size == g._state_sizes(f)})
+        o.put_runoff(r)
+        g.put_runoff(r)
+        nt_o, dt_o = o.advance()
+        nt_g, dt_g, _ = g.advance()
+        assert nt_g[0] == nt_o and dt_g[0] == dt_o, f"step {k}"
+        st = g.get_state()
+        for f in ("pthflw", "rivsto", "fldsto", "rivout", "fldout", "levsto", "damsto"):
+            ok, worst, bad = rel_close(st[f][0], o.d(f), RTOL)
+            assert ok, f"step {k} {f}: worst {worst:.3e}, {bad} above {RTOL}"
+        flowed += float(np.abs(o.d("pthflw")).sum())
+    assert flowed > 0.0
+
+
 def test_graph_and_stream_launch_bit_identical(case_dirs):
     """The device-side conditional loop and the host-driven loop produce identical bits."""
     from cmf_b200 import HostModel, PhysicsGPU
