@@ -398,6 +398,11 @@ class PhysicsGPU:
         """Status of the persistent kernel's bounded-wait check (CMF_E_BARRIER = 5 when it works)."""
         return int(self.lib.cmf_gpu_ctx_persist_selftest(self.h, int(wait_ns)))
 
+    def persist_selftest_step(self, wait_ns: int = 2_000_000, dt_def: float | None = None) -> None:
+        """Launches an outer step that gives up at its first grid barrier; last_nt() or the next step raises."""
+        dt_def = self.host.dt if dt_def is None else dt_def
+        check(self.lib.cmf_gpu_ctx_persist_selftest_step(self.h, dt_def, int(wait_ns)), "persist_selftest_step")
+
     def diag_len(self, name: str) -> int:
         """Elements of the named diagnostic over all members (the host array's size)."""
         MP = self.M * max(self.P, 1)

@@ -729,13 +729,13 @@ int persist_setup(cmf_gpu_ctx *c) {
     return CMF_OK;
 }
 
-// one outer step as one cooperative launch; wait_ns > 0: the bounded-wait self-test instead
-int launch_persist(cmf_gpu_ctx *c, unsigned long long selftest_ns = 0) {
+// one outer step as one cooperative launch; `selftest` (ResArgs): with waits of selftest_ns that cannot end
+int launch_persist(cmf_gpu_ctx *c, int selftest = 0, unsigned long long selftest_ns = 0) {
     if (c->persist_grid < 1) return set_err(CMF_E_UNSUPPORTED, "the persistent kernel cannot be co-resident on this device");
     CUDA_TRY(cudaMemsetAsync(&c->st.loop->bar, 0, sizeof(unsigned), c->stream));
     if (c->res.group > 0) {
         cmf::ResArgs a = c->res;
-        if (selftest_ns) { a.wait_ns = selftest_ns; a.selftest = 1; }
+        if (selftest) { a.wait_ns = selftest_ns; a.selftest = selftest; }
         void *args[] = {&c->net, &c->st, &a};
         CUDA_TRY(cudaLaunchCooperativeKernel((const void *)c->res_kernel, dim3(c->persist_grid), dim3(c->res_threads), args,
                                              cmf::res_smem(a.slots), c->stream));
@@ -743,8 +743,8 @@ int launch_persist(cmf_gpu_ctx *c, unsigned long long selftest_ns = 0) {
         cmf::PersistArgs a{};
         a.tpm = (c->dims.nseqall + cmf::kTile - 1) / cmf::kTile;
         a.ppm = (cmf::path_threads(c->net.P, c->net.Lp) + cmf::kTile - 1) / cmf::kTile;
-        a.wait_ns = selftest_ns ? selftest_ns : cmf::kWaitNsDefault;
-        a.selftest = selftest_ns != 0;
+        a.wait_ns = selftest ? selftest_ns : cmf::kWaitNsDefault;
+        a.selftest = selftest;
         void *args[] = {&c->net, &c->st, &a};
         CUDA_TRY(cudaLaunchCooperativeKernel((const void *)cmf::k_persist, dim3(c->persist_grid), dim3(cmf::kTile), args,
                                              cmf::kPersistSmem, c->stream));
@@ -895,15 +895,27 @@ int d2h(cmf_gpu_ctx *c, T *dst, const T *src, size_t n) {
     return CMF_OK;
 }
 
+// A grid barrier of a step ran out its bound (the word comes with the control blocks: a read of its own would
+// wait for the steps behind).  After every step already launched has drained, the control blocks start
+// afresh: the aborted step may have lowered the CFL minima, which a step takes back only behind its first
+// barrier, and the next one (after set_state) must not take its NT from them.
+int barrier_failed(cmf_gpu_ctx *c) {
+    int rc = read_ctl(c);
+    if (rc) return rc;
+    for (auto &x : c->hctl) {
+        x.bar_err = 0;
+        x.err = 0;
+        std::memcpy(&x.dtmin_bits, &x.dt_def, sizeof x.dtmin_bits);
+    }
+    CUDA_TRY(cudaMemcpyAsync(c->st.ctl, c->hctl.data(), c->hctl.size() * sizeof(cmf::MemberCtl), cudaMemcpyHostToDevice, c->stream));
+    CUDA_TRY(cudaStreamSynchronize(c->stream));
+    return set_err(CMF_E_BARRIER, "persistent kernel: a grid barrier did not complete within its bound");
+}
+
 // state arrays of the boundary are [M][NSEQMAX]; the device keeps [M][NSEQALL] (== NSEQMAX here)
 // NT, DT, budgets and statuses of the step whose control blocks are in c->hctl
 int process_ctl(cmf_gpu_ctx *c, int32_t *nt_out, double *dt_out, cmf_budget *b) {
-    if (c->hctl[0].bar_err) {       // comes with the control blocks: a read of its own would wait for the steps behind
-        c->hctl[0].bar_err = 0;
-        CUDA_TRY(cudaMemsetAsync(&c->st.ctl[0].bar_err, 0, sizeof(int), c->stream));
-        CUDA_TRY(cudaStreamSynchronize(c->stream));
-        return set_err(CMF_E_BARRIER, "persistent kernel: a grid barrier did not complete within its bound");
-    }
+    if (c->hctl[0].bar_err) return barrier_failed(c);
     int err = 0;
     int ntmax = 0;
     for (size_t m = 0; m < c->hctl.size(); m++) {
@@ -1292,7 +1304,7 @@ int cmf_gpu_ctx_persist_selftest(cmf_gpu_ctx *c, int64_t wait_ns) {
     if (!c) return set_err(CMF_E_STATE, "no context");
     if (wait_ns < 1000 || wait_ns > 2000000000LL) return set_err(CMF_E_ARG, "wait_ns must lie in [1 us, 2 s]");
     CUDA_TRY(cudaSetDevice(c->device));
-    int rc = launch_persist(c, (unsigned long long)wait_ns);
+    int rc = launch_persist(c, 1, (unsigned long long)wait_ns);
     if (rc) return rc;
     int berr = 0;
     CUDA_TRY(cudaMemcpyAsync(&berr, &c->st.ctl[0].bar_err, sizeof berr, cudaMemcpyDeviceToHost, c->stream));
@@ -1302,6 +1314,15 @@ int cmf_gpu_ctx_persist_selftest(cmf_gpu_ctx *c, int64_t wait_ns) {
     CUDA_TRY(cudaMemsetAsync(&c->st.ctl[0].bar_err, 0, sizeof(int), c->stream));
     CUDA_TRY(cudaStreamSynchronize(c->stream));
     return set_err(CMF_E_BARRIER, "persistent self-test: the grid barrier ran out its bound and the kernel returned");
+}
+
+int cmf_gpu_ctx_persist_selftest_step(cmf_gpu_ctx *c, double dt_def, int64_t wait_ns) {
+    if (!c) return set_err(CMF_E_STATE, "no context");
+    if (wait_ns < 1000 || wait_ns > 2000000000LL) return set_err(CMF_E_ARG, "wait_ns must lie in [1 us, 2 s]");
+    CUDA_TRY(cudaSetDevice(c->device));
+    int rc;
+    if ((rc = sync_dt_def(c, dt_def))) return rc;
+    return launch_persist(c, 2, (unsigned long long)wait_ns);
 }
 
 int32_t cmf_gpu_ctx_launch_mode(cmf_gpu_ctx *c) { return c ? (c->persist ? 2 : c->opts.launch_mode) : -1; }
@@ -1605,6 +1626,7 @@ int cmf_gpu_ctx_last_nt(cmf_gpu_ctx *c, int32_t *nt_out, double *dt_out) {
     CUDA_TRY(cudaSetDevice(c->device));
     int rc = read_ctl(c);
     if (rc) return rc;
+    if (c->hctl[0].bar_err) return barrier_failed(c);
     for (size_t m = 0; m < c->hctl.size(); m++) {
         if (nt_out) nt_out[m] = c->hctl[m].nt;
         if (dt_out) dt_out[m] = c->hctl[m].dt;

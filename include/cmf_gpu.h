@@ -212,7 +212,8 @@ int cmf_gpu_ctx_io_wait(cmf_gpu_ctx *ctx);
 int cmf_gpu_ctx_advance_device(cmf_gpu_ctx *ctx, double dt_def, int32_t ksteps,
                                const double *runoff_dev, int64_t runoff_stride);
 int cmf_gpu_ctx_synchronize(cmf_gpu_ctx *ctx);
-/* Per-member sub-step counts of the last outer step, read back from the device. */
+/* Per-member sub-step counts of the last outer step, read back from the device.  A barrier timeout of a
+ * persistent step launched by advance_device is reported here, or by the next step that reads back. */
 int cmf_gpu_ctx_last_nt(cmf_gpu_ctx *ctx, int32_t *nt_out, double *dt_out);
 /* CUDA stream (cudaStream_t) the context launches on, for event timing by the caller. */
 void *cmf_gpu_ctx_stream(cmf_gpu_ctx *ctx);
@@ -260,6 +261,10 @@ int cmf_gpu_ctx_get_diag_output(cmf_gpu_ctx *ctx, const cmf_diag_out_ptrs *dg);
  * kernel returns.  Returns CMF_E_BARRIER when the bound worked (the context stays usable: its
  * error word is cleared), another status otherwise.  No state changes. */
 int cmf_gpu_ctx_persist_selftest(cmf_gpu_ctx *ctx, int64_t wait_ns);
+/* The same inside an outer step: launches a step that gives up at its first barrier, as a real timeout
+ * would leave it.  The next call that reads the control blocks (cmf_gpu_ctx_last_nt, a step) returns
+ * CMF_E_BARRIER; the state is then an aborted step's, to be replaced by cmf_gpu_ctx_set_state. */
+int cmf_gpu_ctx_persist_selftest_step(cmf_gpu_ctx *ctx, double dt_def, int64_t wait_ns);
 /* The schedule the context runs: 0 graph, 1 host-driven, 2 persistent. */
 int32_t cmf_gpu_ctx_launch_mode(cmf_gpu_ctx *ctx);
 /* Adaptive-step statistics since creation: near_boundary = (outer step, member) pairs whose

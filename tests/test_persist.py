@@ -148,3 +148,37 @@ def test_persistent_bounded_wait_returns_status(case_dirs):
     sa, sb = g.get_state(), ref.get_state()
     for f in ("rivsto", "fldsto", "rivout", "fldout"):
         assert _same(sa[f], sb[f]), f
+
+
+@pytest.mark.parametrize("scale", [None, 1.05])
+@pytest.mark.parametrize("read", ["last_nt", "advance"])
+def test_step_after_an_aborted_one_takes_its_own_minimum(case_dirs, tmp_path, scale, read):
+    """A step that gives up at its first grid barrier has merged its cells' CFL minima.  The call that
+    reads the control blocks reports CMF_E_BARRIER, and a step from a new state then takes NT and DT
+    from that state alone (resident kernel, and the one over global memory)."""
+    from cmf_b200 import HostModel, PhysicsGPU
+
+    d = case_dirs["cfg1s"]
+    if scale:
+        d = str(tmp_path / "c")
+        synth.write_case(synth.make_case(synth.spec_config1(seed=3, scale=scale)), d)
+    h = HostModel(d)
+    g, ref = PhysicsGPU(h, launch_mode=2), PhysicsGPU(h, launch_mode=2)
+    r = next(iter(runoff_series(h.map("grarea"), "cfg1s", 1)))
+    g.put_runoff(r)
+    ref.put_runoff(r)
+    deep, _, _ = g.advance()
+    g.persist_selftest_step(2_000_000)
+    with pytest.raises(Exception, match="barrier"):
+        getattr(g, read)()
+    shallow = h.initial_state()
+    shallow["rivsto"] = 1e-3 * shallow["rivsto"]
+    for p in (g, ref):
+        p.set_state(shallow)
+    nt, dt, _ = g.advance()
+    nt_ref, dt_ref, _ = ref.advance()
+    assert nt_ref[0] < deep[0]
+    assert nt[0] == nt_ref[0] and _same(dt, dt_ref)
+    sa, sb = g.get_state(), ref.get_state()
+    for f in STATE_KEYS:
+        assert _same(sa[f], sb[f]), f
