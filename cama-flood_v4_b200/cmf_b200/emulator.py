@@ -518,6 +518,7 @@ def train(mlp: MLP, X, t, iters: int, batch: int, seed: int = 0, lr_max: float |
         mlp.adam()
         if it % 50 == 0 or it == iters - 1:
             hist.append((it, float(loss)))
+            echeck(mlp.lib.cmf_emu_mlp_tc_status(), f"train: iteration {it} or one of the 49 before it")
     return hist
 
 

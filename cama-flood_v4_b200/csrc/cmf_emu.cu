@@ -1292,10 +1292,12 @@ __global__ void __launch_bounds__(kTrThreads, 1) k_train(TrainArgs a, int wait_l
     fail = !mbar_wait(smem_u32(mbar + 2), 0u, kTcWaitLimit) || !ok;
     const bool failed = __syncthreads_or(fail);
     tc_fence_after();
+    float *out = a.ws + (size_t)blockIdx.x * kTrPart;
     if (failed) {
+        // no sums: NaN, so that the loss and every gradient show it whether or not the status is read
+        for (int e = tid; e < kTrPart; e += kTrThreads) out[e] = __int_as_float(0x7fc00000);
         if (tid == 0) atomicExch(&g_mlp_tc_status, 1);
     } else {
-        float *out = a.ws + (size_t)blockIdx.x * kTrPart;
         uint32_t d[32];
         // D lanes are n, columns k: consecutive lanes store consecutive n of one k
 #pragma unroll

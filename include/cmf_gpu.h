@@ -409,7 +409,8 @@ int cmf_emu_adam_set(int count, const int32_t *n, float *const *w, void *const *
  * gb[0..3] (fp32, every element) and *loss = sum over the first `valid` rows of (y - t)^2 / valid,
  * with the rounding points of the layer-by-layer chain and the same bits on every run.
  * workspace: cmf_emu_loss_grad_ws_floats(rows) floats.  The three arrays of pointers are host
- * arrays.  A launch that gives up a bounded MMA wait reports through cmf_emu_mlp_tc_status. */
+ * arrays.  A launch that gives up a bounded MMA wait reports through cmf_emu_mlp_tc_status, and its
+ * loss and gradients are NaN. */
 size_t cmf_emu_loss_grad_ws_floats(int rows);
 int cmf_emu_loss_grad(int rows, int valid, const void *X, const float *t, const void *const *W, const float *const *b,
                       float *const *gW, float *const *gb, float *loss, float *workspace, size_t workspace_floats,

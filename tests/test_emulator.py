@@ -571,3 +571,32 @@ def test_fused_training_step_bounded_wait_reports():
     torch.cuda.synchronize()
     assert lib.cmf_emu_mlp_tc_status() == 0
     assert torch.equal(ref, again)
+
+
+@pytest.mark.gpu
+def test_training_step_that_gives_up_leaves_no_stale_gradients():
+    """With a wait bound of 0 the loss and the used gradients are NaN, not the sums of the step before, and
+    train() raises instead of going on from them."""
+    import torch
+
+    from cmf_b200.emulator import MLP, _emu_lib, train
+
+    lib, dev = _emu_lib(), torch.device("cuda", 0)
+    mlp = MLP(dev, seed=5)
+    X = torch.zeros(4096, 64, dtype=torch.bfloat16, device=dev)
+    X[:, :32] = torch.randn(4096, 32, device=dev, generator=torch.Generator(device=dev).manual_seed(1)).to(torch.bfloat16)
+    t = torch.ones(4096, device=dev)
+    assert bool(torch.isfinite(mlp.loss_and_grad(X, t, 4096)))
+    assert len(train(mlp, X, t, iters=2, batch=512)) == 2
+    try:
+        assert lib.cmf_emu_mlp_tc_set_wait_limit(0) == 0
+        loss = mlp.loss_and_grad(X, t, 4096)
+        assert bool(torch.isnan(loss))
+        used = mlp.gW[:3] + [mlp.gW[3][:, 0]] + mlp.gb[:3] + [mlp.gb[3][0]]
+        assert all(bool(torch.isnan(g).all()) for g in used)
+        assert lib.cmf_emu_mlp_tc_status() == 1
+        with pytest.raises(RuntimeError, match="train"):
+            train(mlp, X, t, iters=2, batch=512)
+    finally:
+        lib.cmf_emu_mlp_tc_set_wait_limit(-1)
+    assert lib.cmf_emu_mlp_tc_status() == 0
