@@ -110,7 +110,7 @@ EXPORTS = [
     "cmf_host_load", "cmf_host_free", "cmf_host_describe", "cmf_host_state", "cmf_host_conv_resol", "cmf_host_grid",
     "cmf_gpu_stage_noalloc", "cmf_gpu_ctx_nt_stats", "cmf_gpu_ctx_diag_output", "cmf_gpu_ctx_get_diag_output",
     "cmf_gpu_diag_output", "cmf_gpu_get_diag_output", "cmf_gpu_ctx_persist_selftest", "cmf_gpu_ctx_launch_mode",
-    "cmf_gpu_ctx_persist_selftest_step",
+    "cmf_gpu_ctx_persist_selftest_step", "cmf_gpu_schedule_pick",
     "cmf_gpu_ctx_get_schedule", "cmf_gpu_ctx_set_schedule", "cmf_gpu_ctx_put_runoff_async",
     "cmf_gpu_ctx_advance_async", "cmf_gpu_ctx_wait", "cmf_gpu_ctx_get_diag_async", "cmf_gpu_ctx_io_wait",
 ]
@@ -163,6 +163,7 @@ def load(build_if_missing: bool = True):
     lib.cmf_gpu_ctx_persist_selftest_step.argtypes = [vp, C.c_double, C.c_int64]
     lib.cmf_gpu_ctx_get_schedule.argtypes = [vp, C.POINTER(Schedule)]
     lib.cmf_gpu_ctx_set_schedule.argtypes = [vp, C.POINTER(Schedule)]
+    lib.cmf_gpu_schedule_pick.argtypes = [C.POINTER(Schedule), C.c_int32, C.POINTER(Schedule)]
     lib.cmf_gpu_schedule_cache_clear.restype = None
     lib.cmf_gpu_ctx_launch_mode.argtypes = [vp]
     lib.cmf_gpu_ctx_diag_output.argtypes = [vp, C.c_int32]

@@ -50,7 +50,8 @@ constexpr int kImis = -9999;
 // per-warp partials), so the autotuner may switch between them at any outer step.
 struct Sched {
     int mode = 0;               // 0 graph of phase kernels, 2 persistent kernel
-    int bf = 256, br = 256, bs = 256;
+    int bf = 256, br = 256, bs = 256;   // of the phase kernels, which also a mode 2 context runs: in a batch, in
+                                        // substeps() and time_phases()
     int prof = 0;               // 0 wide, 1 small
     bool operator==(const Sched &o) const {
         return mode == o.mode && bf == o.bf && br == o.br && bs == o.bs && prof == o.prof;
@@ -779,6 +780,22 @@ SchedKey sched_key(const cmf_gpu_ctx *c) {
     return SchedKey{c->device, c->dims.nseqall, c->dims.nseqriv, c->dims.nmembers, c->net.P, c->net.Lp, flags};
 }
 
+// The fastest of the timed schedules.  Where that is the persistent kernel, the block sizes and profile of the
+// fastest graph schedule come with it, for the calls that run the phase kernels all the same.
+Sched pick_sched(const std::vector<Sched> &cands, const std::vector<double> &ms) {
+    size_t best = 0, phase = cands.size();
+    for (size_t k = 0; k < cands.size(); k++) {
+        if (ms[k] < ms[best]) best = k;
+        if (cands[k].mode == 0 && (phase == cands.size() || ms[k] < ms[phase])) phase = k;
+    }
+    Sched q = cands[best];
+    if (q.mode == 2 && phase < cands.size()) {
+        q = cands[phase];
+        q.mode = 2;
+    }
+    return q;
+}
+
 // before an outer step: the tuner's schedule for it, and the start of its timing
 int tune_begin(cmf_gpu_ctx *c, bool &trial) {
     trial = false;
@@ -825,9 +842,10 @@ int tune_end(cmf_gpu_ctx *c, bool trial) {
     t.worst_us = t.ms[worst] * 1e3;
     t.timed = (int)t.cands.size();
     t.active = false;
-    if ((rc = apply_sched(c, t.cands[best]))) return rc;
+    const Sched q = pick_sched(t.cands, t.ms);
+    if ((rc = apply_sched(c, q))) return rc;
     std::lock_guard<std::mutex> lk(g_sched_mu);
-    g_sched_cache[sched_key(c)] = t.cands[best];
+    g_sched_cache[sched_key(c)] = q;
     return CMF_OK;
 }
 
@@ -1154,7 +1172,7 @@ int cmf_gpu_create(const cmf_dims *dims, const cmf_params *params, const cmf_map
                         t.cands.push_back(k);
                     }
             if (c->persist_grid > 0) {
-                Sched k;
+                Sched k = q;
                 k.mode = 2;
                 t.cands.push_back(k);
             }
@@ -1804,6 +1822,28 @@ int cmf_gpu_ctx_get_schedule(cmf_gpu_ctx *c, cmf_schedule *out) {
 void cmf_gpu_schedule_cache_clear(void) {
     std::lock_guard<std::mutex> lk(g_sched_mu);
     g_sched_cache.clear();
+}
+
+int cmf_gpu_schedule_pick(const cmf_schedule *timed, int32_t n, cmf_schedule *out) {
+    if (!timed || n < 1 || !out) return set_err(CMF_E_ARG, "cmf_gpu_schedule_pick: null argument or no schedule");
+    std::vector<Sched> cands(n);
+    std::vector<double> us(n);
+    for (int k = 0; k < n; k++) {
+        cands[k].mode = timed[k].mode;
+        cands[k].bf = timed[k].flux_block;
+        cands[k].br = timed[k].rate_block;
+        cands[k].bs = timed[k].store_block;
+        cands[k].prof = timed[k].profile;
+        us[k] = timed[k].best_us_per_substep;
+    }
+    const Sched q = pick_sched(cands, us);
+    *out = cmf_schedule{};
+    out->mode = q.mode;
+    out->flux_block = q.bf;
+    out->rate_block = q.br;
+    out->store_block = q.bs;
+    out->profile = q.prof;
+    return CMF_OK;
 }
 
 int cmf_gpu_ctx_set_schedule(cmf_gpu_ctx *c, const cmf_schedule *q) {

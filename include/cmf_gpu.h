@@ -239,6 +239,10 @@ typedef struct cmf_schedule {
 } cmf_schedule;
 int cmf_gpu_ctx_get_schedule(cmf_gpu_ctx *ctx, cmf_schedule *out);
 int cmf_gpu_ctx_set_schedule(cmf_gpu_ctx *ctx, const cmf_schedule *sched);
+/* The autotuner's rule on `n` timed schedules (best_us_per_substep): the fastest; where that is the
+ * persistent kernel, with the block sizes and profile of the fastest graph schedule, which batches,
+ * cmf_gpu_ctx_substeps and cmf_gpu_ctx_time_phases run.  Host only. */
+int cmf_gpu_schedule_pick(const cmf_schedule *timed, int32_t n, cmf_schedule *out);
 /* Forgets the cached schedules, so that the next contexts tune again. */
 void cmf_gpu_schedule_cache_clear(void);
 /* Device-side counters since creation: sum over outer steps and members of NT, sum over outer

@@ -80,3 +80,64 @@ def test_batch_rejects_bad_input():
     arr = (C.c_void_p * 1)(None)
     assert lib.cmf_gpu_batch_create(arr, 1, C.byref(h)) == -1
     assert lib.cmf_gpu_batch_launch(None, 3600.0) == -3
+
+
+@pytest.mark.gpu
+def test_batch_of_tuned_contexts_equals_each_domain_alone(case_dirs):
+    """Contexts that have tuned themselves (small nets take the persistent kernel, which a batch does not
+    run) give the same bits in a batch as contexts of a fixed schedule alone."""
+    from cmf_b200 import HostModel, PhysicsBatch, PhysicsGPU, _abi
+
+    _abi.load().cmf_gpu_schedule_cache_clear()
+    hosts = [HostModel(case_dirs[name]) for name, _ in DOMAINS]
+    alone = [PhysicsGPU(h, nmembers=m, block_size=256) for h, (_, m) in zip(hosts, DOMAINS)]
+    batched = [PhysicsGPU(h, nmembers=m) for h, (_, m) in zip(hosts, DOMAINS)]
+    forc = [_runoff(h, name, m, 5 + k) for k, ((name, m), h) in enumerate(zip(DOMAINS, hosts))]
+    for k in range(24):                       # 4 steps, then 2 of each of the 9 candidates
+        for d in range(len(DOMAINS)):
+            for p in (alone[d], batched[d]):
+                p.put_runoff(forc[d][k % STEPS])
+                p.advance()
+    assert all(p.schedule()["tuned"] == 1 for p in batched)
+    batch = PhysicsBatch(batched)
+    for k in range(STEPS):
+        for d in range(len(DOMAINS)):
+            alone[d].put_runoff(forc[d][k])
+            batched[d].put_runoff(forc[d][k])
+        res = batch.advance()
+        for d in range(len(DOMAINS)):
+            nt, dt, bud = alone[d].advance()
+            nt_b, dt_b, bud_b = res[d]
+            assert np.array_equal(nt, nt_b) and np.array_equal(dt.view(np.int64), dt_b.view(np.int64)), (d, k)
+            assert bud == bud_b, (d, k)
+    for d in range(len(DOMAINS)):
+        a, b = _state_bits(alone[d]), _state_bits(batched[d])
+        for f in a:
+            assert np.array_equal(a[f], b[f]), (DOMAINS[d], f)
+    batch.close()
+    for p in alone + batched:
+        p.close()
+
+
+def test_schedule_pick_keeps_the_fastest_phase_schedule():
+    """Where the persistent kernel is the fastest, the phase kernels' block sizes and profile are those of
+    the fastest graph schedule, not of the persistent candidate."""
+    import ctypes as C
+
+    from cmf_b200 import _abi
+
+    lib = _abi.load()
+
+    def pick(rows):
+        timed = (_abi.Schedule * len(rows))(*[_abi.Schedule(mode=m, flux_block=f, rate_block=f, store_block=s, profile=p,
+                                                            best_us_per_substep=t) for m, f, s, p, t in rows])
+        q = _abi.Schedule()
+        assert lib.cmf_gpu_schedule_pick(timed, len(rows), C.byref(q)) == 0
+        return q.mode, q.flux_block, q.rate_block, q.store_block, q.profile
+
+    graphs = [(0, 128, 256, 0, 60.0), (0, 256, 128, 1, 55.0), (0, 256, 256, 0, 57.0)]
+    assert pick(graphs + [(2, 128, 128, 1, 38.0)]) == (2, 256, 256, 128, 1)
+    assert pick([(2, 128, 128, 1, 38.0)] + graphs) == (2, 256, 256, 128, 1)
+    assert pick(graphs + [(2, 128, 128, 1, 80.0)]) == (0, 256, 256, 128, 1)
+    assert pick([(2, 64, 128, 0, 38.0)]) == (2, 64, 64, 128, 0)
+    assert lib.cmf_gpu_schedule_pick(None, 1, None) == -1
