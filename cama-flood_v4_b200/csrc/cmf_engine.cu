@@ -85,7 +85,8 @@ struct cmf_gpu_ctx {
     std::vector<void *> allocs;
     Sched sched;                // the launch schedule of the outer step
     int persist_grid = 0;       // co-resident CTAs of the persistent kernel (0: it cannot run here)
-    cmf::ResArgs res{};         // its resident form (group 0: a member does not fit the SMs)
+    cmf::ResArgs res{};         // its resident form (group 0: a member does not fit the SMs); buffers on first use
+    std::vector<int> res_order, res_xpos;   // ResArgs::order and xpos
     int res_threads = 0;
     void (*res_kernel)(cmf::Net, cmf::State, cmf::ResArgs) = nullptr;   // k_resident with the registers its tasks leave
     bool l2_window = false;     // the hot maps sit under a persisting L2 access-policy window
@@ -221,7 +222,8 @@ int build_net(cmf_gpu_ctx *c, const cmf_map_ptrs *mp) {
         up_ptr[i + 1] = (int)up_idx.size();
     }
     c->E = up_idx.size();
-    std::vector<int> xpos(N, -1);
+    std::vector<int> &xpos = c->res_xpos;
+    xpos.assign(N, -1);
     int degmax = 0;
     for (size_t k = 0; k < up_idx.size(); k++) xpos[up_idx[k]] = (int)k;
     for (int i = 0; i < N; i++) degmax = std::max(degmax, up_ptr[i + 1] - up_ptr[i]);
@@ -235,7 +237,7 @@ int build_net(cmf_gpu_ctx *c, const cmf_map_ptrs *mp) {
     }
     int rc;
     if ((rc = c->upload(&n.next, next)) || (rc = c->upload(&n.up_ptr, up_ptr)) || (rc = c->upload(&n.up_idx, up_idx)) ||
-        (rc = c->upload(&n.up_ell, up_ell)) || (rc = c->upload(&c->res.xpos, xpos)))
+        (rc = c->upload(&n.up_ell, up_ell)))
         return rc;
     std::vector<int> i2mask(mp->i2mask, mp->i2mask + N);
     if ((rc = c->upload(&n.i2mask, i2mask))) return rc;
@@ -398,7 +400,7 @@ int build_net(cmf_gpu_ctx *c, const cmf_map_ptrs *mp) {
     // cells, other ends of paths, the rest, each class ascending
     {
         std::vector<unsigned char> fl(N, 0);
-        std::vector<int> dams, rules, order, pos(N, -1), dup_ptr, dup_idx;
+        std::vector<int> dams, rules, &order = c->res_order, pos(N, -1), dup_ptr, dup_idx;
         std::vector<double> vel, velf;
         for (int p = 0; p < n.P; p++)
             for (int e : {h_pu[p], h_pd[p]})
@@ -442,7 +444,7 @@ int build_net(cmf_gpu_ctx *c, const cmf_map_ptrs *mp) {
         for (int i = 0; i < N; i++) if (!(fl[i] & (cmf::C_PATH | cmf::C_DAM))) order.push_back(i);
         if ((rc = c->upload(&n.cflag, fl)) || (rc = c->upload(&n.dam_cells, dams)) || (rc = c->upload(&n.dam_pos, pos)) ||
             (rc = c->upload(&n.dam_up_ptr, dup_ptr)) || (rc = c->upload(&n.dam_up_idx, dup_idx)) ||
-            (rc = c->upload(&n.kin_vel, vel)) || (rc = c->upload(&n.kin_velf, velf)) || (rc = c->upload(&c->res.order, order)))
+            (rc = c->upload(&n.kin_vel, vel)) || (rc = c->upload(&n.kin_velf, velf)))
             return rc;
         c->res.cells = (int)order.size();
         // levees at the ends of paths
@@ -685,6 +687,15 @@ int sync_dt_def(cmf_gpu_ctx *c, double dt_def) {
 }
 
 // ---- persistent schedule: one cooperative launch per outer step --------------------------------
+int persist_global(cmf_gpu_ctx *c) {
+    int per_sm = 0, nsm = 0;
+    CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->device));
+    CUDA_TRY(cudaFuncSetAttribute(cmf::k_persist, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cmf::kPersistSmem));
+    CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, cmf::k_persist, cmf::kTile, cmf::kPersistSmem));
+    c->persist_grid = per_sm * nsm;
+    return CMF_OK;
+}
+
 // The persistent schedule runs the resident kernel when one member's cells fit the SMs (one CTA per SM
 // with kResMaxSlots tiles), and k_persist for larger members.  Members are grouped evenly over the
 // fewest groups that fit.
@@ -714,25 +725,49 @@ int persist_setup(cmf_gpu_ctx *c) {
             a.group = (int)group;
             a.wait_ns = cmf::kWaitNsDefault;
             a.selftest = 0;
-            int rc;
-            const size_t gn = (size_t)group * c->res.edges;
-            if ((rc = c->alloc(&a.raw, gn)) || (rc = c->alloc(&a.out, gn)) ||
-                (rc = c->alloc(&a.terms, (size_t)cmf::kBudgets * group * tpm * 32)))
-                return rc;
             c->persist_grid = grid;
             c->res_threads = threads;
             return CMF_OK;
         }
     }
-    CUDA_TRY(cudaFuncSetAttribute(cmf::k_persist, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cmf::kPersistSmem));
-    CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, cmf::k_persist, cmf::kTile, cmf::kPersistSmem));
-    c->persist_grid = per_sm * nsm;
+    return persist_global(c);
+}
+
+// The resident kernel's exchange arrays, budget terms and orders: made when a schedule first runs it (up to 128 B
+// per cell and member of a group, which a context of phase kernels keeps for its members), and given back
+// when the autotuner decides against it.  Without the memory the persistent schedule goes on as k_persist.
+void resident_release(cmf_gpu_ctx *c) {
+    cmf::ResArgs &a = c->res;
+    for (const void *p : {(const void *)a.raw, (const void *)a.out, (const void *)a.terms, (const void *)a.order, (const void *)a.xpos}) {
+        auto at = std::find(c->allocs.begin(), c->allocs.end(), p);
+        if (!p || at == c->allocs.end()) continue;
+        cudaFree(*at);
+        c->allocs.erase(at);
+    }
+    a.raw = a.out = nullptr;
+    a.terms = nullptr;
+    a.order = a.xpos = nullptr;
+}
+int resident_buffers(cmf_gpu_ctx *c) {
+    cmf::ResArgs &a = c->res;
+    if (a.group == 0 || a.xpos) return CMF_OK;
+    const size_t gn = (size_t)a.group * a.edges;
+    if (c->alloc(&a.raw, gn) || c->alloc(&a.out, gn) ||
+        c->alloc(&a.terms, (size_t)cmf::kBudgets * a.group * a.tpm * 32) || c->upload(&a.order, c->res_order) ||
+        c->upload(&a.xpos, c->res_xpos)) {
+        cudaGetLastError();     // no memory for them: the persistent kernel over global memory
+        resident_release(c);
+        a.group = 0;
+        return persist_global(c);
+    }
     return CMF_OK;
 }
 
 // one outer step as one cooperative launch; `selftest` (ResArgs): with waits of selftest_ns that cannot end
 int launch_persist(cmf_gpu_ctx *c, int selftest = 0, unsigned long long selftest_ns = 0) {
     if (c->persist_grid < 1) return set_err(CMF_E_UNSUPPORTED, "the persistent kernel cannot be co-resident on this device");
+    int rc;
+    if ((rc = resident_buffers(c))) return rc;
     CUDA_TRY(cudaMemsetAsync(&c->st.loop->bar, 0, sizeof(unsigned), c->stream));
     if (c->res.group > 0) {
         cmf::ResArgs a = c->res;
@@ -764,6 +799,8 @@ int build_graph(cmf_gpu_ctx *c);
 
 // Installs a schedule: the persistent flag and, for graph launches, the graph of the phase kernels.
 int apply_sched(cmf_gpu_ctx *c, const Sched &q) {
+    int rc;
+    if (q.mode == 2 && (rc = resident_buffers(c))) return rc;
     const bool rebuild = c->opts.launch_mode == 0 && q.mode == 0 && (!c->exec || !(q == c->sched) || c->persist);
     c->sched = q;
     c->persist = q.mode == 2;
@@ -796,6 +833,22 @@ Sched pick_sched(const std::vector<Sched> &cands, const std::vector<double> &ms)
     return q;
 }
 
+// after the last candidate: the fastest schedule is installed and cached
+int tune_finish(cmf_gpu_ctx *c) {
+    Tuner &t = c->tune;
+    t.best_us = *std::min_element(t.ms.begin(), t.ms.end()) * 1e3;
+    t.worst_us = *std::max_element(t.ms.begin(), t.ms.end()) * 1e3;
+    t.timed = (int)t.cands.size();
+    t.active = false;
+    const Sched q = pick_sched(t.cands, t.ms);
+    int rc;
+    if ((rc = apply_sched(c, q))) return rc;
+    if (q.mode != 2) resident_release(c);
+    std::lock_guard<std::mutex> lk(g_sched_mu);
+    g_sched_cache[sched_key(c)] = q;
+    return CMF_OK;
+}
+
 // before an outer step: the tuner's schedule for it, and the start of its timing
 int tune_begin(cmf_gpu_ctx *c, bool &trial) {
     trial = false;
@@ -815,8 +868,7 @@ int tune_begin(cmf_gpu_ctx *c, bool &trial) {
     return CMF_OK;
 }
 
-// after a timed outer step: time per sub-step of the candidate; after the last candidate, the
-// fastest schedule is installed and cached
+// after a timed outer step: time per sub-step of the candidate
 int tune_end(cmf_gpu_ctx *c, bool trial) {
     if (!trial) return CMF_OK;
     Tuner &t = c->tune;
@@ -833,20 +885,7 @@ int tune_end(cmf_gpu_ctx *c, bool trial) {
     if (++t.rep < t.reps) return CMF_OK;
     t.rep = 0;
     if (++t.cand < (int)t.cands.size()) return CMF_OK;
-    size_t best = 0, worst = 0;
-    for (size_t k = 1; k < t.cands.size(); k++) {
-        if (t.ms[k] < t.ms[best]) best = k;
-        if (t.ms[k] > t.ms[worst]) worst = k;
-    }
-    t.best_us = t.ms[best] * 1e3;
-    t.worst_us = t.ms[worst] * 1e3;
-    t.timed = (int)t.cands.size();
-    t.active = false;
-    const Sched q = pick_sched(t.cands, t.ms);
-    if ((rc = apply_sched(c, q))) return rc;
-    std::lock_guard<std::mutex> lk(g_sched_mu);
-    g_sched_cache[sched_key(c)] = q;
-    return CMF_OK;
+    return tune_finish(c);
 }
 
 int launch_outer(cmf_gpu_ctx *c) {

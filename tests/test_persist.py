@@ -182,3 +182,36 @@ def test_step_after_an_aborted_one_takes_its_own_minimum(case_dirs, tmp_path, sc
     sa, sb = g.get_state(), ref.get_state()
     for f in STATE_KEYS:
         assert _same(sa[f], sb[f]), f
+
+
+def test_resident_buffers_are_made_on_first_use(case_dirs):
+    """Contexts whose schedule is one of phase kernels hold none of the resident kernel's buffers (budget
+    terms alone are 96 B per cell and member); they appear when a schedule first runs it."""
+    import torch
+
+    from cmf_b200 import HostModel, PhysicsGPU
+
+    h = HostModel(case_dirs["cfg1s"])
+    M, N = 64, h.dims.nseqall
+    need = 96 * M * N
+    free = lambda: torch.cuda.mem_get_info(0)[0]  # noqa: E731
+
+    def made(**kw):
+        torch.cuda.synchronize()
+        before = free()
+        p = PhysicsGPU(h, nmembers=M, **kw)
+        return p, before - free()
+
+    made(launch_mode=2)[0].close()               # modules and streams of a first context
+    resident, with_buffers = made(launch_mode=2)
+    resident.close()
+    for kw in (dict(launch_mode=1), dict(block_size=128)):
+        p, bytes_ = made(**kw)
+        assert bytes_ <= with_buffers - need, (kw, bytes_, with_buffers, need)
+        if "block_size" in kw:
+            at = free()
+            p.set_schedule(mode=2)
+            assert at - free() >= need
+            p.put_runoff(np.zeros((M, N)))
+            p.advance()
+        p.close()
