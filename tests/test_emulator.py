@@ -600,3 +600,58 @@ def test_training_step_that_gives_up_leaves_no_stale_gradients():
     finally:
         lib.cmf_emu_mlp_tc_set_wait_limit(-1)
     assert lib.cmf_emu_mlp_tc_status() == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows,valid,tile", [(64, 64, None), (128 * 148, 16384, None), (128 * 149 + 64, 16384, None),
+                                             (128 * 300, 32768, None), (128 * 300, 32768, 0), (128 * 300, 32768, 147),
+                                             (128 * 300, 32768, 148), (128 * 300, 32768, 255), (128 * 296, 32768, 200)])
+def test_fused_training_step_is_exact_on_integers(rows, valid, tile):
+    """Inputs and weights of -1, 0 and 1 (two per row and column of a hidden layer) and errors of at most 16
+    keep every activation, dZ and sum a whole number that bf16 or fp32 holds, `valid` is a power of two:
+    loss and gradients equal the 64-bit ones bit for bit, over every tile a CTA takes.  With `tile`, only
+    that tile's rows have errors, so a lost or doubled tile changes every gradient."""
+    import torch
+
+    from cmf_b200.emulator import MLP, OUT, _emu_lib
+
+    dev = torch.device("cuda", 0)
+    rng = np.random.default_rng(rows + valid)
+    n = np.arange(128)
+    W = [np.zeros((64, 128), np.float32), np.zeros((128, 128), np.float32), np.zeros((128, 128), np.float32),
+         np.zeros((128, OUT), np.float32)]
+    sign = lambda size: rng.integers(0, 2, size) * 2.0 - 1.0  # noqa: E731
+    for w, shift in zip(W[:3], (5, 7, 11)):
+        w[n % w.shape[0], n] = sign(128)
+        w[(n + shift) % w.shape[0], n] = sign(128)
+    W[3][:, 0] = sign(128)
+    b = [rng.integers(0, 2, 128).astype(np.float32) for _ in range(3)] + [np.full(OUT, 3.0, np.float32)]
+    mlp = MLP(dev, seed=4)
+    mlp.load({"W": W, "b": b})
+    X = torch.tensor(rng.integers(-1, 2, (rows, 64)), device=dev).to(torch.bfloat16)
+    acts = [X.double()]
+    for k in range(3):
+        acts.append(torch.relu(acts[k] @ mlp.W[k].double() + mlp.b[k].double()))
+    y = (acts[3] @ mlp.W[3].double())[:, 0] + 3.0
+    err = torch.tensor(rng.integers(-16, 17, rows), device=dev).double()
+    if tile is not None:
+        at = torch.arange(rows, device=dev) // 128 == tile
+        err = torch.where(at, torch.where(err == 0, 1.0, err), 0.0)
+    t = (y - err).float()
+    loss = mlp.loss_and_grad(X, t, valid)
+    torch.cuda.synchronize()
+    assert _emu_lib().cmf_emu_mlp_tc_status() == 0
+    err[valid:] = 0.0
+    assert bool(err.any()) and float(acts[3].max()) <= 256
+    dZ = (2.0 * err / valid)[:, None]
+    want_w, want_b = [None] * 4, [None] * 4
+    for k in (3, 2, 1, 0):
+        want_w[k], want_b[k] = acts[k].T @ dZ, dZ.sum(0)
+        if k:
+            dZ = (dZ @ (mlp.W[k].double().T if k < 3 else mlp.W[3][:, :1].double().T)) * (acts[k] > 0)
+            assert float(dZ.abs().max()) * valid / 2.0 <= 256
+    assert float(loss) == float((err ** 2).sum() / valid)
+    for k in range(3):
+        assert torch.equal(mlp.gW[k].double(), want_w[k]) and torch.equal(mlp.gb[k].double(), want_b[k]), k
+    assert torch.equal(mlp.gW[3][:, 0].double(), want_w[3][:, 0]) and float(mlp.gb[3][0]) == float(want_b[3][0])
+    assert not mlp.gW[3][:, 1:].any() and not mlp.gb[3][1:].any()
