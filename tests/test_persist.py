@@ -215,3 +215,47 @@ def test_resident_buffers_are_made_on_first_use(case_dirs):
             p.put_runoff(np.zeros((M, N)))
             p.advance()
         p.close()
+
+
+@pytest.mark.parametrize("upstream", [15, 16, 40])
+def test_persistent_with_many_upstream_cells(case_dirs, upstream):
+    """A cell of 15 upstream cells is the widest the resident kernel packs; with more the persistent
+    schedule runs the kernel over global memory.  Both leave the bits of the graph of phase kernels."""
+    import ctypes as C
+
+    from cmf_b200 import HostModel, PhysicsGPU
+
+    h = HostModel(case_dirs["cfg1s"])
+    N, R = h.dims.nseqall, h.dims.nseqriv
+    nxt = np.ctypeslib.as_array(h.maps.i1next, shape=(N,))
+    # headwaters of plain channels drain into the last river cell but a few
+    target = R - 5
+    dam, mask = h.map("i1dam"), h.map("i2mask")
+    heads = [i for i in range(target) if not np.any(nxt[:R] == i + 1) and dam[i] == 0 and mask[i] == 0 and nxt[i] != target + 1]
+    have = int((nxt[:R] == target + 1).sum())
+    for i in heads[:upstream - have]:
+        nxt[i] = target + 1
+    lists = [np.flatnonzero(nxt[:R] == j + 1) + 1 for j in range(N)]
+    most = max(len(v) for v in lists)
+    assert most == upstream
+    upst = np.zeros((most, N), dtype=np.int32)
+    upn = np.array([len(v) for v in lists], dtype=np.int32)
+    for j, v in enumerate(lists):
+        upst[:len(v), j] = v
+    h.dims.upnmax = most
+    h.maps.i1upst = upst.ctypes.data_as(C.POINTER(C.c_int32))
+    h.maps.i1upn = upn.ctypes.data_as(C.POINTER(C.c_int32))
+    series = list(runoff_series(h.map("grarea"), "stress", 4, hourly=True))
+    a = PhysicsGPU(h, nmembers=2, launch_mode=2)
+    b = PhysicsGPU(h, nmembers=2, launch_mode=0, block_size=256)
+    for r in series:
+        for p in (a, b):
+            p.put_runoff(np.stack([r, 2.0 * r]))
+        (na, da, ba), (nb, db, bb) = a.advance(), b.advance()
+        assert np.array_equal(na, nb) and _same(da, db) and ba == bb
+    sa, sb = a.get_state(), b.get_state()
+    ga, gb = a.get_diag(), b.get_diag()
+    for f in STATE_KEYS:
+        assert _same(sa[f], sb[f]), f
+    for f in DIAG_KEYS:
+        assert _same(ga[f], gb[f]), f
