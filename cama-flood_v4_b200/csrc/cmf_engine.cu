@@ -390,7 +390,7 @@ int build_net(cmf_gpu_ctx *c, const cmf_map_ptrs *mp) {
         c->ndam_placed = (int)stat.size();
         if (stat.empty()) stat.push_back(0);
         for (auto *v : {&qn, &qf, &qa, &con, &eme, &nor, &adj, &rvu}) if (v->empty()) v->push_back(0.0);
-        if ((rc = c->upload(&n.i1dam, i1dam)) || (rc = c->upload(&n.dam_id, dam_id)) || (rc = c->upload(&n.dam_stat, stat)) ||
+        if ((rc = c->upload(&n.dam_id, dam_id)) || (rc = c->upload(&n.dam_stat, stat)) ||
             (rc = c->upload(&n.qn, qn)) || (rc = c->upload(&n.qf, qf)) || (rc = c->upload(&n.qa, qa)) ||
             (rc = c->upload(&n.convol, con)) || (rc = c->upload(&n.emevol, eme)) || (rc = c->upload(&n.norvol, nor)) ||
             (rc = c->upload(&n.adjvol, adj)) || (rc = c->upload(&n.r_volupa, rvu)))

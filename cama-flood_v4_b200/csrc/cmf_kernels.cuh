@@ -119,7 +119,6 @@ struct Net {
     const double *__restrict__ levhgt, *__restrict__ levfrc, *__restrict__ bashgt, *__restrict__ levdst;
     const double *__restrict__ levbassto, *__restrict__ levtopsto, *__restrict__ levfilsto;
     // dams
-    const int *__restrict__ i1dam;      // [N]
     const int *__restrict__ dam_id;     // [N] compact dam of the cell or -1
     const int *__restrict__ dam_stat;   // [D]
     // what a cell takes part in (CellFlag), and the cells of reservoir operation (I1DAM > 0), which run
@@ -204,7 +203,6 @@ struct OwnMaps {
     __device__ __forceinline__ int up_lo(int i) const { return __ldg(&n.up_ptr[i]); }
     __device__ __forceinline__ int up_hi(int i) const { return __ldg(&n.up_ptr[i + 1]); }
     __device__ __forceinline__ int up_slot(int k, int i) const { return __ldg(&n.up_ell[(size_t)k * n.N + i]); }
-    __device__ __forceinline__ int i1dam(int i) const { return __ldg(&n.i1dam[i]); }
 };
 struct LazyRate;
 // What phase B leaves of an outflow: a positive one (and a mouth's) is rescaled by its own cell's rate here, and
@@ -633,27 +631,6 @@ __device__ __forceinline__ void begin_cell(const Net &n, const State &s, size_t 
     if (some(s.fldout_pre[gi])) w |= W_FOUT;
     s.wet[gi] = (unsigned char)w;
     s.dph[gi] = make_double2(rivdph, s.rivdph_pre[gi]);
-}
-
-template <int NV>
-__device__ __forceinline__ void block_sum(double (&v)[NV], double *smem /* [32*NV] */) {
-    // fixed-shape tree: warp butterfly, then warp 0 over the warp partials -> deterministic
-#pragma unroll
-    for (int k = 0; k < NV; k++)
-        for (int o = 16; o > 0; o >>= 1) v[k] = v[k] + __shfl_down_sync(0xffffffffu, v[k], o);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
-    if (lane == 0)
-#pragma unroll
-        for (int k = 0; k < NV; k++) smem[warp * NV + k] = v[k];
-    __syncthreads();
-    if (warp == 0) {
-#pragma unroll
-        for (int k = 0; k < NV; k++) {
-            double x = lane < nw ? smem[lane * NV + k] : 0.0;
-            for (int o = 16; o > 0; o >>= 1) x = x + __shfl_down_sync(0xffffffffu, x, o);
-            v[k] = x;
-        }
-    }
 }
 
 // ------------------------------------------------------------------------------------------
