@@ -202,32 +202,46 @@ def closure(budgets: list) -> dict:
 
 
 # ----------------------------------------------------------------------------- algorithmic bytes
-def phase_bytes(N: int, E: int, L_bar: float, P: int, Lp: int, nlev: int, ndam: int, ldiag: bool) -> dict:
-    """Compulsory HBM bytes per launch of each sub-step kernel (every array element the kernel must
-    read or write once every sub-step; gathers of neighbour values are L2 reuse and not counted
-    again; outputs written on the last sub-step only -- D2RIVVEL, D2RIVINF, D2FLDINF, D2PTHOUT,
-    D2OUTFLW, D2FLDARE, D2SFCELV and the runoff average -- are not counted).
-      k_flux : static 7x8 (RIVELV ELEVTN NXTDST RIVWTH RIVHGT RIVLEN RIVMAN) + I1NEXT 4 + state reads
-               8x8 (RIVDPH RIVDPH_PRE RIVOUT_PRE FLDOUT_PRE FLDSTO FLDDPH FLDSTO_PRE STORGE)
-               + writes 2x8 (RIVOUT FLDOUT) = 140 B/cell, + diagnostics: velocity average r/w 16 and
-               the previous sub-step's 7 accumulators r/w 112 (rivout fldout outflw daminf averages,
-               outflw rivdph storge maxima)                                 = 140 (+128) B/cell
+def phase_bytes(N: int, E: int, L_bar: float, P: int, Lp: int, nlev: int, ndam: int, ldiag: bool, wet: tuple) -> dict:
+    """HBM bytes per launch of each sub-step kernel of the graph: every array element the kernel reads or
+    writes once every sub-step.  Gathers of neighbour values are L2 reuse and not counted again, nor are the
+    outputs of the last sub-step alone or maxima and averages that a sub-step leaves unchanged.  `wet` is
+    the share of cells with floodplain storage and of cells with floodplain outflow: the others skip the
+    arrays that hold zero there.
+      k_flux : maps 6x8 (RIVELV of the cell and the one below, RIVWTH, its reciprocal, RIVMAN, the
+               reciprocal of NXTDST) 48 + I1NEXT 4 + flag bytes 2 + depths (RIVDPH, RIVDPH_PRE) 16 + RIVOUT_PRE 8
+               + RIVSTO 8 + outflow pair written 16                                          = 102 B/cell
+               + diagnostics: velocity and river outflow averages r/w 32, three maxima read 24 = 56
+               + wet: FLDSTO LEVSTO RIVLEN FLDDPH ELEVTN RIVHGT FLDSTO_PRE 56, flowing: FLDOUT_PRE 8 and two
+               averages r/w 32
                + per path: endpoints 8, DST 8, skip 4, ELV/WTH/FLW_PRE/FLW 32 x Lp, FLWSUM 8
-      k_rate : RIVOUT FLDOUT 16 + CSR 4 + 4/edge + RIVSTO FLDSTO 16 + RATE 8        = 48 B/cell
-               + path CSR 8 and FLWSUM 8 per path end
-      k_store: RIVOUT FLDOUT RATE 24 + CSR 8 + I1NEXT 4 + RIVSTO FLDSTO RIVDPH FLDFRC RUNOFF 40
-               + RIVSTOMAX RIVLEN RIVWTH GRAREA 32 + layers 16 L_bar + writes 10x8 80 (_PRE x4,
-               RIVSTO FLDSTO RIVDPH FLDDPH FLDFRC STORGE)                   = 188+16 L_bar
-               (the last sub-step's own accumulators, once per outer step, are not counted)
-               + levee: index 4/cell + 7 params + LEVSTO r/w + LEVDPH w per levee cell
-               + dams: 112 B per dam, paths: FLW r/w 16 x Lp + FLWSUM 16 per path
-    This is the pass of a network with water on every floodplain: the kernels skip, cell by cell, the
-    arrays that hold zero there (floodplain and levee state, D2FLDOUT's averages), and exchange
-    outflows and depths as 16-byte pairs.  The count stays the same so that the fractions compare."""
-    flux = N * (140 + (128 if ldiag else 0)) + P * (8 + 8 + 4 + 32 * Lp + 8) + ndam * 112
-    rate = N * 48 + (E - N) * 4 + P * 2 * (8 + 8)
-    store = N * (188 + 16 * L_bar) + N * 4 + nlev * (7 * 8 + 16 + 8) + ndam * 112 + P * (16 * Lp + 16)
+      k_rate : flags 2, outflow pair 16, CSR 4 + 4/edge, RIVSTO 8, RATE 8, rescaled pair written 16 = 54
+               + wet: FLDSTO 8; + per path end: entry 8, FLWSUM 8
+      k_store: flags 2, rescaled pair 16, upstream slots 16, RUNOFF RIVSTO 16, depths r/w 32, RIVSTOMAX RIVLEN
+               RIVWTH 24, RIVOUT_PRE and RIVSTO written 16                                   = 122
+               + wet: FLDSTO FLDFRC LEVSTO r/w 48, FLDDPH FLDSTO_PRE LEVDPH written 24, GRAREA 8, layers
+               16 L_bar (over all cells), flowing: FLDOUT_PRE written 8; levee index 4 and 7 params per wet levee cell
+               + dams: 112 B per dam, paths: FLW r/w 16 x Lp, average r/w 16 x Lp, FLWSUM 16 per path"""
+    w, f = wet
+    lev = 8 if nlev else 0
+    flux = N * (102 + (56 if ldiag else 0) + w * (48 + lev) + f * (8 + (32 if ldiag else 0)))
+    flux += P * (8 + 8 + 4 + 32 * Lp + 8) + ndam * 112
+    rate = N * (54 + w * 8) + E * 4 + P * 2 * (8 + 8)
+    store = N * (122 + w * (56 + 3 * lev) + f * 8 + 16 * L_bar) + nlev * w * 60 + ndam * 112
+    store += P * ((32 if ldiag else 16) * Lp + 16)
     return {"k_flux": flux, "k_rate": rate, "k_store": store}
+
+
+def wet_shares(ctx, dev) -> tuple:
+    """Shares of the context's cells with floodplain storage and with floodplain outflow (device arrays)."""
+    import torch
+
+    from cmf_b200 import emulator as E
+
+    ctx.synchronize()
+    fe = E.Features(ctx, np.ones(ctx.N))
+    return tuple(float(torch.count_nonzero(E._raw_f64(p, ctx.M * ctx.N, dev))) / (ctx.M * ctx.N)
+                 for p in (fe.mb.fldsto, fe.mb.fldout_pre))
 
 
 def mean_layers(state: dict, fldstomax: np.ndarray, rivstomax: np.ndarray, N: int, L: int) -> float:
@@ -439,7 +453,7 @@ def gpu_arm(args) -> int:
     Lp = g.Lp
     nlev = int(np.sum(h.map("levbassto") < 1e17)) if h.opts.llevee else 0
     ndam = h.dims.ndam
-    roof = roofline(g, N, E, Lbar, P, Lp, nlev, ndam, M, loop_iters, K, secs)
+    roof = roofline(g, N, E, Lbar, P, Lp, nlev, ndam, M, loop_iters, K, secs, dev)
 
     # the one-member context is done: closed here, so that the 16-member and surrogate contexts
     # below each hold the hot-map L2 window in turn (one context holds it at a time)
@@ -513,37 +527,33 @@ def gpu_arm(args) -> int:
     return out
 
 
-def roofline(g, N, E, Lbar, P, Lp, nlev, ndam, M, loop_iters, K, secs) -> dict:
-    """Dominant kernel's achieved bandwidth on algorithmic bytes (live CUDA-event timing on the
-    library's stream) and the whole step's, on the fused minimum per cell-sub-step (316 + 16 L_bar
-    B, plus 32 + 40 Lp per path, 80 per levee cell and 112 per dam)."""
+def roofline(g, N, E, Lbar, P, Lp, nlev, ndam, M, loop_iters, K, secs, dev) -> dict:
+    """What bounds the timed region.  A persistent step is one kernel, timed by the region itself; it holds
+    the state on the SMs and is bound by the latency of its phases, so no bandwidth is quoted.  A graph's
+    dominant kernel: its achieved bandwidth on the bytes it moves (live CUDA-event timing on the library's
+    stream), and the whole step's."""
+    peaks = measured_peaks()
+    base = {"peak": peaks["hbm_gbs"], "unit": "GB/s", "peak_source": peaks["source"] + " (hbm_gbs, burst copy)",
+            "traffic": None, "traffic_note": "not measured in this run (ncu summaries under profiles/)", "L_bar": Lbar}
+    if g.launch_mode == 2:
+        return base | {"bound": "latency of three dependent phases per sub-step", "kernel": "persistent kernel",
+                       "kernel_ms": {"persistent kernel": secs / K * 1e3}, "achieved": None, "frac": None,
+                       "us_per_substep": secs / max(loop_iters, 1) * 1e6}
     phases = g.time_phases(reps=10)
-    pb = phase_bytes(N, E, Lbar, P, Lp, nlev, ndam, True)
+    pb = phase_bytes(N, E, Lbar, P, Lp, nlev, ndam, True, wet_shares(g, dev))
     per_sub_ms = {k: phases[k] for k in ("k_flux", "k_rate", "k_store")}
     dominant = max(per_sub_ms, key=per_sub_ms.get)
-    peaks = measured_peaks()
     achieved = pb[dominant] * M / (per_sub_ms[dominant] * 1e-3) / 1e9
-    fused = fused_minimum_bytes(N, Lbar, P, Lp, nlev, ndam)
-    step_gbs = fused * M * (loop_iters / max(K, 1)) / (secs / K) / 1e9
-    return {"bound": "hbm", "achieved": achieved, "peak": peaks["hbm_gbs"], "unit": "GB/s",
-            "frac": achieved / peaks["hbm_gbs"], "traffic": None,
-            "traffic_note": "not measured in this run (ncu summaries under profiles/)",
-            "kernel": dominant, "peak_source": peaks["source"] + " (hbm_gbs, burst copy)",
-            "algorithmic_bytes_per_launch": pb[dominant] * M,
-            "kernel_ms": {k: round(v, 5) for k, v in phases.items()}, "L_bar": Lbar,
-            "step_fused_minimum_bytes_per_substep": fused * M,
-            "step_achieved_gbs": step_gbs, "step_frac": step_gbs / peaks["hbm_gbs"]}
-
-
-def fused_minimum_bytes(N, Lbar, P, Lp, nlev, ndam) -> float:
-    """Compulsory bytes of a fully fused sub-step: (316 + 16 L_bar) per cell, 32 + 40 Lp per
-    bifurcation path, 80 per levee cell, 112 per dam (diagnostic accumulators not counted)."""
-    return N * (316 + 16 * Lbar) + P * (32 + 40 * Lp) + nlev * 80 + ndam * 112
+    step_gbs = sum(pb.values()) * M * (loop_iters / max(K, 1)) / (secs / K) / 1e9
+    return base | {"bound": "hbm", "achieved": achieved, "frac": achieved / peaks["hbm_gbs"], "kernel": dominant,
+                   "algorithmic_bytes_per_launch": pb[dominant] * M,
+                   "kernel_ms": {k: round(v, 5) for k, v in phases.items()},
+                   "step_achieved_gbs": step_gbs, "step_frac": step_gbs / peaks["hbm_gbs"]}
 
 
 def members_line(h, dev, M, base_fields, base, K, roof_args) -> dict:
     """M config-1 members on one context, each member the bench forcing times a lognormal(0, 0.3)
-    factor per cell: cell-substeps/s and the whole step's bandwidth on fused-minimum bytes."""
+    factor per cell: cell-substeps/s and, of a graph schedule, the sub-steps' bandwidth on the bytes they move."""
     import torch
 
     from cmf_b200 import PhysicsGPU
@@ -570,15 +580,16 @@ def members_line(h, dev, M, base_fields, base, K, roof_args) -> dict:
     sub = c1["member_substeps"] - c0["member_substeps"]
     iters = c1["loop_iters"] - c0["loop_iters"]
     Nn, E, Lbar, P, Lp, nlev, ndam = roof_args
-    fused = fused_minimum_bytes(Nn, Lbar, P, Lp, nlev, ndam)
-    gbs = fused * sub / secs / 1e9
-    peak = measured_peaks()["hbm_gbs"]
+    gbs = frac = None
+    if g.launch_mode == 0:
+        gbs = sum(phase_bytes(Nn, E, Lbar, P, Lp, nlev, ndam, True, wet_shares(g, dev)).values()) * sub / secs / 1e9
+        frac = gbs / measured_peaks()["hbm_gbs"]
     sched = {k: v for k, v in g.schedule().items() if k != "kernels"}
     g.close()
     del fields
     torch.cuda.empty_cache()
     return {"members": M, "cell_substeps_per_s": N * sub / secs, "ms_per_step": secs / K * 1e3,
-            "nt_mean": sub / (K * M), "step_achieved_gbs": gbs, "step_frac": gbs / peak,
+            "nt_mean": sub / (K * M), "step_achieved_gbs": gbs, "step_frac": frac,
             "l2": "working set far above L2 (no flush needed)", "steps": K, "schedule": sched}
 
 
@@ -684,7 +695,8 @@ def cfg2_arm(args) -> int:
         cells += h.dims.nseqall * sub
         nts[k] = sub / (K * p.M)
         nlev = int(np.sum(h.map("levbassto") < 1e17)) if h.opts.llevee else 0
-        pb = phase_bytes(h.dims.nseqall, int(h.map("i1upn").sum()), 0.0, p.P, p.Lp, nlev, h.dims.ndam, True)
+        pb = phase_bytes(h.dims.nseqall, int(h.map("i1upn").sum()), 0.0, p.P, p.Lp, nlev, h.dims.ndam, True,
+                         wet_shares(p, dev))
         abytes += sum(pb.values()) * sub
     if ws > 1:
         t = torch.tensor([secs], device=dev, dtype=torch.float64)
@@ -729,7 +741,7 @@ def cfg2_arm(args) -> int:
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peaks["hbm_gbs"], "unit": "GB/s",
                      "frac": achieved / peaks["hbm_gbs"] / ws, "traffic": None, "kernel": "sub-step kernels (all)",
                      "peak_source": peaks["source"] + " (hbm_gbs, burst copy, per GPU)",
-                     "note": "algorithmic bytes of k_flux+k_rate+k_store per member sub-step (L_bar taken as 0), "
+                     "note": "bytes moved by k_flux+k_rate+k_store per member sub-step (L_bar taken as 0), "
                              "stage/CFL and control kernels not counted; achieved over all GPUs"},
         "clocks": clk.summary(),
         "gpu_launches": launches,
@@ -784,7 +796,7 @@ def cfg4_arm(args) -> int:
     del fsm, flooded, scanned, tot
     E_up = int(h.map("i1upn").sum())
     nlev = int(np.sum(h.map("levbassto") < 1e17)) if h.opts.llevee else 0
-    pb = phase_bytes(N, E_up, Lbar, big.P, big.Lp, nlev, h.dims.ndam, True)
+    pb = phase_bytes(N, E_up, Lbar, big.P, big.Lp, nlev, h.dims.ndam, True, wet_shares(big, dev))
     peaks = measured_peaks()
     sweep = []
     top = None
