@@ -2,9 +2,9 @@
 //
 // A 4-layer MLP (input 32 -> 128 -> 128 -> 128 -> 1, ReLU) maps local state plus 8-hop upstream
 // messages of every cell to its mean outflow over the next coupling step.  BF16 operands, FP32
-// accumulation on the tensor cores (mma.sync m16n8k16 tiles for training and a register-chained
-// fused inference; tcgen05 MMAs into tensor memory for the production inference), FP32 master
-// weights updated by Adam.
+// accumulation on the tensor cores: tcgen05 MMAs into tensor memory for the training step, the layer-by-layer
+// GEMMs and the inference; mma.sync m16n8k16 tiles for the cross-checks of both (k_gemm, k_mlp_fused).  FP32
+// master weights updated by Adam.
 // The rollout kernel turns predicted outflows into a mass-conserving storage update along the
 // same upstream CSR the physics uses; the stage scheme then recomputes depths.
 #include <cuda_bf16.h>
@@ -1020,10 +1020,11 @@ __global__ void k_splitk_reduce(int M, int N, int splits, const float *__restric
 // products run in its order, so the dZ are its bits; the row sums of the gradients are taken per CTA
 // and then in CTA order, the same on every run.
 // Tensor memory: D 0..127, gW1 128..255, gW2 256..383, gW0 384..447, gW3 448..463, Y 464..479.
-// Bound: the chain of 8 dependent products of a tile (about 0.5 us each); 16 warps share every
-// epilogue (32 columns of one row per thread) to keep its other half short.  Measured with k_adam
-// (loss_and_grad + adam, per step): 16,384 rows 2136 us (layer by layer, about 45 launches) -> 34.5
-// us; 131,072 rows 4934 -> 90 us.
+// Bound: a tile's 10 products, seven of which wait for the one before and its epilogue: about 9.3 us a tile
+// with one tile in flight (131,072 rows take seven per CTA), the tensor pipe busy a fifth of the time; 16 warps
+// share every epilogue (32 columns of one row per thread) to keep that half of the chain short.  Measured with
+// k_adam (loss_and_grad + adam, per step): 16,384 rows 2136 us (layer by layer, about 45 launches) -> 34.2
+// us; 131,072 rows 4934 -> 90.3 us.
 // ------------------------------------------------------------------------------------------
 constexpr int kTrThreads = 512;
 constexpr int kTrW0 = 0;                                  // [64 k][128 n]

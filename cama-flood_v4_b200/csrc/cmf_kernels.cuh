@@ -1008,8 +1008,8 @@ __device__ __forceinline__ double path_flux(double wth, double pre, double gdt, 
     return (wth * (dout_pr + (gdt * dflw_im) * dslp)) / (1.0 + ((gdt * (man * man)) * fabs(dout_pr)) * pow_depth<7>(dflw_im));
 }
 
-// Coherent: the ends' values come past L1, which may hold an older sub-step's line (kernels that run
-// several phases)
+// Coherent: values of other cells come past L1, of which the resident kernel has hardly any; the phase
+// kernels and k_persist read them through L1, which the launch or the barrier's acquire has emptied
 template <bool Coherent>
 __device__ __forceinline__ double ld_nb(const double *p, size_t g) { return Coherent ? __ldcg(p + g) : p[g]; }
 
