@@ -723,8 +723,6 @@ int persist_setup(cmf_gpu_ctx *c) {
         if (per_sm >= 1) {
             a.tpm = (int)tpm;
             a.group = (int)group;
-            a.wait_ns = cmf::kWaitNsDefault;
-            a.selftest = 0;
             c->persist_grid = grid;
             c->res_threads = threads;
             return CMF_OK;
@@ -763,15 +761,17 @@ int resident_buffers(cmf_gpu_ctx *c) {
     return CMF_OK;
 }
 
-// one outer step as one cooperative launch; `selftest` (ResArgs): with waits of selftest_ns that cannot end
-int launch_persist(cmf_gpu_ctx *c, int selftest = 0, unsigned long long selftest_ns = 0) {
+// one outer step as one cooperative launch; selftest, with waits of wait_ns: 1 a barrier that cannot complete
+// alone, 2 a step whose barriers cannot, as its arrival count starts one short (the first arrival wraps it to 0)
+int launch_persist(cmf_gpu_ctx *c, int selftest = 0, unsigned long long wait_ns = cmf::kWaitNsDefault) {
     if (c->persist_grid < 1) return set_err(CMF_E_UNSUPPORTED, "the persistent kernel cannot be co-resident on this device");
     int rc;
     if ((rc = resident_buffers(c))) return rc;
-    CUDA_TRY(cudaMemsetAsync(&c->st.loop->bar, 0, sizeof(unsigned), c->stream));
+    CUDA_TRY(cudaMemsetAsync(&c->st.loop->bar, selftest == 2 ? 0xff : 0, sizeof(unsigned), c->stream));
     if (c->res.group > 0) {
         cmf::ResArgs a = c->res;
-        if (selftest) { a.wait_ns = selftest_ns; a.selftest = selftest; }
+        a.wait_ns = wait_ns;
+        a.selftest = selftest == 1;
         void *args[] = {&c->net, &c->st, &a};
         CUDA_TRY(cudaLaunchCooperativeKernel((const void *)c->res_kernel, dim3(c->persist_grid), dim3(c->res_threads), args,
                                              cmf::res_smem(a.slots), c->stream));
@@ -779,8 +779,8 @@ int launch_persist(cmf_gpu_ctx *c, int selftest = 0, unsigned long long selftest
         cmf::PersistArgs a{};
         a.tpm = (c->dims.nseqall + cmf::kTile - 1) / cmf::kTile;
         a.ppm = (cmf::path_threads(c->net.P, c->net.Lp) + cmf::kTile - 1) / cmf::kTile;
-        a.wait_ns = selftest ? selftest_ns : cmf::kWaitNsDefault;
-        a.selftest = selftest;
+        a.wait_ns = wait_ns;
+        a.selftest = selftest == 1;
         void *args[] = {&c->net, &c->st, &a};
         CUDA_TRY(cudaLaunchCooperativeKernel((const void *)cmf::k_persist, dim3(c->persist_grid), dim3(cmf::kTile), args,
                                              cmf::kPersistSmem, c->stream));

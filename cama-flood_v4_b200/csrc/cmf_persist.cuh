@@ -90,7 +90,7 @@ struct PersistArgs {
     int tpm;                    // cell tiles per member (ceil(N / kTile))
     int ppm;                    // path tiles per member (ceil(path_threads / kTile))
     unsigned long long wait_ns; // bound of every device-side wait
-    int selftest;               // 1: only run a barrier whose count can never complete (timeout check); 2: a step with it
+    int selftest;               // 1: only run a barrier whose count can never complete (timeout check)
 };
 
 __device__ __forceinline__ void budget_reduce(const Net &n, const State &s, int m, int k) {
@@ -165,10 +165,8 @@ __global__ void __launch_bounds__(kTile, kPersistMinBlocks) k_persist(Net n, Sta
     if (pa.selftest) {
         // barrier timeout check: the count target includes one arrival that never comes
         gb.nblocks = G + 1;
-        if (pa.selftest == 1) {
-            gb.sync();
-            return;
-        }
+        gb.sync();
+        return;
     }
     const int N = n.N, M = n.M, tpm = pa.tpm, ppm = pa.ppm;
     const int T = M * tpm, PT = M * ppm;

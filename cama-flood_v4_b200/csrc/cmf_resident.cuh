@@ -56,7 +56,7 @@ struct ResArgs {
     int tpm;                    // 32-cell tiles per member
     int group;                  // members per group
     int slots;                  // tiles of a CTA
-    int selftest;               // 1: only run a barrier whose count can never complete (timeout check); 2: a step with it
+    int selftest;               // 1: only run a barrier whose count can never complete (timeout check)
     unsigned long long wait_ns; // bound of every device-side wait
     int edges;                  // elements per member of raw and out
     int cells;                  // entries of `order`
@@ -232,10 +232,8 @@ __global__ void __launch_bounds__(Threads, 1) k_resident(Net n, State s, ResArgs
     GridBar gb{&s.loop->bar, &s.ctl[0].bar_err, G, 0u, a.wait_ns, &sflag};
     if (a.selftest) {           // the count target includes one arrival that never comes
         gb.nblocks = G + 1;
-        if (a.selftest == 1) {
-            gb.sync();
-            return;
-        }
+        gb.sync();
+        return;
     }
     const int N = n.N, tpm = a.tpm, slots = a.slots, stride = slots * 32;
     int *s_int = reinterpret_cast<int *>(fields + (size_t)kResFields * stride);    // [kResInts][slots * 32]
