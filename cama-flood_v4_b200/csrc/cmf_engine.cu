@@ -539,6 +539,29 @@ int hot_maps_window(cmf_gpu_ctx *c) {
     return CMF_OK;
 }
 
+// The member state comes from one allocation.  The device rounds each allocation of its own up to 2 MB (4 MB for
+// an array of a 300,000-cell member's 2.4 MB, and there are 60), and where those blocks came to lie moved the
+// resident kernel by 2 % (298,554 cells: 38.4 or 39.3 us per sub-step as an unrelated upload came or went; 38.3
+// in one block).
+struct Arena {
+    struct Part { void **p; size_t bytes; };
+    std::vector<Part> parts;
+    template <class T>
+    void add(T **p, size_t n) { parts.push_back({(void **)p, (std::max(n, (size_t)1) * sizeof(T) + 511) & ~(size_t)511}); }
+    int commit(cmf_gpu_ctx *c) {
+        size_t total = 0;
+        for (const Part &q : parts) total += q.bytes;
+        char *at = nullptr;
+        int rc = c->alloc(&at, total);
+        if (rc) return rc;
+        for (const Part &q : parts) {
+            *q.p = at;
+            at += q.bytes;
+        }
+        return CMF_OK;
+    }
+};
+
 int alloc_state(cmf_gpu_ctx *c) {
     cmf::State &s = c->st;
     const size_t MN = (size_t)c->dims.nmembers * c->dims.nseqall;
@@ -549,37 +572,40 @@ int alloc_state(cmf_gpu_ctx *c) {
                        &s.rivout_cur, &s.fldout_cur, &s.rivdph_pre, &s.fldsto_pre, &s.rivdph, &s.flddph,
                        &s.fldfrc, &s.fldare, &s.sfcelv, &s.storge, &s.rivvel, &s.rivinf, &s.fldinf, &s.pthout,
                        &s.outflw, &s.rate, &s.runoff};
-    int rc;
-    for (double **p : cell)
-        if ((rc = c->alloc(p, MN))) return rc;
-    if ((rc = c->alloc(&s.raw, MN)) || (rc = c->alloc(&s.out, MN)) || (rc = c->alloc(&s.dph, MN)) || (rc = c->alloc(&s.wet, MN)))
-        return rc;
+    Arena a;
+    for (double **p : cell) a.add(p, MN);
+    a.add(&s.raw, MN);
+    a.add(&s.out, MN);
+    a.add(&s.dph, MN);
+    a.add(&s.wet, MN);
     const size_t opt_cells[] = {c->opts.llevee ? MN : 1, c->opts.ldamout ? MN : 1};
-    if ((rc = c->alloc(&s.levsto, opt_cells[0])) || (rc = c->alloc(&s.levdph, opt_cells[0]))) return rc;
-    if ((rc = c->alloc(&s.damsto, opt_cells[1])) || (rc = c->alloc(&s.daminf, opt_cells[1]))) return rc;
-    if ((rc = c->alloc(&s.pthflw_raw, MPL)) || (rc = c->alloc(&s.pthflw_pre, MPL)) || (rc = c->alloc(&s.pthsum_raw, MP)) ||
-        (rc = c->alloc(&s.pthsum, MP)))
-        return rc;
+    a.add(&s.levsto, opt_cells[0]);
+    a.add(&s.levdph, opt_cells[0]);
+    a.add(&s.damsto, opt_cells[1]);
+    a.add(&s.daminf, opt_cells[1]);
+    a.add(&s.pthflw_raw, MPL);
+    a.add(&s.pthflw_pre, MPL);
+    a.add(&s.pthsum_raw, MP);
+    a.add(&s.pthsum, MP);
     double **diag[] = {&s.a_rivout, &s.a_fldout, &s.a_outflw, &s.a_rivvel, &s.a_pthout, &s.a_runoff,
                        &s.m_storge, &s.m_outflw, &s.m_rivdph};
-    for (double **p : diag)
-        if ((rc = c->alloc(p, dg ? MN : 1))) return rc;
-    if ((rc = c->alloc(&s.a_daminf, (dg && c->opts.ldamout) ? MN : 1))) return rc;
-    if ((rc = c->alloc(&s.a_pthflw, dg ? MPL : 1)) || (rc = c->alloc(&s.a_pthsum, dg ? MP : 1))) return rc;
+    for (double **p : diag) a.add(p, dg ? MN : 1);
+    a.add(&s.a_daminf, (dg && c->opts.ldamout) ? MN : 1);
+    a.add(&s.a_pthflw, dg ? MPL : 1);
+    a.add(&s.a_pthsum, dg ? MP : 1);
     // output-interval accumulators (zeroed by alloc: CMF_DIAG_INIT leaves them at zero, NADD_out = 0)
     const bool dout = c->net.ldiag_out;
     double **oarr[] = {&s.o_rivout, &s.o_fldout, &s.o_outflw, &s.o_rivvel, &s.o_pthout, &s.o_runoff,
                        &s.om_storge, &s.om_outflw, &s.om_rivdph};
-    for (double **p : oarr)
-        if ((rc = c->alloc(p, dout ? MN : 1))) return rc;
-    if ((rc = c->alloc(&s.o_daminf, (dout && c->opts.ldamout) ? MN : 1)) || (rc = c->alloc(&s.o_pthflw, dout ? MPL : 1)) ||
-        (rc = c->alloc(&s.o_nadd, c->dims.nmembers)))
-        return rc;
-    if ((rc = c->alloc(&s.ctl, c->dims.nmembers)) || (rc = c->alloc(&s.loop, 1))) return rc;
+    for (double **p : oarr) a.add(p, dout ? MN : 1);
+    a.add(&s.o_daminf, (dout && c->opts.ldamout) ? MN : 1);
+    a.add(&s.o_pthflw, dout ? MPL : 1);
+    a.add(&s.o_nadd, c->dims.nmembers);
+    a.add(&s.ctl, c->dims.nmembers);
+    a.add(&s.loop, 1);
     // budget partials: one per warp of 32 cells, per member and budget
-    if ((rc = c->alloc(&s.partials, (size_t)c->dims.nmembers * cmf::budget_warps(c->dims.nseqall) * cmf::kBudgets)))
-        return rc;
-    return CMF_OK;
+    a.add(&s.partials, (size_t)c->dims.nmembers * cmf::budget_warps(c->dims.nseqall) * cmf::kBudgets);
+    return a.commit(c);
 }
 
 // phase A and phase C in the schedule's occupancy profile; grids cover the cells of every member,

@@ -259,3 +259,27 @@ def test_persistent_with_many_upstream_cells(case_dirs, upstream):
         assert _same(sa[f], sb[f]), f
     for f in DIAG_KEYS:
         assert _same(ga[f], gb[f]), f
+
+
+def test_member_state_takes_its_arrays_and_no_more(case_dirs):
+    """The device memory a member adds is that of its arrays (332 B per cell with diagnostics, levees and
+    dams, and its paths' 144 B each), not of 60 allocations rounded up."""
+    import torch
+
+    from cmf_b200 import HostModel, PhysicsGPU
+
+    h = HostModel(case_dirs["cfg1s"])
+    N, P = h.dims.nseqall, h.dims.npthout
+    assert h.dims.npthlev == 5
+
+    def made(members):
+        torch.cuda.synchronize()
+        before = torch.cuda.mem_get_info(0)[0]
+        p = PhysicsGPU(h, nmembers=members, block_size=128)
+        torch.cuda.synchronize()
+        used = before - torch.cuda.mem_get_info(0)[0]
+        p.close()
+        return used
+
+    made(1)                                      # modules and streams of a first context
+    assert made(64) - made(1) <= 63 * (332 * N + 144 * P) + 8 * 2 ** 20
